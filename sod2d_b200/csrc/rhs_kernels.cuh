@@ -300,14 +300,20 @@ struct RhsArgs {
   int *err;  // mapped host flag: set when a bulk-copy wait of pass B gave up
 };
 
-// Staged pairs of pass B, one float2 per element node:
-//   CONV (and CONV+DIFF): (u0,u1) (u2,rho) (q0,q1) (q2,p) (H,rho*H) [(T,0)]
-//   DIFF only           : (u0,u1) (u2,rho) (T,0)
-// The 18 product fields of the split form -- q_a u_b and u_a u_b (a <= b),
-// rho*H*u_c and H*u_c -- are formed in registers from the staged values of
-// each line node as it is read.  A product rounds the same way whether it
-// is formed here or before staging, so this only trades shared-memory
-// traffic (11 staged values per node instead of 29) for FP32 multiplies.
+// Staged fields of pass B, one entry per element node:
+//   CONV+DIFF (conserved inputs): float4 (u0,u1,u2,H) and (rho,T,p,0)
+//   CONV only : float2 pairs (u0,u1) (u2,rho) (q0,q1) (q2,p) (H,rho*H)
+//   DIFF only : float2 pairs (u0,u1) (u2,rho) (T,0)
+// With the conserved inputs q = rho u, so every split-form term is a product
+// of staged values and one product per line node serves momentum, mass and
+// energy (FLUX2 below).  Instruction issue bounds this kernel: that form
+// issues 829 instructions per Gauss point where 18 product fields, formed
+// from each line node and differentiated one by one, took 1251 (k_rhs at
+// 32^3 117.6 -> 102.1 us; RHS at 64^3 1.72 -> 1.55 ms), with the same error
+// against FP64.
+// With convection inputs u, q, rho, p, E given independently, the 18 product
+// fields -- q_a u_b and u_a u_b (a <= b), rho*H*u_c and H*u_c -- are formed
+// in registers from the staged values of each line node as it is read.
 enum { PB_U01 = 0, PB_U2R = 1, PB_Q01 = 2, PB_Q2P = 3, PB_HRH = 4 };
 
 // Shared-memory plan of k_rhs.  Two prefetch stages (the element group being
@@ -323,8 +329,10 @@ struct RhsPlan {
   static constexpr bool DIFF = (MODE & MODE_DIFF) != 0;
   static constexpr bool LPS = (MODE & MODE_NOLPS) == 0;
   static constexpr int NC = LPS ? 5 : 6;  // staged contravariant flux fields of the weak divergence
-  static constexpr int NPAIR = CONV ? (DIFF ? 6 : 5) : 3;
-  static constexpr int PB_T = CONV ? 5 : 2;
+  // conserved inputs (q = rho u): two float4 per node, otherwise pairs
+  static constexpr bool FLUX2 = CONV && IN == IN_CONS;
+  static constexpr int NPAIR = FLUX2 ? 4 : (CONV ? 5 : 3);
+  static constexpr int PB_T = 2;
   // IN_CONS: rho q0 q1 q2 E | IN_PRIM: rho u0 u1 u2 q0 q1 q2 p h | IN_DIFF: rho rho_n u0 u1 u2 T mu
   static constexpr int NIN = IN == IN_CONS ? 5 : (IN == IN_PRIM ? 9 : 7);
   static constexpr int O_IN = 0, O_GEO = NIN * NTB, O_POS = O_GEO + 10 * NTB, O_MUE = O_POS + NTB,
@@ -344,7 +352,8 @@ __global__ void __launch_bounds__(EPB *Cfg<P>::NT, SOD_RHS_THREADS_PER_SM / (EPB
 k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
   using L = RhsPlan<P, EPB, MODE, IN>;
   constexpr int N1 = L::N1, N = L::N, NT = L::NT, NTB = L::NTB, NC = L::NC, SMF = L::SMF, PB_T = L::PB_T;
-  constexpr bool CONV = L::CONV, DIFF = L::DIFF, LPS = L::LPS;
+  constexpr bool CONV = L::CONV, DIFF = L::DIFF, LPS = L::LPS, FLUX2 = L::FLUX2;
+  static_assert(FLUX2 || !(CONV && DIFF), "convection with diffusion runs on the conserved state");
   extern __shared__ __align__(16) float dsm[];
   const int tid = threadIdx.x, el = tid / NT, t = tid % NT;
   const int i = t % N1, j = (t / N1) % N1, k = t / (N1 * N1);
@@ -352,6 +361,7 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
   const long long ngroups = ((long long)m.nelem + EPB - 1) / EPB, G = gridDim.x;
   float *const sf = dsm + L::O_STG + el * SMF * N;
   float2 *const sp = reinterpret_cast<float2 *>(sf);
+  float4 *const sq = reinterpret_cast<float4 *>(sf);
   const float invR = __frcp_rn(Rgas);
   // P = 3, one element per block: the element's J^-1 and gpvol (2560 B),
   // slot positions and mu_e (256 B each) are contiguous and 16-byte aligned
@@ -452,6 +462,12 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
       if (IN == IN_CONS) {
         eos_fast(ph, invR, A.mu_factor, in[0], in[NTB], in[2 * NTB], in[3 * NTB], in[4 * NTB], s);
         mu = s.mu;
+        const float ri = __frcp_rn(s.rho);
+        if (FLUX2) {  // u = q / rho to half an ulp: rho u stands for q below
+          s.u0 = fmaf(fmaf(-s.rho, s.u0, s.q0), ri, s.u0);
+          s.u1 = fmaf(fmaf(-s.rho, s.u1, s.q1), ri, s.u1);
+          s.u2 = fmaf(fmaf(-s.rho, s.u2, s.q2), ri, s.u2);
+        }
       } else if (IN == IN_PRIM) {
         s.rho = in[0];
         s.u0 = in[NTB]; s.u1 = in[2 * NTB]; s.u2 = in[3 * NTB];
@@ -465,8 +481,6 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
         mu = in[6 * NTB];
         s.q0 = s.q1 = s.q2 = 0.f; s.p = 0.f; s.h = 0.f;
       }
-      sp[PB_U01 * N + t] = make_float2(s.u0, s.u1);
-      sp[PB_U2R * N + t] = make_float2(s.u2, s.rho);
       if (CONV) {
         // H = h + k with k = |u|^2/2: the reference's split-form energy
         // terms for E:=h and for k enter with the same 1/4 weight, so their
@@ -476,11 +490,20 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
         kk = kk + s.u2 * s.u2 * 0.5f;
         H = s.h + kk;
         rH = s.rho * H;
-        sp[PB_Q01 * N + t] = make_float2(s.q0, s.q1);
-        sp[PB_Q2P * N + t] = make_float2(s.q2, s.p);
-        sp[PB_HRH * N + t] = make_float2(H, rH);
       }
-      if (DIFF) sp[PB_T * N + t] = make_float2(s.T, 0.f);
+      if (FLUX2) {
+        sq[t] = make_float4(s.u0, s.u1, s.u2, H);
+        sq[N + t] = make_float4(s.rho, s.T, s.p, 0.f);
+      } else {
+        sp[PB_U01 * N + t] = make_float2(s.u0, s.u1);
+        sp[PB_U2R * N + t] = make_float2(s.u2, s.rho);
+        if (CONV) {
+          sp[PB_Q01 * N + t] = make_float2(s.q0, s.q1);
+          sp[PB_Q2P * N + t] = make_float2(s.q2, s.p);
+          sp[PB_HRH * N + t] = make_float2(H, rH);
+        }
+        if (DIFF) sp[PB_T * N + t] = make_float2(s.T, 0.f);
+      }
     }
     // staged pairs visible; every thread is done with the other stage
     if (!__syncthreads_and(bulk_ok)) {
@@ -494,7 +517,70 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
     float res[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // mass, energy, mom x,y,z
     float gradRho[3] = {0.f, 0.f, 0.f}, gradT[3] = {0.f, 0.f, 0.f};
     float gradU[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    if (active) {
+    if (FLUX2 && active) {
+      // Split form with one product per line node.  With q = rho u and
+      // U = u . He(:,d) (He of the output point), direction d contributes
+      //   f S_d + sum_m D(m) w_m f_m + rho U sum_m D(m) f_m,
+      //   w_m = rho_m U_m + rho_m U + rho U_m,  S_d = sum_m D(m) w_m
+      // to 4 times the terms of f = u_a (momentum) and f = H (energy), and
+      // S_d to twice the mass term; S = div q + rho div u + u . grad rho.
+      const float2 z2 = make_float2(0.f, 0.f);
+      float2 c01 = z2, c2H = z2;  // momentum x, y; momentum z, energy
+      float divQ = 0.f, ugR = 0.f, gradP[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const int cd = d == 0 ? i : (d == 1 ? j : k);
+        const int stride = d == 0 ? 1 : (d == 1 ? N1 : N1 * N1);
+        const int base = t - cd * stride;
+        float Dd[N1];
+#pragma unroll
+        for (int q = 0; q < N1; ++q) Dd[q] = m.Dnat[cd * N1 + q];
+        const float h[3] = {gm[(0 + 3 * d) * NTB], gm[(1 + 3 * d) * NTB], gm[(2 + 3 * d) * NTB]};
+        const float Ud = h[0] * s.u0 + h[1] * s.u1 + h[2] * s.u2;
+        float2 aU01 = z2, aU2H = z2, aRT = z2, d01 = z2, d2H = z2;
+        float aP = 0.f, aQ = 0.f;
+#pragma unroll
+        for (int ss = 0; ss < N1; ++ss) {
+          const int mm = ref_order<P>(ss);  // the reference's 1-D summation order
+          const int tm = base + mm * stride;
+          const float4 a = sq[tm], b = sq[N + tm];
+          const float2 a01 = make_float2(a.x, a.y), a2H = make_float2(a.z, a.w);
+          const float2 D2 = make_float2(Dd[mm], Dd[mm]);
+          const float Um = fmaf(h[0], a.x, fmaf(h[1], a.y, h[2] * a.z)), q = b.x * Um;
+          const float c = Dd[mm] * fmaf(s.rho, Um, fmaf(b.x, Ud, q));
+          const float2 c2 = make_float2(c, c);
+          aQ = fmaf(Dd[mm], q, aQ);
+          d01 = __ffma2_rn(c2, a01, d01);
+          d2H = __ffma2_rn(c2, a2H, d2H);
+          aU01 = __ffma2_rn(D2, a01, aU01);
+          aU2H = __ffma2_rn(D2, a2H, aU2H);
+          aRT = __ffma2_rn(D2, make_float2(b.x, b.y), aRT);
+          aP = fmaf(Dd[mm], b.z, aP);
+        }
+        const float2 Qd2 = make_float2(s.rho * Ud, s.rho * Ud);
+        c01 = __fadd2_rn(c01, __ffma2_rn(Qd2, aU01, d01));
+        c2H = __fadd2_rn(c2H, __ffma2_rn(Qd2, aU2H, d2H));
+        divQ = divQ + aQ;
+        ugR = ugR + Ud * aRT.x;
+        const float dU[3] = {aU01.x, aU01.y, aU2H.x};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          gradRho[a] = gradRho[a] + h[a] * aRT.x;
+          if (DIFF) gradT[a] = gradT[a] + h[a] * aRT.y;
+          gradP[a] = gradP[a] + h[a] * aP;
+#pragma unroll
+          for (int b = 0; b < 3; ++b) gradU[a][b] = gradU[a][b] + h[b] * dU[a];
+        }
+      }
+      const float gc = A.fact_c * gm[9 * NTB];
+      const float S = divQ + s.rho * (gradU[0][0] + gradU[1][1] + gradU[2][2]) + ugR;
+      res[0] = gc * (0.5f * S);
+      res[1] = gc * (0.25f * (c2H.y + H * S));
+      res[2] = gc * (0.25f * (c01.x + s.u0 * S) + gradP[0]);
+      res[3] = gc * (0.25f * (c01.y + s.u1 * S) + gradP[1]);
+      res[4] = gc * (0.25f * (c2H.x + s.u2 * S) + gradP[2]);
+    }
+    if (!FLUX2 && active) {
       // Physical-space sums, accumulated one reference direction d at a
       // time: d_a f = sum_d He(a,d) d_d f, and every convective term is
       // linear in the derivatives, so each direction's derivatives are
