@@ -52,7 +52,7 @@ struct sod_gpu_ctx {
   int *conn = nullptr, *lpoin_w = nullptr, *slot_ptr = nullptr, *slot_idx = nullptr, *slot_pos = nullptr,
       *lelpn = nullptr;
   int *a_of_t = nullptr;  // tensor position -> reference local node (0-based)
-  float *geo = nullptr, *Dnat = nullptr, *invMl = nullptr, *Ml = nullptr, *helem = nullptr, *helem_l_t = nullptr;
+  float *geo = nullptr, *Dnat = nullptr, *Drot = nullptr, *invMl = nullptr, *Ml = nullptr, *helem = nullptr, *helem_l_t = nullptr;
   // scratch
   float *slotsA = nullptr, *slotsB = nullptr, *proj12 = nullptr, *mue_t = nullptr, *musgs_t = nullptr;
   unsigned *vbits = nullptr;  // minimum density of the standalone smart_visc_spectral_imex
@@ -161,7 +161,7 @@ struct sod_gpu_ctx {
   MeshDev md() const {
     MeshDev m;
     m.nelem = nelem; m.npoin = npoin; m.npoin_w = npoin_w;
-    m.conn = conn; m.geo = geo; m.Dnat = Dnat; m.lpoin_w = lpoin_w; m.invMl = invMl;
+    m.conn = conn; m.geo = geo; m.Dnat = Dnat; m.Drot = Drot; m.lpoin_w = lpoin_w; m.invMl = invMl;
     m.slot_ptr = slot_ptr; m.slot_idx = slot_idx; m.slot_pos = slot_pos;
     return m;
   }

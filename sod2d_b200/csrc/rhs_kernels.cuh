@@ -47,6 +47,8 @@ struct MeshDev {
   const int *conn;      // [E][N]
   const float *geo;     // [E][10][N]
   const float *Dnat;    // [N1][N1]
+  const float *Drot;    // [2][N1][8]: rows, then columns, of Dnat rotated to start at the
+                        // diagonal: D[c][(c+s) % N1], D[(c+s) % N1][c], s = 0..P
   const int *lpoin_w;   // 0-based
   const float *invMl;   // [npoin]
   const int *slot_ptr;  // [npoin+1]
@@ -88,6 +90,14 @@ __device__ __forceinline__ void iso_grad(const float *__restrict__ f, int i, int
       g2 = fmaf(Dk[m], f[i + N1 * j + N1 * N1 * m], g2);
     }
   }
+}
+
+// Row c of a table of MeshDev::Drot.
+template <int P>
+__device__ __forceinline__ void load_drot(const float *__restrict__ tab, int c, float (&D)[P + 1]) {
+  const float4 v = *reinterpret_cast<const float4 *>(tab + 8 * c);
+  D[0] = v.x; D[1] = v.y; D[2] = v.z; D[3] = v.w;
+  if (P == 4) D[4] = tab[8 * c + 4];
 }
 
 struct NodeQ {  // primitive quantities of one node
@@ -352,7 +362,7 @@ __global__ void __launch_bounds__(EPB *Cfg<P>::NT, SOD_RHS_THREADS_PER_SM / (EPB
 k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
   using L = RhsPlan<P, EPB, MODE, IN>;
   constexpr int N1 = L::N1, N = L::N, NT = L::NT, NTB = L::NTB, NC = L::NC, SMF = L::SMF, PB_T = L::PB_T;
-  constexpr bool CONV = L::CONV, DIFF = L::DIFF, LPS = L::LPS, FLUX2 = L::FLUX2;
+  constexpr bool CONV = L::CONV, DIFF = L::DIFF, LPS = L::LPS, FLUX2 = L::FLUX2, ROT = P == 3;
   static_assert(FLUX2 || !(CONV && DIFF), "convection with diffusion runs on the conserved state");
   extern __shared__ __align__(16) float dsm[];
   const int tid = threadIdx.x, el = tid / NT, t = tid % NT;
@@ -378,6 +388,32 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
   }
   if (BULK) __syncthreads();
 
+  // ROT (P = 3): a line is summed in cyclic steps 2, 3, 1 from the thread's
+  // own node, which comes last, from registers: three shared loads per line
+  // instead of four, in a kernel whose shared-memory pipe is 71 % busy
+  // (wavefronts 17.1 -> 15.3 M at 32^3; k_rhs 102.1 -> 94.3 us, RHS at 64^3
+  // 1.575 -> 1.515 ms).  Of the 24 orders this one rounds least on constant
+  // and smooth fields (0.75 of the error of the order -1, +1, interior) and
+  // the same on random ones.  At P = 4 the rotated rows of 5 conflict in
+  // shared memory (136.4 against 133.5 us at 23x19x17): node ref_order(q).
+  auto line_step = [](int q) -> int { return q == 0 ? 2 : (q == 1 ? 3 : (q == 2 ? 1 : 0)); };
+  auto line_node = [&](int d, int q) -> int {
+    const int cd = d == 0 ? i : (d == 1 ? j : k), stride = d == 0 ? 1 : (d == 1 ? N1 : N1 * N1);
+    if (ROT) {
+      const int s = line_step(q);
+      return t + (cd + s < N1 ? s : s - N1) * stride;
+    }
+    return t + (ref_order<P>(q) - cd) * stride;
+  };
+  auto line_coef = [&](const float (&D)[N1], int q) -> float { return D[ROT ? line_step(q) : ref_order<P>(q)]; };
+  auto load_row = [&](int c, bool col, float (&D)[N1]) {
+    if (ROT) {
+      load_drot<P>(m.Drot + (col ? 8 * N1 : 0), c, D);
+    } else {
+#pragma unroll
+      for (int q = 0; q < N1; ++q) D[q] = col ? m.Dnat[q * N1 + c] : m.Dnat[c * N1 + q];
+    }
+  };
   auto node_of = [&](long long g) -> int {
     const long long e = g * EPB + el;
     return (g < ngroups && e < m.nelem && t < N) ? m.conn[e * N + t] : -1;
@@ -529,33 +565,30 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
       float divQ = 0.f, ugR = 0.f, gradP[3] = {0.f, 0.f, 0.f};
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const int cd = d == 0 ? i : (d == 1 ? j : k);
-        const int stride = d == 0 ? 1 : (d == 1 ? N1 : N1 * N1);
-        const int base = t - cd * stride;
         float Dd[N1];
-#pragma unroll
-        for (int q = 0; q < N1; ++q) Dd[q] = m.Dnat[cd * N1 + q];
+        load_row(d == 0 ? i : (d == 1 ? j : k), false, Dd);
         const float h[3] = {gm[(0 + 3 * d) * NTB], gm[(1 + 3 * d) * NTB], gm[(2 + 3 * d) * NTB]};
         const float Ud = h[0] * s.u0 + h[1] * s.u1 + h[2] * s.u2;
         float2 aU01 = z2, aU2H = z2, aRT = z2, d01 = z2, d2H = z2;
         float aP = 0.f, aQ = 0.f;
 #pragma unroll
-        for (int ss = 0; ss < N1; ++ss) {
-          const int mm = ref_order<P>(ss);  // the reference's 1-D summation order
-          const int tm = base + mm * stride;
-          const float4 a = sq[tm], b = sq[N + tm];
+        for (int mm = 0; mm < N1; ++mm) {
+          const bool own = ROT && mm == P;  // the node itself comes from its registers
+          const float Dm = line_coef(Dd, mm);
+          const float4 a = own ? make_float4(s.u0, s.u1, s.u2, H) : sq[line_node(d, mm)];
+          const float4 b = own ? make_float4(s.rho, s.T, s.p, 0.f) : sq[N + line_node(d, mm)];
           const float2 a01 = make_float2(a.x, a.y), a2H = make_float2(a.z, a.w);
-          const float2 D2 = make_float2(Dd[mm], Dd[mm]);
+          const float2 D2 = make_float2(Dm, Dm);
           const float Um = fmaf(h[0], a.x, fmaf(h[1], a.y, h[2] * a.z)), q = b.x * Um;
-          const float c = Dd[mm] * fmaf(s.rho, Um, fmaf(b.x, Ud, q));
+          const float c = Dm * fmaf(s.rho, Um, fmaf(b.x, Ud, q));
           const float2 c2 = make_float2(c, c);
-          aQ = fmaf(Dd[mm], q, aQ);
+          aQ = fmaf(Dm, q, aQ);
           d01 = __ffma2_rn(c2, a01, d01);
           d2H = __ffma2_rn(c2, a2H, d2H);
           aU01 = __ffma2_rn(D2, a01, aU01);
           aU2H = __ffma2_rn(D2, a2H, aU2H);
           aRT = __ffma2_rn(D2, make_float2(b.x, b.y), aRT);
-          aP = fmaf(Dd[mm], b.z, aP);
+          aP = fmaf(Dm, b.z, aP);
         }
         const float2 Qd2 = make_float2(s.rho * Ud, s.rho * Ud);
         c01 = __fadd2_rn(c01, __ffma2_rn(Qd2, aU01, d01));
@@ -780,21 +813,19 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
       __syncthreads();
       if (active) {
         // Weak divergence: sum_d sum_m D[m][i_d] C_d(node with d-index m).
-        float Dci[N1], Dcj[N1], Dck[N1];
-#pragma unroll
-        for (int q = 0; q < N1; ++q) { Dci[q] = m.Dnat[q * N1 + i]; Dcj[q] = m.Dnat[q * N1 + j]; Dck[q] = m.Dnat[q * N1 + k]; }
+        float Dc[3][N1];
+        load_row(i, true, Dc[0]);
+        load_row(j, true, Dc[1]);
+        load_row(k, true, Dc[2]);
         float wd[NC];
 #pragma unroll
         for (int q = 0; q < NC; ++q) {
-          const float *c0 = sf + (q * 3 + 0) * N, *c1 = sf + (q * 3 + 1) * N, *c2 = sf + (q * 3 + 2) * N;
           float acc = 0.f;
 #pragma unroll
-          for (int ss = 0; ss < N1; ++ss) {
-            const int mm = ref_order<P>(ss);
-            acc = fmaf(Dci[mm], c0[mm + N1 * j + N1 * N1 * k], acc);
-            acc = fmaf(Dcj[mm], c1[i + N1 * mm + N1 * N1 * k], acc);
-            acc = fmaf(Dck[mm], c2[i + N1 * j + N1 * N1 * mm], acc);
-          }
+          for (int mm = 0; mm < N1; ++mm)
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+              acc = fmaf(line_coef(Dc[d], mm), ROT && mm == P ? C[q][d] : sf[(q * 3 + d) * N + line_node(d, mm)], acc);
           wd[q] = acc;
         }
         if (LPS) {

@@ -53,6 +53,12 @@ int sod_gpu_init(const sod_mesh_t *mesh, const sod_phys_t *phys, sod_gpu_ctx **o
     int mrow = nat_of(P, mesh->gmshAtoI[a] - 1);
     for (int ii = 0; ii < N1; ++ii) D[mrow * N1 + nat_of(P, ii)] = mesh->dlxigp_ip[a + (long long)N * (0 + 3 * ii)];
   }
+  std::vector<float> Drot(2 * N1 * 8, 0.f);
+  for (int a = 0; a < N1; ++a)
+    for (int s = 0; s < N1; ++s) {
+      Drot[8 * a + s] = D[a * N1 + (a + s) % N1];
+      Drot[8 * (N1 + a) + s] = D[((a + s) % N1) * N1 + a];
+    }
   std::vector<int> conn((size_t)E * N);
   std::vector<float> geo((size_t)E * 10 * N);
   std::vector<int> cnt(NP + 1, 0);
@@ -92,7 +98,8 @@ int sod_gpu_init(const sod_mesh_t *mesh, const sod_phys_t *phys, sod_gpu_ctx **o
   c->ph.twoThirds = 2.0f / 3.0f;
   int rc = 0;
   if ((rc = c->upload(&c->conn, conn.data(), conn.size())) || (rc = c->upload(&c->geo, geo.data(), geo.size())) ||
-      (rc = c->upload(&c->Dnat, D.data(), D.size())) || (rc = c->upload(&c->lpoin_w, lw.data(), lw.size())) ||
+      (rc = c->upload(&c->Dnat, D.data(), D.size())) ||
+      (rc = c->upload(&c->Drot, Drot.data(), Drot.size())) || (rc = c->upload(&c->lpoin_w, lw.data(), lw.size())) ||
       (rc = c->upload(&c->slot_ptr, cnt.data(), cnt.size())) ||
       (rc = c->upload(&c->slot_idx, slot_idx.data(), slot_idx.size())) ||
       (rc = c->upload(&c->slot_pos, slot_pos.data(), slot_pos.size())) ||
