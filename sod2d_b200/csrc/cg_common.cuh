@@ -137,7 +137,7 @@ inline int ensure_cg_loop(sod_gpu_ctx *c) {
   if (G.S) return 0;
   int rc;
   if ((rc = c->alloc(&G.S, 1)) || (rc = c->alloc(&G.hist, CG_HIST)) || (rc = c->alloc(&G.ticket, 1)) ||
-      (rc = c->alloc(&G.gpart, (size_t)3 * cg_blocks(c->npoin, 2))))
+      (rc = c->alloc(&G.gpart, (size_t)3 * cg_blocks(c->npoin, 1))))
     return rc;
   CUDA_TRY(cudaMemset(G.ticket, 0, sizeof(unsigned)));
   CUDA_TRY(cudaMemset(G.S, 0, sizeof(CgScal)));

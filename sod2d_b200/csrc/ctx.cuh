@@ -52,6 +52,7 @@ struct sod_gpu_ctx {
   int *conn = nullptr, *lpoin_w = nullptr, *slot_ptr = nullptr, *slot_idx = nullptr, *slot_pos = nullptr,
       *lelpn = nullptr;
   int *a_of_t = nullptr;  // tensor position -> reference local node (0-based)
+  double *D64 = nullptr;
   float *geo = nullptr, *Dnat = nullptr, *Drot = nullptr, *invMl = nullptr, *Ml = nullptr, *helem = nullptr, *helem_l_t = nullptr;
   // scratch
   float *slotsA = nullptr, *slotsB = nullptr, *proj12 = nullptr, *mue_t = nullptr, *musgs_t = nullptr;
@@ -161,7 +162,7 @@ struct sod_gpu_ctx {
   MeshDev md() const {
     MeshDev m;
     m.nelem = nelem; m.npoin = npoin; m.npoin_w = npoin_w;
-    m.conn = conn; m.geo = geo; m.Dnat = Dnat; m.Drot = Drot; m.lpoin_w = lpoin_w; m.invMl = invMl;
+    m.conn = conn; m.geo = geo; m.Dnat = Dnat; m.Drot = Drot; m.D64 = D64; m.lpoin_w = lpoin_w; m.invMl = invMl;
     m.slot_ptr = slot_ptr; m.slot_idx = slot_idx; m.slot_pos = slot_pos;
     return m;
   }
@@ -317,6 +318,22 @@ inline int num_sms() {
     return v;
   }();
   return n;
+}
+
+// Launch with programmatic stream serialization (see pdl_wait).
+template <class... KA, class... A>
+inline cudaError_t launch_pdl(void (*k)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A &&...a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<KA>(a)...);
 }
 
 inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }

@@ -77,9 +77,64 @@ int sod_gpu_full_convec_ijk_incomp(sod_gpu_ctx *c, const float *u, const float *
   return c->finish();
 }
 
+}  // extern "C"
+
+namespace {
+
+// conjGrad_pressure_incomp with the iteration on the device: three launches
+// per iteration (search direction and element Laplacian; assembly, p.Ap and
+// alpha; update, norms and beta) and one host read per batch of iterations,
+// where six launches and a host read per iteration left the GPU idle a third
+// of the time.  The scalars are rounded as on the host: same iterates but
+// for the order of the FP64 sums.  (A partitioned mesh, whose dot products
+// pass through the caller's allreduce, keeps the host loop below.)
+int conjgrad_pressure_dev(sod_gpu_ctx *c, const float *Rp0, float *R, int maxIter, double tol, int *iters,
+                          double *res_rel) {
+  int rc;
+  if ((rc = ensure_diag(c)) || (rc = ensure_cg32(c)) || (rc = ensure_cg_loop(c))) return rc;
+  auto &G = c->cg;
+  const long long N = c->npoin;
+  const cudaStream_t st = c->stream;
+  lap<float>(c, Rp0, G.q32);
+  k_cg_start32<<<cg_blocks(N, CG_U), CG_THREADS, 0, st>>>(N, R, G.q32, G.diag, tol, G.x32, G.r32, G.p32, G.z032, G.S,
+                                                          G.gpart, G.ticket);
+  const int batch_max = 20;  // the solver's usual maxIter; launches after convergence return at once
+  int it = 0;
+  while (it < maxIter) {
+    const int it0 = it, nbat = std::min(batch_max, maxIter - it);
+    for (int k = 0; k < nbat; ++k)
+      dispatch(c, [&](auto L) {
+        using LL = decltype(L);
+        launch_pdl(k_lap_elem<LL::P_, LL::EPB, float, true>, LL::grid(c->nelem), LL::TPB, 0, st, c->md(), G.p32,
+                   (float *)c->slotsB, &G.S->status, G.z032, &G.S->beta);
+        launch_pdl(k_cg_q<float>, cg_blocks(N, CG_QU), CG_THREADS, 0, st, c->md(), (const float *)c->slotsB, G.p32,
+                   G.q32, G.S, G.gpart, G.ticket, G.z032);
+        launch_pdl(k_cg_update32, cg_blocks(N, CG_U), CG_THREADS, 0, st, N, G.p32, G.q32, G.diag, G.x32, G.r32,
+                   G.z032, G.S, G.gpart, G.ticket);
+        return 0;
+      });
+    CUDA_TRY(cudaMemcpyAsync(G.S_h, G.S, sizeof(CgScal), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    it = G.S_h->iter;
+    if (G.S_h->status == 3) return fail(SOD_GPU_ENONFINITE, "non-finite residual in pressure CG");
+    if (G.S_h->status == 1) break;
+    if (it == it0) return fail(SOD_GPU_ECUDA, "pressure CG did not advance");
+  }
+  // R = x0 + x on every node (x is zero off the working nodes)
+  k_add_all<float><<<nblk(N, 256), 256, 0, st>>>(N, Rp0, G.x32, R);
+  if (iters) *iters = it;
+  if (res_rel) *res_rel = G.S_h->bnorm > 0 ? std::sqrt(G.S_h->rr) / G.S_h->bnorm : 0.0;
+  return c->finish();
+}
+
+}  // namespace
+
+extern "C" {
+
 int sod_gpu_conjgrad_pressure(sod_gpu_ctx *c, const float *Rp0, float *R, int maxIter, double tol, int *iters,
                               double *res_rel) {
   if (!c || !Rp0 || !R || maxIter < 1) return fail(SOD_GPU_EINVAL, "bad argument");
+  if (!c->halo.on) return conjgrad_pressure_dev(c, Rp0, R, maxIter, tol, iters, res_rel);
   int rc;
   if ((rc = ensure_diag(c)) || (rc = ensure_cg32(c))) return rc;
   auto &G = c->cg;
@@ -405,23 +460,21 @@ int sod_gpu_pressure_solve(sod_gpu_ctx *c, const double *b_in, double *x, const 
       using LL = decltype(L);
       constexpr int P = LL::P_;
       // the search direction p = z + beta p is formed inside these two
-      k_lap_elem<P, LL::EPB, double, true><<<LL::grid(c->nelem), LL::TPB, 0, st>>>(
-          md, G.p, (double *)c->slotsB, &G.S->status, G.z0, &G.S->beta);
-      k_cg_q<true><<<cg_blocks(c->npoin, 2), CG_THREADS, 0, st>>>(md, (const double *)c->slotsB, G.p, G.q, G.S,
-                                                                  G.gpart, G.ticket, G.z0);
+      launch_pdl(k_lap_elem<P, LL::EPB, double, true>, LL::grid(c->nelem), LL::TPB, 0, st, md, G.p,
+                 (double *)c->slotsB, &G.S->status, G.z0, &G.S->beta);
+      launch_pdl(k_cg_q<double>, cg_blocks(c->npoin, CG_QU), CG_THREADS, 0, st, md, (const double *)c->slotsB, G.p, G.q, G.S,
+                 G.gpart, G.ticket, G.z0);
       if (kind == 0) {
-        k_cg_update<true><<<cg_blocks(nw, CG_U), CG_THREADS, 0, st>>>(nw, c->lpoin_w, G.p, G.q, G.Minv, x, G.r, G.z0,
-                                                                     G.S, G.hist, CG_HIST, G.gpart, G.ticket);
+        launch_pdl(k_cg_update<true>, cg_blocks(c->npoin, CG_U), CG_THREADS, 0, st, c->npoin, G.p, G.q, G.Minv, x,
+                   G.r, G.z0, G.S, G.hist, CG_HIST, G.gpart, G.ticket, nullptr);
       } else {
         using D = NetDims<P>;
-        k_cg_update<false><<<cg_blocks(nw, CG_U), CG_THREADS, 0, st>>>(nw, c->lpoin_w, G.p, G.q, G.Minv, x, G.r,
-                                                                      G.z0, G.S, G.hist, CG_HIST, G.gpart,
-                                                                      G.ticket, NT.Dh, NT.uf);
-        k_patch_apply_tc<P><<<tc_grid<P>(c->nelem), TC_THREADS, TcDims<P>::smem(), st>>>(
-            c->nelem, NT.pt, NT.pos, NT.uf, NT.params, NT.gains, c->slotsB, &G.S->status);
-        k_cg_patch_z<<<cg_blocks(c->npoin, CG_U), CG_THREADS, 0, st>>>(c->npoin, NT.pptr, c->slotsB, G.r, NT.Dh,
-                                                                       NT.params, D::O_ALPHA, G.z0, G.S, G.gpart,
-                                                                       G.ticket);
+        launch_pdl(k_cg_update<false>, cg_blocks(c->npoin, CG_U), CG_THREADS, 0, st, c->npoin, G.p, G.q, NT.Dh, x,
+                   G.r, G.z0, G.S, G.hist, CG_HIST, G.gpart, G.ticket, NT.uf);
+        launch_pdl(k_patch_apply_tc<P>, tc_grid<P>(c->nelem), TC_THREADS, TcDims<P>::smem(), st, c->nelem, NT.pt,
+                   NT.pos, NT.uf, NT.params, NT.gains, c->slotsB, &G.S->status);
+        launch_pdl(k_cg_patch_z, cg_blocks(c->npoin, CG_U), CG_THREADS, 0, st, c->npoin, NT.pptr, c->slotsB, G.r,
+                   NT.Dh, NT.params, D::O_ALPHA, G.z0, G.S, G.gpart, G.ticket);
       }
       return 0;
     });

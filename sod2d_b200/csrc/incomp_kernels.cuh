@@ -7,6 +7,24 @@
 
 namespace sod {
 
+// Row (or column) c of the 1-D derivative matrix in V.
+template <int P>
+__device__ __forceinline__ void load_d(const MeshDev &m, int c, bool col, double (&D)[P + 1]) {
+  const double2 *r = reinterpret_cast<const double2 *>(m.D64 + 8 * (c + (col ? P + 1 : 0)));
+#pragma unroll
+  for (int q = 0; q < (P + 1) / 2; ++q) {
+    const double2 v = r[q];
+    D[2 * q] = v.x;
+    D[2 * q + 1] = v.y;
+  }
+  if (P == 4) D[4] = r[2].x;
+}
+template <int P>
+__device__ __forceinline__ void load_d(const MeshDev &m, int c, bool col, float (&D)[P + 1]) {
+#pragma unroll
+  for (int q = 0; q <= P; ++q) D[q] = col ? m.Dnat[q * (P + 1) + c] : m.Dnat[c * (P + 1) + q];
+}
+
 // ---- Laplacian: ResP = sum_e int grad N . grad p  (mod_operators.f90:16-112)
 // One thread per Gauss point; V = float (reference arithmetic) or double.
 // Writes one V per element node into slots (width 1), element-ordered.
@@ -14,39 +32,53 @@ namespace sod {
 // z + beta p, formed on the fly from z, the previous p and *beta (the
 // update p = z + beta p itself is stored by k_cg_q), and the slots are
 // written node-sorted (slot_pos) for k_cg_q's contiguous sums.
+// The chain connectivity -> operand -> derivative bounds it, not bandwidth.
+// So everything that depends on no other kernel -- J^-1, weight, node, slot
+// position -- is requested first, before the programmatic wait and the
+// staging barrier, and the derivative matrix comes in V (converting its FP32
+// rows and columns took 24 of 34 conversions per point on a pipe of 16 per
+// clock and SM).
 template <int P, int EPB, class V, bool DIR = false>
 __global__ void __launch_bounds__(EPB *Cfg<P>::NT)
 k_lap_elem(MeshDev m, const V *__restrict__ p, V *__restrict__ slots, const int *__restrict__ stop = nullptr,
-           const V *__restrict__ z = nullptr, const V *__restrict__ beta = nullptr) {
+           const V *__restrict__ z = nullptr, const double *__restrict__ beta = nullptr) {
   constexpr int N1 = Cfg<P>::N1, N = Cfg<P>::N, NT = Cfg<P>::NT;
-  if (stop && *stop) return;
   __shared__ V sm[EPB][4][N];
   const int el = threadIdx.x / NT, t = threadIdx.x % NT;
   const long long e = (long long)blockIdx.x * EPB + el;
   const bool active = (e < m.nelem) && (t < N);
+  int n = 0, pos = 0;
+  float G[10];
   if (active) {
-    const int n = m.conn[e * N + t];
+    n = m.conn[e * N + t];
+    pos = DIR ? m.slot_pos[e * N + t] : 0;
+    const float *g = m.geo + e * 10 * N + t;
+#pragma unroll
+    for (int c = 0; c < 10; ++c) G[c] = g[c * N];
+  }
+  const int i = t % N1, j = (t / N1) % N1, k = t / (N1 * N1);
+  pdl_wait();
+  pdl_trigger();
+  if (stop && *stop) return;
+  if (active) {
     if (DIR) {
-      const V bt = *beta;
+      const V bt = (V)*beta;
       sm[el][0][t] = z[n] + bt * p[n];
     } else {
       sm[el][0][t] = p[n];
     }
   }
   __syncthreads();
-  const int i = t % N1, j = (t / N1) % N1, k = t / (N1 * N1);
   V C0 = 0, C1 = 0, C2 = 0;
-  V Di[N1], Dj[N1], Dk[N1];
   if (active) {
-#pragma unroll
-    for (int s = 0; s < N1; ++s) {
-      Di[s] = (V)m.Dnat[i * N1 + s]; Dj[s] = (V)m.Dnat[j * N1 + s]; Dk[s] = (V)m.Dnat[k * N1 + s];
-    }
-    const float *g = m.geo + e * 10 * N + t;
+    V Di[N1], Dj[N1], Dk[N1];
+    load_d<P>(m, i, false, Di);
+    load_d<P>(m, j, false, Dj);
+    load_d<P>(m, k, false, Dk);
     V He[9];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) He[c] = (V)g[c * N];
-    const V gv = (V)g[9 * N];
+    for (int c = 0; c < 9; ++c) He[c] = (V)G[c];
+    const V gv = (V)G[9];
     const V *f = sm[el][0];
     V g0 = 0, g1 = 0, g2 = 0;
 #pragma unroll
@@ -62,20 +94,23 @@ k_lap_elem(MeshDev m, const V *__restrict__ p, V *__restrict__ slots, const int 
     C0 = gv * (He[0] * gP[0] + He[1] * gP[1] + He[2] * gP[2]);
     C1 = gv * (He[3] * gP[0] + He[4] * gP[1] + He[5] * gP[2]);
     C2 = gv * (He[6] * gP[0] + He[7] * gP[1] + He[8] * gP[2]);
+    sm[el][1][t] = C0; sm[el][2][t] = C1; sm[el][3][t] = C2;
   }
   __syncthreads();
-  if (active) { sm[el][1][t] = C0; sm[el][2][t] = C1; sm[el][3][t] = C2; }
-  __syncthreads();
   if (!active) return;
+  V Di[N1], Dj[N1], Dk[N1];
+  load_d<P>(m, i, true, Di);
+  load_d<P>(m, j, true, Dj);
+  load_d<P>(m, k, true, Dk);
   V acc = 0;
 #pragma unroll
   for (int s = 0; s < N1; ++s) {
     const int mm = ref_order<P>(s);
-    acc += (V)m.Dnat[mm * N1 + i] * sm[el][1][mm + N1 * j + N1 * N1 * k];
-    acc += (V)m.Dnat[mm * N1 + j] * sm[el][2][i + N1 * mm + N1 * N1 * k];
-    acc += (V)m.Dnat[mm * N1 + k] * sm[el][3][i + N1 * j + N1 * N1 * mm];
+    acc += Di[mm] * sm[el][1][mm + N1 * j + N1 * N1 * k];
+    acc += Dj[mm] * sm[el][2][i + N1 * mm + N1 * N1 * k];
+    acc += Dk[mm] * sm[el][3][i + N1 * j + N1 * N1 * mm];
   }
-  slots[DIR ? (long long)m.slot_pos[e * N + t] : e * N + t] = acc;
+  slots[DIR ? (long long)pos : e * N + t] = acc;
 }
 
 // Scalar-slot assembly out(p) = scale * sum(slots of p); float sums are
@@ -325,12 +360,14 @@ struct CgScal {
   double pq;     // p . A p
   double alpha, beta;
   double rr;     // ||r||^2 after the last update
-  double thr2;   // (tol ||b||)^2
+  double thr2;   // (tol ||b||)^2; in the FP32 solve tol ||b||
+  double bnorm;  // ||b|| of the FP32 solve
   int iter;      // iterations done in this solve
   int status;    // 0 running, 1 converged (recursive residual), 2 breakdown, 3 non-finite
 };
 
-constexpr int CG_THREADS = 256, CG_U = 4;
+// threads per block; nodes per thread of the update and assembly kernels
+constexpr int CG_THREADS = 256, CG_U = 4, CG_QU = 2;
 
 // Node loops of the CG kernels handle several nodes per thread and issue all
 // their loads before any store, so that each thread keeps several memory
@@ -367,14 +404,20 @@ __device__ bool grid_sum(double (&v)[ND], double *__restrict__ part, unsigned *t
   __syncthreads();
   if (!last) return false;
   __threadfence();
+  double s[ND];  // all values' loads in flight at once, one barrier
+#pragma unroll
+  for (int d = 0; d < ND; ++d) s[d] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+    for (int d = 0; d < ND; ++d) s[d] += __ldcg(part + d * gridDim.x + b);
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += __ldcg(part + d * gridDim.x + b);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __syncthreads();
-    if (lane == 0) sh[d][warp] = s;
-    __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) s[d] += __shfl_xor_sync(0xffffffffu, s[d], o);
+    if (lane == 0) sh[d][warp] = s[d];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
     double t = 0.0;
     for (int w = 0; w < nw; ++w) t += sh[d][w];
     tot[d] = t;
@@ -383,62 +426,66 @@ __device__ bool grid_sum(double (&v)[ND], double *__restrict__ part, unsigned *t
   return true;
 }
 
-// q = assembled Laplacian slots (Kahan, as k_gather1) with the p.q partials;
-// the last block sets alpha = rz / pq.  DIR: the slots are node-sorted
-// (k_lap_elem<DIR>), and the new search direction p = z + beta p is formed
-// and stored here for every node with slots (the working nodes).
-template <bool DIR = false>
+// q = assembled Laplacian slots (Kahan, as k_gather1; node-sorted by
+// k_lap_elem<DIR>) with the p.q partials; the last block sets alpha = rz / pq.
+// The new search direction p = z + beta p is formed and stored here for every
+// node with slots (the working nodes).  V = float: the reference's FP32
+// solve, whose alpha is rounded to FP32 and taken as it comes.
+template <class V>
 __global__ void __launch_bounds__(CG_THREADS)
-k_cg_q(MeshDev m, const double *__restrict__ slots, double *__restrict__ p, double *__restrict__ q,
-       CgScal *S, double *__restrict__ part, unsigned *ticket, const double *__restrict__ z = nullptr) {
-  if (S->status) return;
-  constexpr int U = 2, MS = 8;  // nodes per thread, slots loaded ahead per node
-  const double bt = DIR ? S->beta : 0.0;
-  double v[1] = {0.0};
-  for (long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x; base < m.npoin;
-       base += (long long)gridDim.x * blockDim.x * U) {
-    int b[U], en[U];
-    double pn[U];
+k_cg_q(MeshDev m, const V *__restrict__ slots, V *__restrict__ p, V *__restrict__ q, CgScal *S,
+       double *__restrict__ part, unsigned *ticket, const V *__restrict__ z) {
+  constexpr int U = CG_QU, MS = 8;  // nodes per thread, slots loaded ahead per node
+  const long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
+  int b[U], en[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long n = base + (long long)u * blockDim.x;
-      b[u] = en[u] = 0;
-      pn[u] = 0.0;
-      if (n < m.npoin) {
-        b[u] = m.slot_ptr[n]; en[u] = m.slot_ptr[n + 1]; pn[u] = p[n];
-        if (DIR) pn[u] = z[n] + bt * pn[u];
+  for (int u = 0; u < U; ++u) {
+    const long long n = base + (long long)u * blockDim.x;
+    b[u] = en[u] = 0;
+    if (n < m.npoin) { b[u] = m.slot_ptr[n]; en[u] = m.slot_ptr[n + 1]; }
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (S->status) return;
+  const V bt = (V)S->beta;
+  double v[1] = {0.0};
+  V pn[U], zn[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long n = base + (long long)u * blockDim.x;
+    pn[u] = zn[u] = 0;
+    if (b[u] != en[u]) { pn[u] = p[n]; zn[u] = z[n]; }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long n = base + (long long)u * blockDim.x;
+    V sum = 0, cmp = 0;
+    for (int s0 = b[u]; s0 < en[u]; s0 += MS) {
+      V y[MS];
+#pragma unroll
+      for (int k = 0; k < MS; ++k) y[k] = s0 + k < en[u] ? slots[s0 + k] : (V)0;
+#pragma unroll
+      for (int k = 0; k < MS; ++k) {
+        if (s0 + k >= en[u]) break;
+        const V yy = y[k] - cmp;
+        const V tt = sum + yy;
+        cmp = (tt - sum) - yy;
+        sum = tt;
       }
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long n = base + (long long)u * blockDim.x;
-      if (n >= m.npoin) continue;
-      if (DIR && b[u] != en[u]) p[n] = pn[u];
-      double sum = 0.0, cmp = 0.0;
-      for (int s0 = b[u]; s0 < en[u]; s0 += MS) {
-        int id[MS];
-        double y[MS];
-#pragma unroll
-        for (int k = 0; k < MS; ++k) id[k] = s0 + k < en[u] ? (DIR ? s0 + k : m.slot_idx[s0 + k]) : -1;
-#pragma unroll
-        for (int k = 0; k < MS; ++k) y[k] = id[k] >= 0 ? slots[id[k]] : 0.0;
-#pragma unroll
-        for (int k = 0; k < MS; ++k) {
-          if (id[k] < 0) break;
-          const double yy = y[k] - cmp;
-          const double tt = sum + yy;
-          cmp = (tt - sum) - yy;
-          sum = tt;
-        }
-      }
+    if (b[u] != en[u]) {
+      pn[u] = zn[u] + bt * pn[u];
+      p[n] = pn[u];
       q[n] = sum;
-      if (b[u] != en[u]) v[0] += pn[u] * sum;
+      v[0] += (double)(pn[u] * sum);
     }
   }
   double tot[1];
   if (grid_sum<1>(v, part, ticket, tot) && threadIdx.x == 0) {
     S->pq = tot[0];
-    if (!isfinite(tot[0])) {
+    if (sizeof(V) == 4) {
+      S->alpha = (double)(float)(S->rz / tot[0]);
+    } else if (!isfinite(tot[0])) {
       S->status = 3;
     } else if (!(tot[0] > 0.0)) {
       S->status = 2;
@@ -448,54 +495,52 @@ k_cg_q(MeshDev m, const double *__restrict__ slots, double *__restrict__ p, doub
   }
 }
 
-// x += alpha p ; r -= alpha q ; with JAC also z = Minv r (reading the old z),
-// otherwise, when uf is given, uf = (float)(Dh r); the last block records
-// ||r||^2, detects convergence and, with JAC, sets the Polak-Ribiere
-// beta = r.(z - z_old) / rz_old.
+// x += alpha p ; r -= alpha q ; with JAC also z = Minv r (the old z is Minv
+// times the old r again), otherwise uf = (float)(Minv r) with Minv = D^-1/2;
+// the last block records ||r||^2, detects convergence and, with JAC, sets
+// the Polak-Ribiere beta = r.(z - z_old) / rz_old.  Runs over all nodes in
+// order, with no index loads: Minv is 0 off the working nodes, which are
+// left alone.
 template <bool JAC>
 __global__ void __launch_bounds__(CG_THREADS)
-k_cg_update(int npoin_w, const int *__restrict__ lpoin_w, const double *__restrict__ p,
-            const double *__restrict__ q, const double *__restrict__ Minv, double *__restrict__ x,
-            double *__restrict__ r, double *__restrict__ z, CgScal *S, double *__restrict__ hist, int hist_cap,
-            double *__restrict__ part, unsigned *ticket, const double *__restrict__ Dh = nullptr,
-            float *__restrict__ uf = nullptr) {
-  if (S->status) return;
+k_cg_update(long long npoin, const double *__restrict__ p, const double *__restrict__ q,
+            const double *__restrict__ Minv, double *__restrict__ x, double *__restrict__ r, double *__restrict__ z,
+            CgScal *S, double *__restrict__ hist, int hist_cap, double *__restrict__ part, unsigned *ticket,
+            float *__restrict__ uf) {
   constexpr int U = CG_U;
+  const long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
+  double mv[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + (long long)u * blockDim.x;
+    mv[u] = i < npoin ? Minv[i] : 0.0;
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (S->status) return;
   const double a = S->alpha;
   double v[3] = {0.0, 0.0, 0.0};
-  for (long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x; base < npoin_w;
-       base += (long long)gridDim.x * blockDim.x * U) {
-    int id[U];
-    double pv[U], qv[U], xv[U], rv[U], mv[U], zv[U];
+  double pv[U], qv[U], xv[U], rv[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long t = base + (long long)u * blockDim.x;
-      id[u] = t < npoin_w ? lpoin_w[t] : -1;
-    }
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + (long long)u * blockDim.x;
+    if (i < npoin) { pv[u] = p[i]; qv[u] = q[i]; xv[u] = x[i]; rv[u] = r[i]; }
+  }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (id[u] < 0) continue;
-      const int i = id[u];
-      pv[u] = p[i]; qv[u] = q[i]; xv[u] = x[i]; rv[u] = r[i];
-      if (JAC) { mv[u] = Minv[i]; zv[u] = z[i]; }
-      if (!JAC && uf) mv[u] = Dh[i];
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (id[u] < 0) continue;
-      const int i = id[u];
-      x[i] = xv[u] + a * pv[u];
-      const double rn = rv[u] - a * qv[u];
-      r[i] = rn;
-      v[0] += rn * rn;
-      if (JAC) {
-        const double zn = rn * mv[u];
-        z[i] = zn;
-        v[1] += rn * zn;
-        v[2] += rn * zv[u];
-      } else if (uf) {
-        uf[i] = (float)(mv[u] * rn);  // D^-1/2 r for the learned preconditioner
-      }
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + (long long)u * blockDim.x;
+    if (mv[u] == 0.0) continue;
+    x[i] = xv[u] + a * pv[u];
+    const double rn = rv[u] - a * qv[u];
+    r[i] = rn;
+    v[0] += rn * rn;
+    if (JAC) {
+      const double zn = rn * mv[u];
+      z[i] = zn;
+      v[1] += rn * zn;
+      v[2] += rn * (rv[u] * mv[u]);
+    } else {
+      uf[i] = (float)(mv[u] * rn);  // D^-1/2 r for the learned preconditioner
     }
   }
   double tot[3];
@@ -516,6 +561,92 @@ k_cg_update(int npoin_w, const int *__restrict__ lpoin_w, const double *__restri
   }
 }
 
+// The same update of the reference's FP32 solve (mod_solver_incomp.f90:
+// 395-440): z = r / M with M the Laplacian's diagonal (0 off the working
+// nodes), FP64 sums of FP32 products, beta rounded to FP32, converged when
+// ||r|| < thr2 (here tol ||b||).
+static __global__ void __launch_bounds__(CG_THREADS)
+k_cg_update32(long long npoin, const float *__restrict__ p, const float *__restrict__ q, const float *__restrict__ M,
+              float *__restrict__ x, float *__restrict__ r, float *__restrict__ z, CgScal *S,
+              double *__restrict__ part, unsigned *ticket) {
+  constexpr int U = CG_U;
+  const long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
+  float mv[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + (long long)u * blockDim.x;
+    mv[u] = i < npoin ? M[i] : 0.f;
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (S->status) return;
+  const float a = (float)S->alpha;
+  double v[3] = {0.0, 0.0, 0.0};
+  float pv[U], qv[U], xv[U], rv[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + (long long)u * blockDim.x;
+    if (mv[u] != 0.f) { pv[u] = p[i]; qv[u] = q[i]; xv[u] = x[i]; rv[u] = r[i]; }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + (long long)u * blockDim.x;
+    if (mv[u] == 0.f) continue;
+    x[i] = xv[u] + a * pv[u];
+    const float rn = rv[u] - a * qv[u], zn = rn / mv[u], zo = rv[u] / mv[u];
+    r[i] = rn;
+    z[i] = zn;
+    v[0] += (double)(rn * rn);
+    v[1] += (double)(rn * zn);
+    v[2] += (double)(rn * (zn - zo));
+  }
+  double tot[3];
+  if (grid_sum<3>(v, part, ticket, tot) && threadIdx.x == 0) {
+    S->iter += 1;
+    S->rr = tot[0];
+    if (!isfinite(tot[0])) {
+      S->status = 3;
+    } else if (sqrt(tot[0]) < S->thr2) {
+      S->status = 1;
+    }
+    S->beta = (double)(float)(tot[2] / S->rz);
+    S->rz = tot[1];
+  }
+}
+
+// Start of that solve: r = R - A x0 (Ax0 in q), z = r / M, x = p = 0 on
+// every node; the last block sets the scalars.
+static __global__ void __launch_bounds__(CG_THREADS)
+k_cg_start32(long long npoin, const float *__restrict__ R, const float *__restrict__ q, const float *__restrict__ M,
+             double tol, float *__restrict__ x, float *__restrict__ r, float *__restrict__ p, float *__restrict__ z,
+             CgScal *S, double *__restrict__ part, unsigned *ticket) {
+  constexpr int U = CG_U;
+  const long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
+  double v[2] = {0.0, 0.0};
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = base + (long long)u * blockDim.x;
+    if (i >= npoin) continue;
+    const float mv = M[i];
+    const float rn = mv != 0.f ? R[i] - q[i] : 0.f, zn = mv != 0.f ? rn / mv : 0.f;
+    x[i] = 0.f;
+    p[i] = 0.f;
+    r[i] = rn;
+    z[i] = zn;
+    v[0] += (double)(rn * rn);
+    v[1] += (double)(rn * zn);
+  }
+  double tot[2];
+  if (grid_sum<2>(v, part, ticket, tot) && threadIdx.x == 0) {
+    S->rz = tot[1];
+    S->rr = tot[0];
+    S->bnorm = sqrt(tot[0]);
+    S->thr2 = tol * S->bnorm;
+    S->alpha = S->beta = 0.0;
+    S->iter = S->status = 0;
+  }
+}
+
 // Learned preconditioner: z(n) = D^-1/2(n) (exp(alpha) D^-1/2(n) r(n) + sum of
 // the node's contributions, stored contiguously from pptr[n]) (as
 // k_patch_gather_perm), with the partials r.z and r.z_old; the last block
@@ -524,40 +655,43 @@ static __global__ void __launch_bounds__(CG_THREADS)
 k_cg_patch_z(long long npoin, const int *__restrict__ pptr, const float *__restrict__ ctr,
              const double *__restrict__ r, const double *__restrict__ Dh, const float *__restrict__ prm, int o_alpha,
              double *__restrict__ z, CgScal *S, double *__restrict__ part, unsigned *ticket) {
-  if (S->status) return;
   constexpr int U = CG_U;
+  const long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
+  int b[U], en[U];
+  double dv[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long n = base + (long long)u * blockDim.x;
+    b[u] = en[u] = 0;
+    dv[u] = 0.0;
+    if (n < npoin) { b[u] = pptr[n]; en[u] = pptr[n + 1]; dv[u] = Dh[n]; }
+  }
   const double gam = exp((double)prm[o_alpha]);
-  double v[2] = {0.0, 0.0};
-  for (long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x; base < npoin;
-       base += (long long)gridDim.x * blockDim.x * U) {
-    int b[U], en[U];
-    double dv[U], rv[U], zo[U];
+  pdl_wait();
+  pdl_trigger();
+  if (S->status) return;
+  double v[2] = {0.0, 0.0}, rv[U], zo[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long n = base + (long long)u * blockDim.x;
-      b[u] = en[u] = 0;
-      if (n < npoin) {
-        b[u] = pptr[n]; en[u] = pptr[n + 1];
-        dv[u] = Dh[n]; rv[u] = r[n]; zo[u] = z[n];
-      }
+  for (int u = 0; u < U; ++u) {
+    const long long n = base + (long long)u * blockDim.x;
+    if (b[u] != en[u]) { rv[u] = r[n]; zo[u] = z[n]; }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (b[u] == en[u]) continue;
+    const long long n = base + (long long)u * blockDim.x;
+    double acc = 0.0;
+    for (int s0 = b[u]; s0 < en[u]; s0 += 8) {
+      float y[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) y[k] = s0 + k < en[u] ? ctr[s0 + k] : 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc += (double)y[k];
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (b[u] == en[u]) continue;
-      const long long n = base + (long long)u * blockDim.x;
-      double acc = 0.0;
-      for (int s0 = b[u]; s0 < en[u]; s0 += 8) {
-        float y[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) y[k] = s0 + k < en[u] ? ctr[s0 + k] : 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc += (double)y[k];
-      }
-      const double zn = dv[u] * (gam * dv[u] * rv[u] + acc);
-      z[n] = zn;
-      v[0] += rv[u] * zn;
-      v[1] += rv[u] * zo[u];
-    }
+    const double zn = dv[u] * (gam * dv[u] * rv[u] + acc);
+    z[n] = zn;
+    v[0] += rv[u] * zn;
+    v[1] += rv[u] * zo[u];
   }
   double tot[2];
   if (grid_sum<2>(v, part, ticket, tot) && threadIdx.x == 0) {

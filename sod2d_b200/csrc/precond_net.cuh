@@ -274,7 +274,6 @@ k_patch_apply_tc(long long nelem, const int *__restrict__ pt, const int *__restr
   using D = NetDims<P>;
   using T = TcDims<P>;
   constexpr int NP = D::NP, KP = T::KP, K = NET_K, NT2 = KP / 8, KS = KP / 8, KC = T::KC;
-  if (stop && *stop) return;
   extern __shared__ __align__(16) float smem[];
   float *B1 = smem, *B2 = B1 + K * T::S1;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -286,6 +285,9 @@ k_patch_apply_tc(long long nelem, const int *__restrict__ pt, const int *__restr
     B2[j * T::S2 + kpair_pos(k)] = b;
   }
   __syncthreads();
+  pdl_wait();  // the parameters do not change during a solve: staged while the update kernel ends
+  pdl_trigger();
+  if (stop && *stop) return;
   const int g = lane >> 2, t = lane & 3;
   const long long ngroups = (nelem + 15) / 16;
   // groups dealt round-robin over the blocks, so that every SM holds the

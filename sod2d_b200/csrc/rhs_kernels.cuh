@@ -42,6 +42,15 @@ struct Phys {
   float twoThirds;
 };
 
+// Programmatic dependent launch: a kernel started with launch_pdl (ctx.cuh)
+// may begin while the kernel before it in the stream still runs.  What it
+// reads or writes of earlier kernels' results comes after pdl_wait(), which
+// returns when they are complete and visible; before it, only arrays that no
+// kernel of the stream's current work writes (the mesh).  pdl_trigger() lets
+// the next such kernel begin.  Both do nothing in an ordinary launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 struct MeshDev {
   int nelem, npoin, npoin_w;
   const int *conn;      // [E][N]
@@ -49,6 +58,7 @@ struct MeshDev {
   const float *Dnat;    // [N1][N1]
   const float *Drot;    // [2][N1][8]: rows, then columns, of Dnat rotated to start at the
                         // diagonal: D[c][(c+s) % N1], D[(c+s) % N1][c], s = 0..P
+  const double *D64;    // [2][N1][8]: rows, then columns, of Dnat in FP64
   const int *lpoin_w;   // 0-based
   const float *invMl;   // [npoin]
   const int *slot_ptr;  // [npoin+1]

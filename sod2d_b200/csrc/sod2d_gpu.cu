@@ -54,10 +54,13 @@ int sod_gpu_init(const sod_mesh_t *mesh, const sod_phys_t *phys, sod_gpu_ctx **o
     for (int ii = 0; ii < N1; ++ii) D[mrow * N1 + nat_of(P, ii)] = mesh->dlxigp_ip[a + (long long)N * (0 + 3 * ii)];
   }
   std::vector<float> Drot(2 * N1 * 8, 0.f);
+  std::vector<double> D64(2 * N1 * 8, 0.0);
   for (int a = 0; a < N1; ++a)
     for (int s = 0; s < N1; ++s) {
       Drot[8 * a + s] = D[a * N1 + (a + s) % N1];
       Drot[8 * (N1 + a) + s] = D[((a + s) % N1) * N1 + a];
+      D64[8 * a + s] = D[a * N1 + s];
+      D64[8 * (N1 + a) + s] = D[s * N1 + a];
     }
   std::vector<int> conn((size_t)E * N);
   std::vector<float> geo((size_t)E * 10 * N);
@@ -99,7 +102,8 @@ int sod_gpu_init(const sod_mesh_t *mesh, const sod_phys_t *phys, sod_gpu_ctx **o
   int rc = 0;
   if ((rc = c->upload(&c->conn, conn.data(), conn.size())) || (rc = c->upload(&c->geo, geo.data(), geo.size())) ||
       (rc = c->upload(&c->Dnat, D.data(), D.size())) ||
-      (rc = c->upload(&c->Drot, Drot.data(), Drot.size())) || (rc = c->upload(&c->lpoin_w, lw.data(), lw.size())) ||
+      (rc = c->upload(&c->Drot, Drot.data(), Drot.size())) ||
+      (rc = c->upload(&c->D64, D64.data(), D64.size())) || (rc = c->upload(&c->lpoin_w, lw.data(), lw.size())) ||
       (rc = c->upload(&c->slot_ptr, cnt.data(), cnt.size())) ||
       (rc = c->upload(&c->slot_idx, slot_idx.data(), slot_idx.size())) ||
       (rc = c->upload(&c->slot_pos, slot_pos.data(), slot_pos.size())) ||
