@@ -323,7 +323,7 @@ struct RhsArgs {
 // Staged fields of pass B, one entry per element node:
 //   CONV+DIFF (conserved inputs): float4 (u0,u1,u2,H) and (rho,T,p,0)
 //   CONV only : float2 pairs (u0,u1) (u2,rho) (q0,q1) (q2,p) (H,rho*H)
-//   DIFF only : float2 pairs (u0,u1) (u2,rho) (T,0)
+//   DIFF only : float2 pairs (u0,u1) (u2,rho), then T
 // With the conserved inputs q = rho u, so every split-form term is a product
 // of staged values and one product per line node serves momentum, mass and
 // energy (FLUX2 below).  Instruction issue bounds this kernel: that form
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(EPB *Cfg<P>::NT, SOD_RHS_THREADS_PER_SM / (EPB
 k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
   using L = RhsPlan<P, EPB, MODE, IN>;
   constexpr int N1 = L::N1, N = L::N, NT = L::NT, NTB = L::NTB, NC = L::NC, SMF = L::SMF, PB_T = L::PB_T;
-  constexpr bool CONV = L::CONV, DIFF = L::DIFF, LPS = L::LPS, FLUX2 = L::FLUX2, ROT = P == 3;
+  constexpr bool CONV = L::CONV, DIFF = L::DIFF, LPS = L::LPS, FLUX2 = L::FLUX2, ROT = P == 3 && DIFF;
   static_assert(FLUX2 || !(CONV && DIFF), "convection with diffusion runs on the conserved state");
   extern __shared__ __align__(16) float dsm[];
   const int tid = threadIdx.x, el = tid / NT, t = tid % NT;
@@ -548,7 +548,7 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
           sp[PB_Q2P * N + t] = make_float2(s.q2, s.p);
           sp[PB_HRH * N + t] = make_float2(H, rH);
         }
-        if (DIFF) sp[PB_T * N + t] = make_float2(s.T, 0.f);
+        if (DIFF) sf[2 * PB_T * N + t] = s.T;
       }
     }
     // staged pairs visible; every thread is done with the other stage
@@ -634,26 +634,27 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
             divG[3] = {0.f, 0.f, 0.f};
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const int cd = d == 0 ? i : (d == 1 ? j : k);
-        const int stride = d == 0 ? 1 : (d == 1 ? N1 : N1 * N1);
-        const int base = t - cd * stride;
         float Dd[N1];
-#pragma unroll
-        for (int q = 0; q < N1; ++q) Dd[q] = m.Dnat[cd * N1 + q];
+        load_row(d == 0 ? i : (d == 1 ? j : k), false, Dd);
         const float2 z2 = make_float2(0.f, 0.f);
-        float2 aU01 = z2, aU2R = z2, aQ01 = z2, aQ2P = z2, aHRH = z2, aT = z2;
+        float2 aU01 = z2, aU2R = z2, aQ01 = z2, aQ2P = z2, aHRH = z2;
+        float aT = 0.f;
         float2 aF0 = z2, aF1 = z2, aF2 = z2, aG0 = z2, aG1 = z2, aG2 = z2, aR0 = z2, aR1 = z2, aR2 = z2;
 #pragma unroll
-        for (int ss = 0; ss < N1; ++ss) {
-          const int mm = ref_order<P>(ss);  // the reference's 1-D summation order
-          const float2 D2 = make_float2(Dd[mm], Dd[mm]);
-          const int tm = base + mm * stride;
-          const float2 u01 = sp[PB_U01 * N + tm], u2r = sp[PB_U2R * N + tm];
+        for (int mm = 0; mm < N1; ++mm) {
+          const bool own = ROT && mm == P;  // the node itself comes from its registers
+          const float Dm = line_coef(Dd, mm);
+          const float2 D2 = make_float2(Dm, Dm);
+          const int tm = own ? t : line_node(d, mm);
+          const float2 u01 = own ? make_float2(s.u0, s.u1) : sp[PB_U01 * N + tm];
+          const float2 u2r = own ? make_float2(s.u2, s.rho) : sp[PB_U2R * N + tm];
           aU01 = __ffma2_rn(D2, u01, aU01);
           aU2R = __ffma2_rn(D2, u2r, aU2R);
-          if (DIFF) aT = __ffma2_rn(D2, sp[PB_T * N + tm], aT);
+          if (DIFF) aT = fmaf(Dm, own ? s.T : sf[2 * PB_T * N + tm], aT);
           if (CONV) {
-            const float2 q01 = sp[PB_Q01 * N + tm], q2p = sp[PB_Q2P * N + tm], hrh = sp[PB_HRH * N + tm];
+            const float2 q01 = own ? make_float2(s.q0, s.q1) : sp[PB_Q01 * N + tm];
+            const float2 q2p = own ? make_float2(s.q2, s.p) : sp[PB_Q2P * N + tm];
+            const float2 hrh = own ? make_float2(H, rH) : sp[PB_HRH * N + tm];
             aQ01 = __ffma2_rn(D2, q01, aQ01);
             aQ2P = __ffma2_rn(D2, q2p, aQ2P);
             aHRH = __ffma2_rn(D2, hrh, aHRH);
@@ -674,7 +675,7 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           gradRho[a] = gradRho[a] + h[a] * aU2R.y;
-          if (DIFF) gradT[a] = gradT[a] + h[a] * aT.x;
+          if (DIFF) gradT[a] = gradT[a] + h[a] * aT;
 #pragma unroll
           for (int b = 0; b < 3; ++b) gradU[a][b] = gradU[a][b] + h[b] * dU[a];
         }
