@@ -320,9 +320,10 @@ inline int num_sms() {
   return n;
 }
 
-// Launch with programmatic stream serialization (see pdl_wait).
+// Launch with programmatic stream serialization (see pdl_wait), or without.
 template <class... KA, class... A>
-inline cudaError_t launch_pdl(void (*k)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A &&...a) {
+inline cudaError_t launch_pdl_if(bool on, void (*k)(KA...), unsigned grid, unsigned block, size_t smem,
+                                 cudaStream_t st, A &&...a) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -332,11 +333,22 @@ inline cudaError_t launch_pdl(void (*k)(KA...), unsigned grid, unsigned block, s
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = on ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, k, static_cast<KA>(a)...);
+}
+template <class... KA, class... A>
+inline cudaError_t launch_pdl(void (*k)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A &&...a) {
+  return launch_pdl_if(true, k, grid, block, smem, st, a...);
 }
 
 inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }
+
+// Whether pass A and its gather start programmatically: up to 5 M element
+// nodes.  us per RHS with and without: 16^3 32.9 / 34.9, 24^3 82.7 / 85.8,
+// 32^3 190.4 / 194.6, 40^3 344.5 / 346.5, 48^3 593 / 594, 64^3 1485 / 1469
+// (the gather's waiting blocks take their place on the SMs before pass A has
+// ended).  Pass B never does (64^3: 1515 / 1484), the residual gather always.
+inline bool pdl_chain(const sod_gpu_ctx *c) { return (long long)c->nelem * c->N <= 5000000; }
 
 // ---- launch helpers templated on the element order --------------------
 
@@ -354,12 +366,8 @@ struct Launch {
   static unsigned grid(int nelem) { return nblk(nelem, EPB); }
 
   static void proj(sod_gpu_ctx *c, bool prim, const float *a0, const float *a1, const float *a2) {
-    if (prim)
-      k_proj<P, EPB_A, true><<<nblk(c->nelem, EPB_A), TPB_A, 0, c->stream>>>(c->md(), c->ph, c->phys.Rgas, a0, a1, a2,
-                                                                          c->slotsA);
-    else
-      k_proj<P, EPB_A, false><<<nblk(c->nelem, EPB_A), TPB_A, 0, c->stream>>>(c->md(), c->ph, c->phys.Rgas, a0, a1,
-                                                                           a2, c->slotsA);
+    launch_pdl_if(pdl_chain(c), prim ? k_proj<P, EPB_A, true> : k_proj<P, EPB_A, false>, nblk(c->nelem, EPB_A), TPB_A, 0, c->stream,
+               c->md(), c->ph, c->phys.Rgas, a0, a1, a2, c->slotsA);
   }
   // Persistent pass B: as many blocks as fit on the GPU at once (at most
   // one per element group), each walking the groups with a stride.
@@ -377,7 +385,7 @@ struct Launch {
     const unsigned g = (unsigned)std::min<long long>(groups, (long long)per_sm * num_sms());
     RhsArgs Ae = A;
     Ae.err = c->err_d;
-    k_rhs<P, EPB, MODE, IN><<<g, TPB, PL::BYTES, c->stream>>>(c->md(), c->ph, c->phys.Rgas, Ae, c->slotsB);
+    launch_pdl_if(false, k_rhs<P, EPB, MODE, IN>, g, TPB, PL::BYTES, c->stream, c->md(), c->ph, c->phys.Rgas, Ae, c->slotsB);
   }
 };
 
@@ -391,7 +399,7 @@ inline int dispatch(sod_gpu_ctx *c, F &&f) {
 inline void gather_proj_aos(sod_gpu_ctx *c) {
   OutPtrs none{};
   // 128-thread blocks: 1.642-1.650 ms per RHS against 1.660 with 256 (64^3 bench)
-  k_gather<12, 12, true><<<nblk(c->npoin, 128), 128, 0, c->stream>>>(c->md(), c->slotsA, c->proj12, none, 0, 1);
+  launch_pdl_if(pdl_chain(c), k_gather<12, 12, true>, nblk(c->npoin, 128), 128, 0, c->stream, c->md(), c->slotsA, c->proj12, none, 0, 1);
 }
 
 // Sum the view's components over the ranks that share each node (no-op
@@ -478,8 +486,8 @@ inline void gather_res(sod_gpu_ctx *c, float *Rmass, float *Rmom, float *Rener, 
   OutPtrs o{};
   const long long N = c->npoin;
   o.p[0] = Rmass; o.p[1] = Rener; o.p[2] = Rmom; o.p[3] = Rmom + N; o.p[4] = Rmom + 2 * N;
-  k_gather_sorted_res5<<<nblk(c->npoin, 128), 128, 0, c->stream>>>(c->md(), c->slotsB, (long long)c->nelem * c->N,
-                                                                    o, accumulate, invml);
+  launch_pdl(k_gather_sorted_res5, nblk(c->npoin, 128), 128, 0, c->stream, c->md(), c->slotsB,
+             (long long)c->nelem * c->N, o, accumulate, invml);
 }
 
 }  // namespace

@@ -224,13 +224,17 @@ k_proj(MeshDev m, Phys ph, float Rgas, const float *__restrict__ a0, const float
   const bool active = (e < m.nelem) && (t < N);
   const long long NP = m.npoin;
   float He[9], gv = 0.f;
-  if (active) {
-    const int node = m.conn[e * N + t];
-    // geometry loads issued before the staging barrier (independent of it)
+  int node = 0;
+  if (active) {  // mesh loads first: they depend on no earlier kernel
+    node = m.conn[e * N + t];
     const float *g = m.geo + e * 10 * N + t;
 #pragma unroll
     for (int c = 0; c < 9; ++c) He[c] = g[c * N];
     gv = g[9 * N];
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (active) {
     float rho, u0, u1, u2, T;
     if (PRIM) {  // a0 = rho, a1 = u(N,3), a2 = Tem
       rho = a0[node]; u0 = a1[node]; u1 = a1[node + NP]; u2 = a1[node + 2 * NP]; T = a2[node];
@@ -486,9 +490,12 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
   };
 
   long long g = blockIdx.x;
-  issue(dsm, g, node_of(g));
-  cp_async_commit();
+  const int nd_first = node_of(g);
   int nd_next = node_of(g + G);
+  pdl_wait();
+  pdl_trigger();
+  issue(dsm, g, nd_first);
+  cp_async_commit();
   for (int buf = 0; g < ngroups; g += G, buf ^= 1) {
     const float *cur = dsm + buf * L::STAGE;
     float *nxt = dsm + (buf ^ 1) * L::STAGE;
@@ -879,13 +886,16 @@ __global__ void k_gather(MeshDev m, const float *__restrict__ slots, float *__re
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= m.npoin) return;
   constexpr int MS = W >= 12 ? 1 : 4;  // slots whose loads are issued together (registers permitting)
+  const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
+  const float sc = use_invMl ? m.invMl[p] : 1.f;
+  pdl_wait();
+  pdl_trigger();
   float sum[NFO], cmp[NFO];
 #pragma unroll
   for (int f = 0; f < NFO; ++f) {
     sum[f] = (accumulate && !AOS) ? out_soa.p[f][p] : 0.f;
     cmp[f] = 0.f;
   }
-  const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
   for (int s0 = b; s0 < en; s0 += MS) {
     int id[MS];
 #pragma unroll
@@ -914,7 +924,6 @@ __global__ void k_gather(MeshDev m, const float *__restrict__ slots, float *__re
       }
     }
   }
-  const float sc = use_invMl ? m.invMl[p] : 1.f;
   if (AOS) {
     float4 *o = reinterpret_cast<float4 *>(out + p * W);
     float r[W];
@@ -942,14 +951,16 @@ static __global__ void k_gather_sorted_res5(MeshDev m, const float *__restrict__
   if (p >= m.npoin) return;
   const float *sz = slots + 4 * zoff;
   const float4 *s4 = reinterpret_cast<const float4 *>(slots);
+  const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
+  const float sc = use_invMl ? m.invMl[p] : 1.f;
+  pdl_wait();
+  pdl_trigger();
   float sum[5], cmp[5];
 #pragma unroll
   for (int f = 0; f < 5; ++f) {
     sum[f] = accumulate ? out_soa.p[f][p] : 0.f;
     cmp[f] = 0.f;
   }
-  const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
-  const float sc = use_invMl ? m.invMl[p] : 1.f;
   for (int s = b; s < en; ++s) {
     const float4 v = s4[s];
     const float x[5] = {v.x, v.y, v.z, v.w, sz[s]};
