@@ -136,7 +136,7 @@ struct sod_gpu_ctx {
   // IMEX integrator scratch (five-variable blocks [mass][energy][momentum])
   struct Imex {
     float *R = nullptr, *D = nullptr;  // [4 stages][5N] explicit / implicit residuals
-    float *stab = nullptr, *lvl1 = nullptr, *aux_h = nullptr;
+    float *stab = nullptr, *lvl1 = nullptr, *aux_h = nullptr, *Dx0 = nullptr;
     float *x = nullptr, *r = nullptr, *p = nullptr, *qn = nullptr, *b = nullptr, *z = nullptr, *z1 = nullptr;
     float *au = nullptr, *aT = nullptr, *zmu = nullptr, *zmue = nullptr;  // CG primitives; zero viscosities
     int cg_iters = 0;

@@ -321,6 +321,7 @@ struct RhsArgs {
   const float *proj12;    // [npoin][12] mass-inverted projections (internal):
                           // tau00 tau01 tau02 tau11 tau12 tau22 gradRho(3) gradT(3)
   float fact_c, fact_d;
+  const int *stop;  // non-zero: return at once (an iteration that has ended); null: run
   int *err;  // mapped host flag: set when a bulk-copy wait of pass B gave up
 };
 
@@ -494,6 +495,7 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
   int nd_next = node_of(g + G);
   pdl_wait();
   pdl_trigger();
+  if (A.stop && *A.stop) return;
   issue(dsm, g, nd_first);
   cp_async_commit();
   for (int buf = 0; g < ngroups; g += G, buf ^= 1) {
