@@ -54,9 +54,8 @@ void launch_stage(sod_gpu_ctx *c, double l1, double li, double gdt, int first) {
   auto &S = c->comp;
   State5<T> U1, U2;
   for (int f = 0; f < 5; ++f) { U1.f[f] = (T *)S.U1[f]; U2.f[f] = (T *)S.U2[f]; }
-  k_stage<T><<<nblk(c->npoin_w, 256), 256, 0, c->stream>>>(c->npoin_w, c->npoin, c->lpoin_w, U1, U2, S.Rmass,
-                                                           S.Rmom, S.Rener, (T)l1, (T)li, (T)gdt, first, S.rho32,
-                                                           S.q32, S.E32);
+  launch_pdl(k_stage<T>, nblk(c->npoin_w, 256), 256, 0, c->stream, c->npoin_w, c->npoin, c->lpoin_w, U1, U2, S.Rmass,
+             S.Rmom, S.Rener, (T)l1, (T)li, (T)gdt, first, S.rho32, S.q32, S.E32);
 }
 
 // RHS at the current FP32 shadow state into comp.R* (updateF body).
@@ -85,16 +84,12 @@ int comp_entropy_pass(sod_gpu_ctx *c, float *Reta_out, bool dc) {
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
     constexpr int P = LL::P_;
-    if (dc)
-      k_entropy_elem<P, LL::EPB, true><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), S.feta, S.eta1, S.u1,
-                                                                                     S.u2, c->slotsB);
-    else
-      k_entropy_elem<P, LL::EPB, false><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), S.feta, S.eta1, S.u1,
-                                                                                      S.u2, c->slotsB);
+    launch_pdl(dc ? k_entropy_elem<P, LL::EPB, true> : k_entropy_elem<P, LL::EPB, false>, LL::grid(c->nelem), LL::TPB, 0,
+               c->stream, c->md(), S.feta, S.eta1, S.u1, S.u2, c->slotsB, 1.0f);
     return 0;
   });
-  k_gather_entropy<<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, c->lelpn, c->is_work, Reta_out,
-                                                               S.divU, S.vort, dc ? 1 : 0);
+  launch_pdl(dc ? k_gather_entropy<true> : k_gather_entropy<false>, nblk(c->npoin, 256), 256, 0, c->stream, c->md(),
+             c->slotsB, (long long)c->nelem * c->N, c->lelpn, c->is_work, Reta_out, S.divU, S.vort);
   // halo sums of the lumped entropy residual (time_integ_ls.f90:287, :431),
   // the divergence and the vorticity (mod_operators.f90:566, :759)
   HaloView v{};
@@ -108,8 +103,7 @@ int comp_entropy_pass(sod_gpu_ctx *c, float *Reta_out, bool dc) {
 
 int comp_visc(sod_gpu_ctx *c, const float *Reta, const float *rho, const float *u, bool ducros) {
   auto &S = c->comp;
-  const unsigned init_bits = 0x47C35000u;  // 100000.0f
-  CUDA_TRY(cudaMemcpyAsync(S.bits, &init_bits, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(cudaMemsetAsync(S.bits, 0x7f, sizeof(unsigned), c->stream));
   k_min_rho<<<MINMAX_BLOCKS, 256, 0, c->stream>>>(c->npoin_w, c->lpoin_w, rho, S.bits);
   // the bits of a positive float order like the float: reduce as float
   int rc = allreduce(c, S.bits, 1, SOD_REDUCE_MIN_F32);
@@ -121,7 +115,7 @@ int comp_visc(sod_gpu_ctx *c, const float *Reta, const float *rho, const float *
   V.inv_p = 1.0f / (float)c->P; V.ducros = ducros ? 1 : 0;
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_visc<LL::P_><<<nblk(c->nelem, 8), 256, 0, c->stream>>>(c->md(), V, c->a_of_t, c->mue_t, nullptr);
+    launch_pdl(k_visc<LL::P_>, nblk(c->nelem, 8), 256, 0, c->stream, c->md(), V, c->a_of_t, c->mue_t, nullptr);
     return 0;
   });
   return 0;
@@ -140,10 +134,7 @@ int sod_gpu_generic_scalar_convec_ijk(sod_gpu_ctx *c, const float *q, const floa
                                                                                         nullptr, c->slotsB, fact);
     return 0;
   });
-  OutPtrs o{};
-  o.p[0] = R;
-  k_gather<8, 1, false><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, nullptr, o,
-                                                                     initialze ? 0 : 1, 0);
+  k_gather_sorted1<<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, R, initialze ? 0 : 1);
   return c->finish();
 }
 
@@ -153,8 +144,7 @@ int sod_gpu_smart_visc_spectral_imex(sod_gpu_ctx *c, const float *Reta, const fl
   if (!c->helem) return fail(SOD_GPU_EINVAL, "smart_visc_spectral_imex needs helem at init");
   int rc;
   if (!c->vbits && (rc = c->alloc(&c->vbits, 4))) return rc;
-  const unsigned init_bits = 0x47C35000u;  // 100000.0f, the reference's initial minimum
-  CUDA_TRY(cudaMemcpyAsync(c->vbits, &init_bits, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(cudaMemsetAsync(c->vbits, 0x7f, sizeof(unsigned), c->stream));
   k_min_rho<<<MINMAX_BLOCKS, 256, 0, c->stream>>>(c->npoin_w, c->lpoin_w, rho, c->vbits);
   if ((rc = allreduce(c, c->vbits, 1, SOD_REDUCE_MIN_F32))) return rc;
   ViscArgs V{};
@@ -235,6 +225,7 @@ int sod_gpu_comp_init_state(sod_gpu_ctx *c, const sod_rk_cfg_t *cfg, const float
   CUDA_TRY(cudaMemcpyAsync(S.q32, q, 3 * N * 4, cudaMemcpyDeviceToDevice, st));
   CUDA_TRY(cudaMemcpyAsync(S.E32, E, N * 4, cudaMemcpyDeviceToDevice, st));
   CUDA_TRY(cudaMemcpyAsync(S.u2, u, 3 * N * 4, cudaMemcpyDeviceToDevice, st));
+  CUDA_TRY(cudaMemcpyAsync(S.u1, u, 3 * N * 4, cudaMemcpyDeviceToDevice, st));
   CUDA_TRY(cudaMemcpyAsync(S.pr, pr, N * 4, cudaMemcpyDeviceToDevice, st));
   CUDA_TRY(cudaMemcpyAsync(S.Tem, Tem, N * 4, cudaMemcpyDeviceToDevice, st));
   CUDA_TRY(cudaMemcpyAsync(S.csound, csound, N * 4, cudaMemcpyDeviceToDevice, st));
@@ -271,14 +262,13 @@ int sod_gpu_comp_rk_ls_step(sod_gpu_ctx *c, float dt) {
   auto &S = c->comp;
   const cudaStream_t st = c->stream;
   const size_t N = c->npoin;
-  const size_t tb = S.fp64 ? 8 : 4;
-  // level 1 <- level 2 (CFDSolverBase.f90:1951-1960)
-  for (int f = 0; f < 5; ++f) CUDA_TRY(cudaMemcpyAsync(S.U1[f], S.U2[f], N * tb, cudaMemcpyDeviceToDevice, st));
-  CUDA_TRY(cudaMemcpyAsync(S.u1, S.u2, 3 * N * 4, cudaMemcpyDeviceToDevice, st));
-  CUDA_TRY(cudaMemcpyAsync(S.eta1, S.eta2, N * 4, cudaMemcpyDeviceToDevice, st));
   // tau from level 2 (comp_tau)
-  k_comp_tau<<<nblk(c->nelem, 8), 256, 0, st>>>(c->nelem, c->N, c->conn, c->helem, S.csound, S.u2, c->npoin,
-                                                c->phys.c_species_stab / (float)c->P, S.tau);
+  comp_tau(c, S.csound, S.u2, S.tau);
+  // level 1 <- level 2 (CFDSolverBase.f90:1951-1960): the first stage fills
+  // U1, thermo_entropy eta1; the velocity changes buffers (u2 is written at
+  // the end of the step, and read before that nowhere)
+  std::swap(S.u1, S.u2);
+  if (S.first) CUDA_TRY(cudaMemcpyAsync(S.eta1, S.eta2, N * 4, cudaMemcpyDeviceToDevice, st));
   if (S.first) {
     S.first = false;
     k_feta<<<nblk(c->npoin_w, 256), 256, 0, st>>>(c->npoin_w, c->npoin, c->lpoin_w, S.u1, S.eta1, S.feta);
@@ -302,18 +292,16 @@ int sod_gpu_comp_rk_ls_step(sod_gpu_ctx *c, float dt) {
     stage(as_rp(S.lam[i + 1][1], S.fp64), as_rp(S.lam[i + 1][i], S.fp64), as_rp(S.gam[i + 1][i], S.fp64), 0);
   }
   const float gm = c->phys.gamma_gas;
-  k_eos_end<<<nblk(c->npoin_w, 256), 256, 0, st>>>(c->npoin_w, c->npoin, c->lpoin_w, gm - 1.0f, gm, c->phys.Rgas,
-                                                   S.rho32, S.q32, S.E32, S.u2, S.eint, S.pr, S.csound, S.machno,
-                                                   S.Tem);
-  k_thermo_entropy<<<nblk(c->npoin_w, 256), 256, 0, st>>>(c->npoin_w, c->npoin, c->lpoin_w, gm, c->phys.p_inf,
-                                                          c->phys.rho_inf, S.rho32, S.pr, S.u1, S.eta1, S.eta2,
-                                                          S.feta);
+  launch_pdl(k_eos_end, nblk(c->npoin_w, 256), 256, 0, st, c->npoin_w, c->npoin, c->lpoin_w, gm - 1.0f, gm,
+             c->phys.Rgas, S.rho32, S.q32, S.E32, S.u2, S.eint, S.pr, S.csound, S.machno, S.Tem, S.mu_factor,
+             S.mu_fluid);
+  launch_pdl(k_thermo_entropy, nblk(c->npoin_w, 256), 256, 0, st, c->npoin_w, c->npoin, c->lpoin_w, gm, c->phys.p_inf,
+             c->phys.rho_inf, S.rho32, S.pr, S.u1, S.eta1, S.eta2, S.feta);
   int rc = comp_entropy_pass(c, S.Reta2, true);
   if (rc) return rc;
   k_aux_reta<<<nblk(c->npoin_w, 256), 256, 0, st>>>(c->npoin_w, c->lpoin_w, dt, S.Reta1, S.Reta2, S.eta1, S.eta2,
                                                     S.aux);
   if ((rc = comp_visc(c, S.aux, S.rho32, S.u2, true))) return rc;
-  k_sutherland<<<nblk(c->npoin_w, 256), 256, 0, st>>>(c->npoin_w, c->lpoin_w, S.mu_factor, S.Tem, S.mu_fluid);
   return c->finish();
 }
 
@@ -572,8 +560,7 @@ int sod_gpu_comp_imex_step(sod_gpu_ctx *c, float dt, int maxIter, double tol) {
   // LPS stabilisation of the step's initial state (comp_tau, full_proj_ijk,
   // full_stab_ijk with fact -1 = the LPS part of full_diff_stab_ijk with zero
   // viscosities and fact +1)
-  k_comp_tau<<<nblk(c->nelem, 8), 256, 0, st>>>(c->nelem, c->N, c->conn, c->helem, S.csound, S.u2, c->npoin,
-                                                c->phys.c_species_stab / (float)c->P, S.tau);
+  comp_tau(c, S.csound, S.u2, S.tau);
   {
     RhsArgs A{};
     A.rho = S.rho32; A.u = S.u2; A.Tem = S.Tem; A.mu_fluid = X.zmu; A.mue_t = X.zmue; A.musgs_t = nullptr;
@@ -613,7 +600,7 @@ int sod_gpu_comp_imex_step(sod_gpu_ctx *c, float dt, int maxIter, double tol) {
     }
     iters += X.cg_iters;
     k_eos_end<<<nb, 256, 0, st>>>(nw, N, c->lpoin_w, gm - 1.0f, gm, c->phys.Rgas, S.rho32, S.q32, S.E32, S.u2, S.eint,
-                                  S.pr, S.csound, S.machno, S.Tem);
+                                  S.pr, S.csound, S.machno, S.Tem, 0.f, nullptr);
     k_aux_h<<<nb, 256, 0, st>>>(nw, c->lpoin_w, gm / (gm - 1.0f), S.rho32, S.pr, X.aux_h);
     if ((rc = imex_convec(c, S.rho32, S.u2, S.q32, S.pr, X.aux_h, X.R + (is - 1) * B)) ||
         (rc = imex_diffusion(c, nullptr, S.rho32, S.u2, S.Tem, X.D + (is - 1) * B))) {
@@ -649,11 +636,10 @@ int sod_gpu_comp_imex_stats(sod_gpu_ctx *c, int *cg_iters, double *cg_res) {
 int sod_gpu_comp_adapt_dt(sod_gpu_ctx *c, float cfl_conv, float cfl_diff, float *dt) {
   if (!c || !c->comp.ready || !dt) return fail(SOD_GPU_EINVAL, "bad argument");
   auto &S = c->comp;
-  const unsigned init_bits = 0x56B5E621u;  // 1e14f
-  CUDA_TRY(cudaMemcpyAsync(S.bits + 1, &init_bits, 4, cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(cudaMemsetAsync(S.bits + 1, 0x7f, 4, c->stream));
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_dt<LL::P_><<<nblk(c->nelem, 8), 256, 0, c->stream>>>(c->md(), c->helem, S.u2, S.csound, S.mu_fluid,
+    k_dt<LL::P_><<<dt_grid(c->nelem), 256, 0, c->stream>>>(c->md(), c->helem, S.u2, S.csound, S.mu_fluid,
                                                             c->mue_t, S.rho32, cfl_conv, cfl_diff, S.bits + 1);
     return 0;
   });
@@ -664,7 +650,7 @@ int sod_gpu_comp_adapt_dt(sod_gpu_ctx *c, float cfl_conv, float cfl_diff, float 
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   float v;
   std::memcpy(&v, &b, 4);
-  *dt = v;
+  *dt = std::min(v, 1e14f);  // the reference's initial value
   return 0;
 }
 
@@ -712,8 +698,7 @@ int sod_gpu_comp_get_state(sod_gpu_ctx *c, float *rho, float *q, float *E, float
   if (q) CUDA_TRY(cudaMemcpyAsync(q, S.q32, 3 * N * 4, cudaMemcpyDeviceToDevice, c->stream));
   if (E) CUDA_TRY(cudaMemcpyAsync(E, S.E32, N * 4, cudaMemcpyDeviceToDevice, c->stream));
   if (mu_e) {
-    const long long EN = (long long)c->nelem * c->N;
-    k_t_to_elem<<<nblk(EN, 256), 256, 0, c->stream>>>(c->nelem, c->N, c->a_of_t, c->mue_t, mu_e);
+    k_t_to_elem<<<nblk(c->nelem, E2T_TILE), E2T_THREADS, 0, c->stream>>>(c->nelem, c->N, c->a_of_t, c->mue_t, mu_e);
   }
   return c->finish();
 }

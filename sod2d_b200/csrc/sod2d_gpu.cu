@@ -323,8 +323,7 @@ int sod_gpu_lumped_solver(sod_gpu_ctx *c, float *R, int ncomp) {
 int sod_gpu_comp_tau(sod_gpu_ctx *c, const float *csound, const float *u, float *tau) {
   if (!c || !csound || !u || !tau) return fail(SOD_GPU_EINVAL, "bad argument");
   if (!c->helem) return fail(SOD_GPU_EINVAL, "comp_tau needs helem at init");
-  k_comp_tau<<<nblk(c->nelem, 8), 256, 0, c->stream>>>(c->nelem, c->N, c->conn, c->helem, csound, u, c->npoin,
-                                                      c->phys.c_species_stab / (float)c->P, tau);
+  comp_tau(c, csound, u, tau);
   return c->finish();
 }
 

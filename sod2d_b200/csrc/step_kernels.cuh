@@ -15,6 +15,9 @@ struct State5 {
 // ---- RK stage update (time_integ_ls.f90:323-332 and :350-359) ---------
 // first != 0: U2 += g*dt*R.  Otherwise U2 = l1*U1 + li*U2 + g*dt*R.
 // The FP32 shadow (reference layout: rho, q(N,3), E) receives the result.
+// The first stage also fills U1: U1 receives the level that U2 held, in place of a copy
+// before the step; U1 is read only where l1 is not zero.  Bound by HBM
+// (48^3, FP64: 192 B a node in 71-80 us, 6.0 TB/s).
 template <class T>
 __global__ void k_stage(int npoin_w, long long npoin, const int *__restrict__ lpoin_w, State5<T> U1, State5<T> U2,
                         const float *__restrict__ Rmass, const float *__restrict__ Rmom,
@@ -23,32 +26,42 @@ __global__ void k_stage(int npoin_w, long long npoin, const int *__restrict__ lp
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npoin_w) return;
   const long long p = lpoin_w[t];
+  pdl_wait();
+  pdl_trigger();
   const float R[5] = {Rmass[p], Rmom[p], Rmom[p + npoin], Rmom[p + 2 * npoin], Rener[p]};
+  T u2[5], u1[5];
 #pragma unroll
   for (int f = 0; f < 5; ++f) {
-    T v;
-    if (first)
-      v = U2.f[f][p] + gdt * (T)R[f];
-    else
-      v = l1 * U1.f[f][p] + li * U2.f[f][p] + gdt * (T)R[f];
-    U2.f[f][p] = v;
+    u2[f] = U2.f[f][p];
+    u1[f] = (T)0;
+    if (!first && l1 != (T)0) u1[f] = U1.f[f][p];
   }
-  rho32[p] = (float)U2.f[0][p];
-  q32[p] = (float)U2.f[1][p];
-  q32[p + npoin] = (float)U2.f[2][p];
-  q32[p + 2 * npoin] = (float)U2.f[3][p];
-  E32[p] = (float)U2.f[4][p];
+#pragma unroll
+  for (int f = 0; f < 5; ++f) {
+    if (first) U1.f[f][p] = u2[f];
+    const T v = first ? u2[f] + gdt * (T)R[f] : l1 * u1[f] + li * u2[f] + gdt * (T)R[f];
+    U2.f[f][p] = v;
+    u2[f] = v;
+  }
+  rho32[p] = (float)u2[0];
+  q32[p] = (float)u2[1];
+  q32[p + npoin] = (float)u2[2];
+  q32[p + 2 * npoin] = (float)u2[3];
+  E32[p] = (float)u2[4];
 }
 
-// ---- end-of-step EOS (time_integ_ls.f90:391-407) -----------------------
+// ---- end-of-step EOS (time_integ_ls.f90:391-407), with the Sutherland
+// viscosity of the new temperature (as k_sutherland) when mu is given ------
 static __global__ void k_eos_end(int npoin_w, long long npoin, const int *__restrict__ lpoin_w, float gm1, float gamma,
                           float Rgas, const float *__restrict__ rho, const float *__restrict__ q,
                           const float *__restrict__ E, float *__restrict__ u, float *__restrict__ eint,
                           float *__restrict__ pr, float *__restrict__ csound, float *__restrict__ machno,
-                          float *__restrict__ Tem) {
+                          float *__restrict__ Tem, float mu_factor, float *__restrict__ mu) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npoin_w) return;
   const long long p = lpoin_w[t];
+  pdl_wait();
+  pdl_trigger();
   const float r = rho[p];
   float umag = 0.f;
   float uu[3];
@@ -65,7 +78,9 @@ static __global__ void k_eos_end(int npoin_w, long long npoin, const int *__rest
   const float c = sqrtf(gamma * pp / r);
   csound[p] = c;
   machno[p] = sqrtf(umag) / c;
-  Tem[p] = pp / (r * Rgas);
+  const float T = pp / (r * Rgas);
+  Tem[p] = T;
+  if (mu) mu[p] = mu_factor * 1.458e-6f * powf(T, 1.5f) / (T + 110.4f);
 }
 
 // ---- thermo_entropy, mod_entropy_viscosity.f90:411-433 ----------------
@@ -78,6 +93,8 @@ static __global__ void k_thermo_entropy(int npoin_w, long long npoin, const int 
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npoin_w) return;
   const long long p = lpoin_w[t];
+  pdl_wait();
+  pdl_trigger();
   const float e1 = eta2[p];
   eta1[p] = e1;
   const float r = rho[p];
@@ -97,7 +114,8 @@ static __global__ void k_feta(int npoin_w, long long npoin, const int *__restric
 }
 
 // ---- entropy flux residual + divergence + vorticity, one element pass --
-// Slot fields (width 8): 0 = generic_scalar_convec_ijk of (feta, eta1, u1)
+// Node-sorted slots (as pass B's): a float4 and a float array with WANT_DC,
+// else one float per element node.  Fields: 0 = generic_scalar_convec_ijk of (feta, eta1, u1)
 // (elem_convec.f90:472-594), 1 = eval_divergence of u2
 // (mod_operators.f90:485-570), 2..4 = compute_vorticity of u2 before the
 // per-node averaging (mod_operators.f90:684-775).  WANT_DC = 0 skips 1..4.
@@ -112,8 +130,21 @@ k_entropy_elem(MeshDev m, const float *__restrict__ feta, const float *__restric
   const long long e = (long long)blockIdx.x * EPB + el;
   const bool active = (e < m.nelem) && (t < N);
   const long long NP = m.npoin;
+  // mesh loads first (no other kernel writes them): J^-1 after the staging
+  // barrier doubled the latency chain
+  int node = 0, pos = 0;
+  float He[9], gv = 0.f;
   if (active) {
-    const int node = m.conn[e * N + t];
+    node = m.conn[e * N + t];
+    pos = m.slot_pos[e * N + t];
+    const float *g = m.geo + e * 10 * N + t;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) He[c] = g[c * N];
+    gv = g[9 * N];
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (active) {
     sm[el][0][t] = eta1[node];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -128,11 +159,6 @@ k_entropy_elem(MeshDev m, const float *__restrict__ feta, const float *__restric
   float Di[N1], Dj[N1], Dk[N1];
 #pragma unroll
   for (int s = 0; s < N1; ++s) { Di[s] = m.Dnat[i * N1 + s]; Dj[s] = m.Dnat[j * N1 + s]; Dk[s] = m.Dnat[k * N1 + s]; }
-  const float *g = m.geo + e * 10 * N + t;
-  float He[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) He[c] = g[c * N];
-  const float gv = g[9 * N];
   float a0, a1, a2;
   iso_grad<P>(sm[el][0], i, j, k, Di, Dj, Dk, a0, a1, a2);
   float gradE[3];
@@ -167,39 +193,70 @@ k_entropy_elem(MeshDev m, const float *__restrict__ feta, const float *__restric
     out[3] = -gu[0][2] + gu[2][0];
     out[4] = gu[0][1] - gu[1][0];
   }
-  float4 *o = reinterpret_cast<float4 *>(slots + (e * N + t) * 8);
-  o[0] = make_float4(out[0], out[1], out[2], out[3]);
-  o[1] = make_float4(out[4], 0.f, 0.f, 0.f);
+  if (WANT_DC) {
+    reinterpret_cast<float4 *>(slots)[pos] = make_float4(out[0], out[1], out[2], out[3]);
+    slots[(long long)m.nelem * N * 4 + pos] = out[4];
+  } else {
+    slots[pos] = out[0];
+  }
 }
 
 // Gather of the entropy pass: Reta (lumped: x invMl at working nodes),
 // divU (raw), curl / lelpn (working nodes).  Kahan-compensated, element order.
-static __global__ void k_gather_entropy(MeshDev m, const float *__restrict__ slots, const int *__restrict__ lelpn,
-                                 const int *__restrict__ is_work, float *__restrict__ Reta, float *__restrict__ divU,
-                                 float *__restrict__ vort, int want_dc) {
+template <bool WANT_DC>
+__global__ void k_gather_entropy(MeshDev m, const float *__restrict__ slots, long long zoff,
+                                 const int *__restrict__ lelpn, const int *__restrict__ is_work,
+                                 float *__restrict__ Reta, float *__restrict__ divU, float *__restrict__ vort) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= m.npoin) return;
-  const int nf = want_dc ? 5 : 1;
-  float sum[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, cmp[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  constexpr int NF = WANT_DC ? 5 : 1;
   const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
+  const float iml = m.invMl[p];
+  const bool w = is_work[p] != 0;
+  const float inv = WANT_DC && w ? (float)lelpn[p] : 1.f;
+  pdl_wait();
+  pdl_trigger();
+  const float4 *s4 = reinterpret_cast<const float4 *>(slots);
+  const float *sz = slots + 4 * zoff;
+  float sum[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, cmp[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
   for (int s = b; s < en; ++s) {
-    const float4 *v = reinterpret_cast<const float4 *>(slots + (long long)m.slot_idx[s] * 8);
-    const float4 x0 = v[0], x1 = v[1];
-    const float x[5] = {x0.x, x0.y, x0.z, x0.w, x1.x};
-    for (int f = 0; f < nf; ++f) {
+    float x[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    if (WANT_DC) {
+      const float4 v = s4[s];
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; x[4] = sz[s];
+    } else {
+      x[0] = slots[s];
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
       const float y = x[f] - cmp[f];
       const float tt = sum[f] + y;
       cmp[f] = (tt - sum[f]) - y;
       sum[f] = tt;
     }
   }
-  Reta[p] = sum[0] * m.invMl[p];
-  if (want_dc) {
+  Reta[p] = sum[0] * iml;
+  if (WANT_DC) {
     divU[p] = sum[1];
-    const bool w = is_work[p] != 0;
-    const float inv = w ? (float)lelpn[p] : 1.f;
+#pragma unroll
     for (int d = 0; d < 3; ++d) vort[p + m.npoin * d] = w ? sum[2 + d] / inv : sum[2 + d];
   }
+}
+
+// Node sums of scalar node-sorted slots into (or onto) out, Kahan, element order.
+static __global__ void k_gather_sorted1(MeshDev m, const float *__restrict__ slots, float *__restrict__ out,
+                                        int accumulate) {
+  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= m.npoin) return;
+  const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
+  float sum = accumulate ? out[p] : 0.f, cmp = 0.f;
+  for (int s = b; s < en; ++s) {
+    const float y = slots[s] - cmp;
+    const float tt = sum + y;
+    cmp = (tt - sum) - y;
+    sum = tt;
+  }
+  out[p] = sum;
 }
 
 // auxReta = (1.5 R2 - 0.5 R1) + (eta2 - eta1)/dt; R1 <- R2 (time_integ_ls.f90:437-443)
@@ -214,6 +271,8 @@ static __global__ void k_aux_reta(int npoin_w, const int *__restrict__ lpoin_w, 
 }
 
 // Minimum of rho over working nodes (order-independent, deterministic).
+// out_bits starts as 0x7f7f7f7f (one memset); the reference's initial value
+// 100000 enters in k_visc.
 // grid of the node min / max reductions: 8 blocks of 256 per SM
 constexpr int MINMAX_BLOCKS = 148 * 8;
 static __global__ void k_min_rho(int npoin_w, const int *__restrict__ lpoin_w, const float *__restrict__ rho,
@@ -248,42 +307,66 @@ struct ViscArgs {
   int ducros;
 };
 
+// A lane holds its nodes' loads (two at P = 3, four at P = 4), all issued
+// before the element maximum is formed.
 template <int P>
 __global__ void k_visc(MeshDev m, ViscArgs A, const int *__restrict__ a_of_t, float *__restrict__ mue_t,
                        float *__restrict__ mue_ref) {
-  constexpr int N = Cfg<P>::N;
+  constexpr int N = Cfg<P>::N, IT = (N + 31) / 32;
   const long long e = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
   if (e >= m.nelem) return;
   const long long NP = m.npoin;
-  const float norm = __uint_as_float(*A.min_rho_bits);
+  int p[IT];
+  float hl[IT];
   const float he = A.helem[e];
-  float betae = 0.f;
-  for (int t = lane; t < N; t += 32) {
-    const int p = m.conn[e * N + t];
-    const float u0 = A.u[p], u1 = A.u[p + NP], u2 = A.u[p + 2 * NP];
-    const float aux2 = sqrtf(u0 * u0 + u1 * u1 + u2 * u2);
-    const float aux1 = aux2 + 1.0f * A.csound[p];
-    betae = fmaxf(betae, (A.rho[p] * he) * (A.cmax * A.inv_p) * aux1);
+#pragma unroll
+  for (int q = 0; q < IT; ++q) {
+    const int t = lane + 32 * q;
+    p[q] = t < N ? m.conn[e * N + t] : -1;
+    hl[q] = A.ducros && t < N ? A.helem_l_t[e * N + t] : 1.f;
   }
+  pdl_wait();
+  pdl_trigger();
+  const float norm = fminf(__uint_as_float(*A.min_rho_bits), 100000.0f);
+  float um[IT], cs[IT], rh[IT], re[IT], dv[IT], vv[IT];
+#pragma unroll
+  for (int q = 0; q < IT; ++q) {
+    if (p[q] < 0) continue;
+    const long long n = p[q];
+    const float u0 = A.u[n], u1 = A.u[n + NP], u2 = A.u[n + 2 * NP];
+    cs[q] = A.csound[n];
+    rh[q] = A.rho[n];
+    re[q] = A.Reta[n];
+    um[q] = sqrtf(u0 * u0 + u1 * u1 + u2 * u2);
+    if (A.ducros) {
+      dv[q] = A.divU[n] / A.Ml[n];
+      const float v0 = A.vort[n], v1 = A.vort[n + NP], v2 = A.vort[n + 2 * NP];
+      vv[q] = v0 * v0 + v1 * v1 + v2 * v2;
+    }
+  }
+  float betae = 0.f;
+#pragma unroll
+  for (int q = 0; q < IT; ++q)
+    if (p[q] >= 0) {
+      const float aux1 = um[q] + 1.0f * cs[q];
+      betae = fmaxf(betae, (rh[q] * he) * (A.cmax * A.inv_p) * aux1);
+    }
   for (int o = 16; o > 0; o >>= 1) betae = fmaxf(betae, __shfl_xor_sync(0xffffffffu, betae, o));
   const float hp = he * A.inv_p;
-  for (int t = lane; t < N; t += 32) {
-    const int p = m.conn[e * N + t];
-    const float R1 = A.rho[p] * fabsf(A.Reta[p]) / norm;
+#pragma unroll
+  for (int q = 0; q < IT; ++q) {
+    if (p[q] < 0) continue;
+    const int t = lane + 32 * q;
+    const float R1 = rh[q] * fabsf(re[q]) / norm;
     const float Ve = A.ce * R1 * (hp * hp);
     float mu = A.cglob * fminf(Ve, betae);
     if (A.ducros) {
-      const float divUl = A.divU[p] / A.Ml[p];
-      const float u0 = A.u[p], u1 = A.u[p + NP], u2 = A.u[p + 2 * NP];
-      const float aux2 = sqrtf(u0 * u0 + u1 * u1 + u2 * u2);
-      const float v0 = A.vort[p], v1 = A.vort[p + NP], v2 = A.vort[p + 2 * NP];
-      const float vv = v0 * v0 + v1 * v1 + v2 * v2;
-      const float d2 = divUl * divUl;
+      const float d2 = dv[q] * dv[q];
       const float eps = 1.1920929e-07f;
-      const float phi = fminf((4.0f / 3.0f) * d2 / (d2 + vv + eps), 1.0f);
-      const float hl = 1.0f * aux2 / A.helem_l_t[e * N + t];
-      const float phi2 = d2 / (d2 + hl * hl + eps);
+      const float phi = fminf((4.0f / 3.0f) * d2 / (d2 + vv[q] + eps), 1.0f);
+      const float hq = 1.0f * um[q] / hl[q];
+      const float phi2 = d2 / (d2 + hq * hq + eps);
       mu = mu * (fmaxf(phi - A.ducros_min, 0.f) * phi2 + A.ducros_min);
     }
     mue_t[e * N + t] = mu;
@@ -359,35 +442,55 @@ static __global__ void k_sutherland(int npoin_w, const int *__restrict__ lpoin_w
 }
 
 // ---- adapt_dt_cfl, mod_time_ops.f90:11-62: per element, then min -------
+// Warps stride over the elements and a block issues one atomic: one atomic
+// per element to the same word was half of this kernel's time (110,592
+// elements: 120 us).  out_bits starts as 0x7f7f7f7f; the caller applies the
+// reference's initial 1e14.
 template <int P>
-__global__ void k_dt(MeshDev m, const float *__restrict__ helem, const float *__restrict__ u,
-                     const float *__restrict__ csound, const float *__restrict__ mu_fluid,
-                     const float *__restrict__ mue_t, const float *__restrict__ rho, float cfl_conv, float cfl_diff,
-                     unsigned int *__restrict__ out_bits) {
-  constexpr int N = Cfg<P>::N;
-  const long long e = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x % 32;
-  if (e >= m.nelem) return;
+__global__ void __launch_bounds__(256)
+k_dt(MeshDev m, const float *__restrict__ helem, const float *__restrict__ u, const float *__restrict__ csound,
+     const float *__restrict__ mu_fluid, const float *__restrict__ mue_t, const float *__restrict__ rho, float cfl_conv,
+     float cfl_diff, unsigned int *__restrict__ out_bits) {
+  constexpr int N = Cfg<P>::N, IT = (N + 31) / 32;
+  __shared__ unsigned sh[8];
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   const long long NP = m.npoin;
-  float L3 = 0.f, maxMU = 0.f;
-  for (int t = lane; t < N; t += 32) {
-    const int p = m.conn[e * N + t];
-    float um = fabsf(u[p]);
-    um = fmaxf(um, fabsf(u[p + NP]));
-    um = fmaxf(um, fabsf(u[p + 2 * NP]));
-    L3 = fmaxf(L3, um + csound[p]);
-    maxMU = fmaxf(maxMU, (0.0f + mu_fluid[p] + mue_t[e * N + t]) / rho[p]);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    L3 = fmaxf(L3, __shfl_xor_sync(0xffffffffu, L3, o));
-    maxMU = fmaxf(maxMU, __shfl_xor_sync(0xffffffffu, maxMU, o));
-  }
-  if (lane == 0) {
+  unsigned best = 0x7f7f7f7fu;
+  for (long long e = (long long)blockIdx.x * 8 + warp; e < m.nelem; e += (long long)gridDim.x * 8) {
+    int p[IT];
+    float me[IT];
+#pragma unroll
+    for (int q = 0; q < IT; ++q) {
+      const int t = lane + 32 * q;
+      p[q] = t < N ? m.conn[e * N + t] : -1;
+      me[q] = t < N ? mue_t[e * N + t] : 0.f;
+    }
+    float L3 = 0.f, maxMU = 0.f;
+#pragma unroll
+    for (int q = 0; q < IT; ++q) {
+      if (p[q] < 0) continue;
+      const long long n = p[q];
+      float um = fabsf(u[n]);
+      um = fmaxf(um, fabsf(u[n + NP]));
+      um = fmaxf(um, fabsf(u[n + 2 * NP]));
+      L3 = fmaxf(L3, um + csound[n]);
+      maxMU = fmaxf(maxMU, (0.0f + mu_fluid[n] + me[q]) / rho[n]);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      L3 = fmaxf(L3, __shfl_xor_sync(0xffffffffu, L3, o));
+      maxMU = fmaxf(maxMU, __shfl_xor_sync(0xffffffffu, maxMU, o));
+    }
     const float hp = helem[e] / (float)(2 * P + 1);
     const float dconv = cfl_conv * hp / L3;
     const float ddiff = cfl_diff * (hp * hp) / maxMU;
-    const float dtl = fminf(dconv, ddiff);
-    atomicMin(out_bits, __float_as_uint(dtl));  // dt > 0
+    best = min(best, __float_as_uint(fminf(dconv, ddiff)));  // dt > 0: bit order = value order
+  }
+  if (lane == 0) sh[warp] = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) best = min(best, sh[w]);
+    atomicMin(out_bits, best);
   }
 }
 
