@@ -58,12 +58,13 @@ int net_forward_fp32(sod_gpu_ctx *c, const double *r, double *z) {
 
 namespace {
 
+// g = -2 A d / eAe; eAe from device memory where the host has not read it
 __global__ void k_loss_grad_vec(int npoin_w, const int *__restrict__ lpoin_w, const double *__restrict__ Ad,
-                                double scale, double *__restrict__ g) {
+                                double eAe, const double *__restrict__ eAe_dev, double *__restrict__ g) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npoin_w) return;
   const int i = lpoin_w[t];
-  g[i] = scale * Ad[i];
+  g[i] = -2.0 / (eAe_dev ? *eAe_dev : eAe) * Ad[i];
 }
 
 
@@ -119,7 +120,7 @@ void net_backward(sod_gpu_ctx *c, const double *r, const double *g, float *part,
 // loss = d^T A d / eAe with d = e - M r; the gradient partials go to part
 // (or are added to it: accumulate).
 int net_loss_grad(sod_gpu_ctx *c, const double *r, const double *e, double eAe, float *part, double *loss,
-                  int accumulate = 0) {
+                  int accumulate = 0, const double *eAe_dev = nullptr) {
   auto &NT = c->net;
   auto &G = c->cg;
   const int nw = c->npoin_w;
@@ -129,7 +130,7 @@ int net_loss_grad(sod_gpu_ctx *c, const double *r, const double *e, double eAe, 
   k_axpby<double><<<nb, 256, 0, c->stream>>>(nw, c->lpoin_w, 1.0, e, -1.0, NT.tmp1);        // d = e - z
   lap<double>(c, NT.tmp1, NT.tmp2);                                                         // A d
   dots<double, 1>(c, DotArgs<double, 1>{{NT.tmp1}, {NT.tmp2}, {nullptr}}, G.dots + 2);
-  k_loss_grad_vec<<<nb, 256, 0, c->stream>>>(nw, c->lpoin_w, NT.tmp2, -2.0 / eAe, NT.tmp2);
+  k_loss_grad_vec<<<nb, 256, 0, c->stream>>>(nw, c->lpoin_w, NT.tmp2, eAe, eAe_dev, NT.tmp2);
   net_backward(c, r, NT.tmp2, part, accumulate);
   if (loss) {
     double h;
@@ -370,14 +371,16 @@ int sod_gpu_precond_loss_grad(sod_gpu_ctx *c, const double *r, const double *e, 
   auto &NT = c->net;
   lap<double>(c, e, NT.tmp2);
   dots<double, 1>(c, DotArgs<double, 1>{{e}, {NT.tmp2}, {nullptr}}, c->cg.dots + 5);
-  double eAe;
-  CUDA_TRY(cudaMemcpyAsync(&eAe, c->cg.dots + 5, 8, cudaMemcpyDeviceToHost, c->stream));
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  if (!(eAe > 0)) return fail(SOD_GPU_EINVAL, "target has zero energy norm");
-  int rc = net_loss_grad(c, r, e, eAe, NT.part, loss);
+  int rc = net_loss_grad(c, r, e, 0.0, NT.part, nullptr, 0, c->cg.dots + 5);
   if (rc) return rc;
-  k_adam<<<nblk(NT.nparam, 256), 256, 0, c->stream>>>(NT.nparam, NT.nblk_bwd, NT.part, NT.params, NT.m1, NT.m2, 0.f,
-                                                      0.9f, 0.999f, 1e-8f, 1.f, 1.f, 1.f, NT.grad);
+  k_adam<<<nblk(NT.nparam, 32), 32 * ADAM_GROUPS, 0, c->stream>>>(NT.nparam, NT.nblk_bwd, NT.part, NT.params, NT.m1,
+                                                                  NT.m2, 0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f, 1.f,
+                                                                  NT.grad);
+  double h[4];  // d.A d and e.A e
+  CUDA_TRY(cudaMemcpyAsync(h, c->cg.dots + 2, 32, cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  if (!(h[3] > 0)) return fail(SOD_GPU_EINVAL, "target has zero energy norm");
+  *loss = h[0] / h[3];
   if (grad_host) CUDA_TRY(cudaMemcpyAsync(grad_host, NT.grad, (size_t)NT.nparam * 4, cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   return c->finish();
@@ -421,7 +424,7 @@ int sod_gpu_precond_train(sod_gpu_ctx *c, int steps, int batch, float lr, uint64
     }
     NT.step += 1;
     const float bc1 = 1.f - std::pow(0.9f, (float)NT.step), bc2 = 1.f - std::pow(0.999f, (float)NT.step);
-    k_adam<<<nblk(NT.nparam, 256), 256, 0, c->stream>>>(NT.nparam, NT.nblk_bwd, NT.part, NT.params, NT.m1,
+    k_adam<<<nblk(NT.nparam, 32), 32 * ADAM_GROUPS, 0, c->stream>>>(NT.nparam, NT.nblk_bwd, NT.part, NT.params, NT.m1,
                                                         NT.m2, lr, 0.9f, 0.999f, 1e-8f, bc1, bc2, 1.f / batch,
                                                         nullptr);
     NT.gains_ok = false;

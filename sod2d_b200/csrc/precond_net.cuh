@@ -634,13 +634,27 @@ static __global__ void k_alpha_part(int npoin_w, const int *__restrict__ lpoin_w
 }
 
 // grad[i] = sum over blocks of part[b][i] (fixed order), then Adam.
-static __global__ void k_adam(int nparam, int nblocks, const float *__restrict__ part, float *__restrict__ params,
-                       float *__restrict__ m1, float *__restrict__ m2, float lr, float b1, float b2, float eps,
-                       float bc1, float bc2, float gscale, float *__restrict__ grad_out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nparam) return;
+// A block takes 32 parameters, its 16 warps every 16th row of the partials
+// (a row of 32 is one 128-byte line); the warps' sums are added in warp
+// order.  One thread per parameter walking all 592 rows kept 30 blocks busy
+// for 40 us (17.8 MB: 3 us of HBM time).
+constexpr int ADAM_GROUPS = 16;
+static __global__ void __launch_bounds__(32 * ADAM_GROUPS)
+k_adam(int nparam, int nblocks, const float *__restrict__ part, float *__restrict__ params, float *__restrict__ m1,
+       float *__restrict__ m2, float lr, float b1, float b2, float eps, float bc1, float bc2, float gscale,
+       float *__restrict__ grad_out) {
+  __shared__ float sh[ADAM_GROUPS][32];
+  const int lane = threadIdx.x % 32, grp = threadIdx.x / 32, i = blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (i < nparam)
+#pragma unroll 8
+    for (int b = grp; b < nblocks; b += ADAM_GROUPS) s += part[(long long)b * nparam + i];
+  sh[grp][lane] = s;
+  __syncthreads();
+  if (grp != 0 || i >= nparam) return;
   float g = 0.f;
-  for (int b = 0; b < nblocks; ++b) g += part[(long long)b * nparam + i];
+#pragma unroll
+  for (int w = 0; w < ADAM_GROUPS; ++w) g += sh[w][lane];
   g *= gscale;
   if (grad_out) grad_out[i] = g;
   if (lr == 0.f) return;
