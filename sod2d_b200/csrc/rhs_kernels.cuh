@@ -189,6 +189,18 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// Shared -> global bulk copy: every writer of the source fences its stores
+// (before the barrier that precedes the copy), one thread copies and waits
+// until the source has been read.
+__device__ __forceinline__ void bulk_s2g_fence() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, unsigned bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\ncp.async.bulk.commit_group;\n" ::"l"(dst),
+               "r"(smem_u32(src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_s2g_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+}
 // Bounded wait for the phase `parity` of bar (try_wait itself suspends the
 // thread for a while): false after SOD_BULK_WAIT_LIMIT polls.
 #ifndef SOD_BULK_WAIT_LIMIT
@@ -283,12 +295,15 @@ k_proj(MeshDev m, Phys ph, float Rgas, const float *__restrict__ a0, const float
   o[1] = make_float4(gv * tau[1][2], gv * tau[2][2], gv * gradRho[0], gv * gradRho[1]);
   o[2] = make_float4(gv * gradRho[2], gv * gradT[0], gv * gradT[1], gv * gradT[2]);
   }
+  bulk_s2g_fence();
   __syncthreads();
+  // one bulk copy (48 N bytes per element, a multiple of 16) by one thread
   const long long e0 = (long long)blockIdx.x * EPB;
   const long long ne = (m.nelem - e0) < EPB ? (m.nelem - e0) : EPB;
-  const float4 *src = reinterpret_cast<const float4 *>(ost);
-  float4 *dst = reinterpret_cast<float4 *>(slots + e0 * N * 12);
-  for (int q = threadIdx.x; q < ne * N * 3; q += blockDim.x) dst[q] = src[q];
+  if (threadIdx.x == 0) {
+    bulk_s2g(slots + e0 * N * 12, ost, (unsigned)(ne * N * 48));
+    bulk_s2g_wait_read();
+  }
 }
 
 // ---------------------------------------------------------------------
