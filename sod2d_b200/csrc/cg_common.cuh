@@ -60,11 +60,20 @@ __global__ void k_add_all(long long n, const V *__restrict__ a, const V *__restr
   if (i < n) out[i] = a[i] + b[i];
 }
 
+template <int P, class V>
+inline DMat<P, V> dmat(const sod_gpu_ctx *c) {
+  DMat<P, V> D;
+  for (int a = 0; a <= P; ++a)
+    for (int b = 0; b <= P; ++b) D.d[a][b] = (V)c->D_h[a * (P + 1) + b];
+  return D;
+}
+
 template <class V>
 inline void lap(sod_gpu_ctx *c, const V *p, V *out) {
   dispatch(c, [&](auto L) {
-    using LL = decltype(L);
-    k_lap_elem<LL::P_, LL::EPB, V><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), p, (V *)c->slotsB);
+    constexpr int P = decltype(L)::P_;
+    k_lap_elem<P, V><<<nblk(c->nelem, LapCfg<P>::EPB), 32 * LAP_WARPS, 0, c->stream>>>(c->md(), dmat<P, V>(c), p,
+                                                                                      (V *)c->slotsB);
     return 0;
   });
   k_gather1<V><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), (const V *)c->slotsB, out, 0);

@@ -53,6 +53,7 @@ struct sod_gpu_ctx {
       *lelpn = nullptr;
   int *a_of_t = nullptr;  // tensor position -> reference local node (0-based)
   double *D64 = nullptr;
+  float D_h[25];  // host copy of the derivative matrix
   float *geo = nullptr, *Dnat = nullptr, *Drot = nullptr, *invMl = nullptr, *Ml = nullptr, *helem = nullptr, *helem_l_t = nullptr;
   // scratch
   float *slotsA = nullptr, *slotsB = nullptr, *proj12 = nullptr, *mue_t = nullptr, *musgs_t = nullptr;

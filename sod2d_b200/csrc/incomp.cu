@@ -104,9 +104,9 @@ int conjgrad_pressure_dev(sod_gpu_ctx *c, const float *Rp0, float *R, int maxIte
     const int it0 = it, nbat = std::min(batch_max, maxIter - it);
     for (int k = 0; k < nbat; ++k)
       dispatch(c, [&](auto L) {
-        using LL = decltype(L);
-        launch_pdl(k_lap_elem<LL::P_, LL::EPB, float, true>, LL::grid(c->nelem), LL::TPB, 0, st, c->md(), G.p32,
-                   (float *)c->slotsB, &G.S->status, G.z032, &G.S->beta);
+        constexpr int P = decltype(L)::P_;
+        launch_pdl(k_lap_elem<P, float, true>, nblk(c->nelem, LapCfg<P>::EPB), 32 * LAP_WARPS, 0, st, c->md(),
+                   dmat<P, float>(c), G.p32, (float *)c->slotsB, &G.S->status, G.z032, &G.S->beta);
         launch_pdl(k_cg_q<float>, cg_blocks(N, CG_QU), CG_THREADS, 0, st, c->md(), (const float *)c->slotsB, G.p32,
                    G.q32, G.S, G.gpart, G.ticket, G.z032);
         launch_pdl(k_cg_update32, cg_blocks(N, CG_U), CG_THREADS, 0, st, N, G.p32, G.q32, G.diag, G.x32, G.r32,
@@ -460,8 +460,8 @@ int sod_gpu_pressure_solve(sod_gpu_ctx *c, const double *b_in, double *x, const 
       using LL = decltype(L);
       constexpr int P = LL::P_;
       // the search direction p = z + beta p is formed inside these two
-      launch_pdl(k_lap_elem<P, LL::EPB, double, true>, LL::grid(c->nelem), LL::TPB, 0, st, md, G.p,
-                 (double *)c->slotsB, &G.S->status, G.z0, &G.S->beta);
+      launch_pdl(k_lap_elem<P, double, true>, nblk(c->nelem, LapCfg<P>::EPB), 32 * LAP_WARPS, 0, st, md,
+                 dmat<P, double>(c), G.p, (double *)c->slotsB, &G.S->status, G.z0, &G.S->beta);
       launch_pdl(k_cg_q<double>, cg_blocks(c->npoin, CG_QU), CG_THREADS, 0, st, md, (const double *)c->slotsB, G.p, G.q, G.S,
                  G.gpart, G.ticket, G.z0);
       if (kind == 0) {

@@ -7,110 +7,145 @@
 
 namespace sod {
 
-// Row (or column) c of the 1-D derivative matrix in V.
+// Rows and columns of the 1-D derivative matrix in V, rotated to start at the
+// diagonal (MeshDev::Drot, D64).
 template <int P>
-__device__ __forceinline__ void load_d(const MeshDev &m, int c, bool col, double (&D)[P + 1]) {
+__device__ __forceinline__ void load_rot(const MeshDev &m, int c, bool col, double (&D)[P + 1]) {
   const double2 *r = reinterpret_cast<const double2 *>(m.D64 + 8 * (c + (col ? P + 1 : 0)));
-#pragma unroll
-  for (int q = 0; q < (P + 1) / 2; ++q) {
-    const double2 v = r[q];
-    D[2 * q] = v.x;
-    D[2 * q + 1] = v.y;
-  }
+  const double2 v0 = r[0], v1 = r[1];
+  D[0] = v0.x; D[1] = v0.y; D[2] = v1.x; D[3] = v1.y;
   if (P == 4) D[4] = r[2].x;
 }
 template <int P>
-__device__ __forceinline__ void load_d(const MeshDev &m, int c, bool col, float (&D)[P + 1]) {
-#pragma unroll
-  for (int q = 0; q <= P; ++q) D[q] = col ? m.Dnat[q * (P + 1) + c] : m.Dnat[c * (P + 1) + q];
+__device__ __forceinline__ void load_rot(const MeshDev &m, int c, bool col, float (&D)[P + 1]) {
+  load_drot<P>(m.Drot + (col ? 8 * (P + 1) : 0), c, D);
 }
 
+// The derivative matrix as a kernel argument: entries at fixed indices are
+// operands from the constant bank.
+template <int P, class V>
+struct DMat {
+  V d[P + 1][P + 1];
+};
+
 // ---- Laplacian: ResP = sum_e int grad N . grad p  (mod_operators.f90:16-112)
-// One thread per Gauss point; V = float (reference arithmetic) or double.
-// Writes one V per element node into slots (width 1), element-ordered.
+// V = float (reference arithmetic) or double.  Writes one V per element node
+// into slots (width 1), element-ordered.
 // DIR (the CG iteration): the operand is the new search direction
 // z + beta p, formed on the fly from z, the previous p and *beta (the
 // update p = z + beta p itself is stored by k_cg_q), and the slots are
 // written node-sorted (slot_pos) for k_cg_q's contiguous sums.
-// The chain connectivity -> operand -> derivative bounds it, not bandwidth.
-// So everything that depends on no other kernel -- J^-1, weight, node, slot
-// position -- is requested first, before the programmatic wait and the
-// staging barrier, and the derivative matrix comes in V (converting its FP32
-// rows and columns took 24 of 34 conversions per point on a pipe of 16 per
-// clock and SM).
-template <int P, int EPB, class V, bool DIR = false>
-__global__ void __launch_bounds__(EPB *Cfg<P>::NT)
-k_lap_elem(MeshDev m, const V *__restrict__ p, V *__restrict__ slots, const int *__restrict__ stop = nullptr,
-           const V *__restrict__ z = nullptr, const double *__restrict__ beta = nullptr) {
-  constexpr int N1 = Cfg<P>::N1, N = Cfg<P>::N, NT = Cfg<P>::NT;
-  __shared__ V sm[EPB][4][N];
-  const int el = threadIdx.x / NT, t = threadIdx.x % NT;
-  const long long e = (long long)blockIdx.x * EPB + el;
-  const bool active = (e < m.nelem) && (t < N);
-  int n = 0, pos = 0;
-  float G[10];
-  if (active) {
-    n = m.conn[e * N + t];
-    pos = DIR ? m.slot_pos[e * N + t] : 0;
-    const float *g = m.geo + e * 10 * N + t;
+//
+// A thread owns the line of P + 1 points along zeta over its (i, j); 16
+// lanes (P = 3) or 25 of 32 (P = 4) take an element, so nothing but warp
+// barriers is needed.  The zeta derivatives and their transpose stay in
+// registers with the matrix as constant operands; in xi and eta a point
+// reads its line's other P nodes from shared memory, its own from registers
+// (cyclic order 2, 3, .., 1, own: see k_rhs).  With one point per thread the
+// shared and L1 pipe was 82 % busy -- 24 FP64 shared loads and 24 matrix
+// loads per point -- and bound the kernel; this form has 12 and 4.  All of a
+// thread's mesh loads (J^-1, weights, nodes, slot positions: 48 at P = 3)
+// are in flight before the programmatic wait.
+constexpr int LAP_WARPS = 2;
+template <int P>
+struct LapCfg {
+  static constexpr int LPE = P == 3 ? 16 : 32, EPW = 32 / LPE, EPB = LAP_WARPS * EPW;  // lanes and elements
+  static constexpr int MINB = P == 3 ? 8 : 6;                                          // blocks per SM
+};
+template <int P, class V, bool DIR = false>
+__global__ void __launch_bounds__(32 * LAP_WARPS, LapCfg<P>::MINB)
+k_lap_elem(MeshDev m, DMat<P, V> D, const V *__restrict__ p, V *__restrict__ slots,
+           const int *__restrict__ stop = nullptr, const V *__restrict__ z = nullptr,
+           const double *__restrict__ beta = nullptr) {
+  using L = LapCfg<P>;
+  constexpr int N1 = P + 1, N2 = N1 * N1, N = N1 * N2;
+  __shared__ V sm[L::EPB][2][N];
+  const int el = threadIdx.x / L::LPE, c = threadIdx.x % L::LPE;
+  const long long e = (long long)blockIdx.x * L::EPB + el;
+  const bool active = e < m.nelem && c < N2;
+  const int i = c % N1, j = c / N1;
+  int n[N1], pos[N1];
+  float G[N1][10];
+  V Di[N1], Dj[N1];
 #pragma unroll
-    for (int c = 0; c < 10; ++c) G[c] = g[c * N];
+  for (int k = 0; k < N1; ++k) n[k] = pos[k] = 0;
+  if (active) {
+    const long long b = e * N + c;
+#pragma unroll
+    for (int k = 0; k < N1; ++k) {
+      n[k] = m.conn[b + N2 * k];
+      if (DIR) pos[k] = m.slot_pos[b + N2 * k];
+    }
+    const float *g = m.geo + e * 10 * N + c;
+#pragma unroll
+    for (int k = 0; k < N1; ++k)
+#pragma unroll
+      for (int q = 0; q < 10; ++q) G[k][q] = g[q * N + N2 * k];
+    load_rot<P>(m, i, false, Di);
+    load_rot<P>(m, j, false, Dj);
   }
-  const int i = t % N1, j = (t / N1) % N1, k = t / (N1 * N1);
+  // the q-th node of a line: cyclic step from the own node, own last
+  auto step = [](int q) -> int { return q == P ? 0 : (q == P - 1 ? 1 : q + 2); };
+  auto xi = [&](int q, int k) -> int { const int s = step(q); return c + (i + s < N1 ? s : s - N1) + N2 * k; };
+  auto et = [&](int q, int k) -> int { const int s = step(q); return c + (j + s < N1 ? s : s - N1) * N1 + N2 * k; };
+  V *A = sm[el][0], *B = sm[el][1];
   pdl_wait();
   pdl_trigger();
   if (stop && *stop) return;
+  V f[N1];
   if (active) {
-    if (DIR) {
-      const V bt = (V)*beta;
-      sm[el][0][t] = z[n] + bt * p[n];
-    } else {
-      sm[el][0][t] = p[n];
+    const V bt = DIR ? (V)*beta : (V)0;
+#pragma unroll
+    for (int k = 0; k < N1; ++k) f[k] = DIR ? z[n[k]] + bt * p[n[k]] : p[n[k]];
+#pragma unroll
+    for (int k = 0; k < N1; ++k) A[c + N2 * k] = f[k];
+  }
+  __syncwarp();
+  V C0[N1], C1[N1], C2[N1];
+  if (active) {
+#pragma unroll
+    for (int k = 0; k < N1; ++k) {
+      V g0 = 0, g1 = 0, g2 = 0;
+#pragma unroll
+      for (int q = 0; q < N1; ++q) {
+        g0 += Di[step(q)] * (q == P ? f[k] : A[xi(q, k)]);
+        g1 += Dj[step(q)] * (q == P ? f[k] : A[et(q, k)]);
+        const int mm = ref_order<P>(q);
+        g2 += D.d[k][mm] * f[mm];
+      }
+      V He[9];
+#pragma unroll
+      for (int q = 0; q < 9; ++q) He[q] = (V)G[k][q];
+      const V gv = (V)G[k][9];
+      V gP[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) gP[a] = He[a] * g0 + He[a + 3] * g1 + He[a + 6] * g2;
+      C0[k] = gv * (He[0] * gP[0] + He[1] * gP[1] + He[2] * gP[2]);
+      C1[k] = gv * (He[3] * gP[0] + He[4] * gP[1] + He[5] * gP[2]);
+      C2[k] = gv * (He[6] * gP[0] + He[7] * gP[1] + He[8] * gP[2]);
     }
   }
-  __syncthreads();
-  V C0 = 0, C1 = 0, C2 = 0;
+  __syncwarp();  // the operand has been read
   if (active) {
-    V Di[N1], Dj[N1], Dk[N1];
-    load_d<P>(m, i, false, Di);
-    load_d<P>(m, j, false, Dj);
-    load_d<P>(m, k, false, Dk);
-    V He[9];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) He[c] = (V)G[c];
-    const V gv = (V)G[9];
-    const V *f = sm[el][0];
-    V g0 = 0, g1 = 0, g2 = 0;
-#pragma unroll
-    for (int s = 0; s < N1; ++s) {
-      const int mm = ref_order<P>(s);
-      g0 += Di[mm] * f[mm + N1 * j + N1 * N1 * k];
-      g1 += Dj[mm] * f[i + N1 * mm + N1 * N1 * k];
-      g2 += Dk[mm] * f[i + N1 * j + N1 * N1 * mm];
-    }
-    V gP[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) gP[a] = He[a] * g0 + He[a + 3] * g1 + He[a + 6] * g2;
-    C0 = gv * (He[0] * gP[0] + He[1] * gP[1] + He[2] * gP[2]);
-    C1 = gv * (He[3] * gP[0] + He[4] * gP[1] + He[5] * gP[2]);
-    C2 = gv * (He[6] * gP[0] + He[7] * gP[1] + He[8] * gP[2]);
-    sm[el][1][t] = C0; sm[el][2][t] = C1; sm[el][3][t] = C2;
+    for (int k = 0; k < N1; ++k) { A[c + N2 * k] = C0[k]; B[c + N2 * k] = C1[k]; }
+    load_rot<P>(m, i, true, Di);
+    load_rot<P>(m, j, true, Dj);
   }
-  __syncthreads();
+  __syncwarp();
   if (!active) return;
-  V Di[N1], Dj[N1], Dk[N1];
-  load_d<P>(m, i, true, Di);
-  load_d<P>(m, j, true, Dj);
-  load_d<P>(m, k, true, Dk);
-  V acc = 0;
 #pragma unroll
-  for (int s = 0; s < N1; ++s) {
-    const int mm = ref_order<P>(s);
-    acc += Di[mm] * sm[el][1][mm + N1 * j + N1 * N1 * k];
-    acc += Dj[mm] * sm[el][2][i + N1 * mm + N1 * N1 * k];
-    acc += Dk[mm] * sm[el][3][i + N1 * j + N1 * N1 * mm];
+  for (int k = 0; k < N1; ++k) {
+    V acc = 0;
+#pragma unroll
+    for (int q = 0; q < N1; ++q) {
+      acc += Di[step(q)] * (q == P ? C0[k] : A[xi(q, k)]);
+      acc += Dj[step(q)] * (q == P ? C1[k] : B[et(q, k)]);
+      const int mm = ref_order<P>(q);
+      acc += D.d[mm][k] * C2[mm];
+    }
+    slots[DIR ? (long long)pos[k] : e * N + c + N2 * k] = acc;
   }
-  slots[DIR ? (long long)pos : e * N + t] = acc;
 }
 
 // Scalar-slot assembly out(p) = scale * sum(slots of p); float sums are
@@ -390,26 +425,44 @@ __device__ bool grid_sum(double (&v)[ND], double *__restrict__ part, unsigned *t
   for (int d = 0; d < ND; ++d)
     for (int o = 16; o > 0; o >>= 1) v[d] += __shfl_xor_sync(0xffffffffu, v[d], o);
   if (lane == 0)
+#pragma unroll
     for (int d = 0; d < ND; ++d) sh[d][warp] = v[d];
   __syncthreads();
   if (threadIdx.x == 0) {
+#pragma unroll
     for (int d = 0; d < ND; ++d) {
       double s = 0.0;
       for (int w = 0; w < nw; ++w) s += sh[d][w];
       part[d * gridDim.x + blockIdx.x] = s;
     }
-    __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    // releases this block's partials, acquires the others'
+    unsigned got;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;\n" : "=r"(got) : "l"(ticket) : "memory");
+    last = got == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return false;
-  __threadfence();
-  double s[ND];  // all values' loads in flight at once, one barrier
+  // Eight partials of every value are requested before the first is added:
+  // this block is alone on the GPU here, and one load at a time made the
+  // tail of each sum grow by 0.6 us per load.
+  constexpr int LD = 8;
+  double s[ND];
 #pragma unroll
   for (int d = 0; d < ND; ++d) s[d] = 0.0;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += LD * blockDim.x) {
+    double t[ND][LD];
 #pragma unroll
-    for (int d = 0; d < ND; ++d) s[d] += __ldcg(part + d * gridDim.x + b);
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+      for (int k = 0; k < LD; ++k) {
+        const int bb = b + k * (int)blockDim.x;
+        t[d][k] = bb < (int)gridDim.x ? __ldcg(part + d * gridDim.x + bb) : 0.0;
+      }
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+#pragma unroll
+      for (int k = 0; k < LD; ++k) s[d] += t[d][k];
+  }
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
     for (int o = 16; o > 0; o >>= 1) s[d] += __shfl_xor_sync(0xffffffffu, s[d], o);
@@ -446,28 +499,33 @@ k_cg_q(MeshDev m, const V *__restrict__ slots, V *__restrict__ p, V *__restrict_
   }
   pdl_wait();
   pdl_trigger();
-  if (S->status) return;
+  // every load of the usual case (at most MS slots a node) in flight before
+  // the status is looked at
+  const int status = S->status;
   const V bt = (V)S->beta;
   double v[1] = {0.0};
-  V pn[U], zn[U];
+  V pn[U], zn[U], y[U][MS];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long long n = base + (long long)u * blockDim.x;
     pn[u] = zn[u] = 0;
     if (b[u] != en[u]) { pn[u] = p[n]; zn[u] = z[n]; }
+#pragma unroll
+    for (int k = 0; k < MS; ++k) y[u][k] = b[u] + k < en[u] ? slots[b[u] + k] : (V)0;
   }
+  if (status) return;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long long n = base + (long long)u * blockDim.x;
     V sum = 0, cmp = 0;
     for (int s0 = b[u]; s0 < en[u]; s0 += MS) {
-      V y[MS];
+      if (s0 != b[u])
 #pragma unroll
-      for (int k = 0; k < MS; ++k) y[k] = s0 + k < en[u] ? slots[s0 + k] : (V)0;
+        for (int k = 0; k < MS; ++k) y[u][k] = s0 + k < en[u] ? slots[s0 + k] : (V)0;
 #pragma unroll
       for (int k = 0; k < MS; ++k) {
         if (s0 + k >= en[u]) break;
-        const V yy = y[k] - cmp;
+        const V yy = y[u][k] - cmp;
         const V tt = sum + yy;
         cmp = (tt - sum) - yy;
         sum = tt;
@@ -517,7 +575,7 @@ k_cg_update(long long npoin, const double *__restrict__ p, const double *__restr
   }
   pdl_wait();
   pdl_trigger();
-  if (S->status) return;
+  const int status = S->status;
   const double a = S->alpha;
   double v[3] = {0.0, 0.0, 0.0};
   double pv[U], qv[U], xv[U], rv[U];
@@ -526,6 +584,7 @@ k_cg_update(long long npoin, const double *__restrict__ p, const double *__restr
     const long long i = base + (long long)u * blockDim.x;
     if (i < npoin) { pv[u] = p[i]; qv[u] = q[i]; xv[u] = x[i]; rv[u] = r[i]; }
   }
+  if (status) return;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long long i = base + (long long)u * blockDim.x;
@@ -579,7 +638,7 @@ k_cg_update32(long long npoin, const float *__restrict__ p, const float *__restr
   }
   pdl_wait();
   pdl_trigger();
-  if (S->status) return;
+  const int status = S->status;
   const float a = (float)S->alpha;
   double v[3] = {0.0, 0.0, 0.0};
   float pv[U], qv[U], xv[U], rv[U];
@@ -588,6 +647,7 @@ k_cg_update32(long long npoin, const float *__restrict__ p, const float *__restr
     const long long i = base + (long long)u * blockDim.x;
     if (mv[u] != 0.f) { pv[u] = p[i]; qv[u] = q[i]; xv[u] = x[i]; rv[u] = r[i]; }
   }
+  if (status) return;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long long i = base + (long long)u * blockDim.x;

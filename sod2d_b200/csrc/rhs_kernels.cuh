@@ -58,7 +58,7 @@ struct MeshDev {
   const float *Dnat;    // [N1][N1]
   const float *Drot;    // [2][N1][8]: rows, then columns, of Dnat rotated to start at the
                         // diagonal: D[c][(c+s) % N1], D[(c+s) % N1][c], s = 0..P
-  const double *D64;    // [2][N1][8]: rows, then columns, of Dnat in FP64
+  const double *D64;    // Drot in FP64
   const int *lpoin_w;   // 0-based
   const float *invMl;   // [npoin]
   const int *slot_ptr;  // [npoin+1]

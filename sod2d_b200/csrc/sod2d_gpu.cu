@@ -59,8 +59,8 @@ int sod_gpu_init(const sod_mesh_t *mesh, const sod_phys_t *phys, sod_gpu_ctx **o
     for (int s = 0; s < N1; ++s) {
       Drot[8 * a + s] = D[a * N1 + (a + s) % N1];
       Drot[8 * (N1 + a) + s] = D[((a + s) % N1) * N1 + a];
-      D64[8 * a + s] = D[a * N1 + s];
-      D64[8 * (N1 + a) + s] = D[s * N1 + a];
+      D64[8 * a + s] = Drot[8 * a + s];
+      D64[8 * (N1 + a) + s] = Drot[8 * (N1 + a) + s];
     }
   std::vector<int> conn((size_t)E * N);
   std::vector<float> geo((size_t)E * 10 * N);
@@ -93,6 +93,7 @@ int sod_gpu_init(const sod_mesh_t *mesh, const sod_phys_t *phys, sod_gpu_ctx **o
   sod_gpu_ctx *c = new sod_gpu_ctx();
   c->P = P; c->N1 = N1; c->N = N; c->nelem = mesh->nelem; c->npoin = mesh->npoin; c->npoin_w = mesh->npoin_w;
   c->phys = *phys;
+  std::copy(D.begin(), D.end(), c->D_h);
   c->ph.gm1 = phys->gamma_gas - 1.0f;
   c->ph.gogm1 = phys->gamma_gas / (phys->gamma_gas - 1.0f);
   c->ph.Rgas = phys->Rgas; c->ph.Cp = phys->Cp; c->ph.Prt = phys->Prt;

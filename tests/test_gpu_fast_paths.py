@@ -1,0 +1,164 @@
+"""The device-resident solves, the line-per-thread Laplacian and the
+programmatic launches at the sizes where they can go wrong: remainders of a
+block's elements, edges of a batch of iterations, one iteration, stream
+capture.  The oracle (oracle/) is the reference."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle as O
+from sod2d_b200 import host
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from sod2d_b200 import gpu as g
+    return g
+
+
+def dv(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def rel_l2(a, b):
+    return float(np.linalg.norm(np.asarray(a, np.float64) - b) / np.linalg.norm(b))
+
+
+# blocks of the Laplacian take 4 (order 3) or 2 (order 4) elements: 27, 30
+# and 36 elements leave 3, 2 and 0 (order 3), 27 one (order 4)
+@pytest.mark.parametrize("porder,size", [(3, (3, 3, 3)), (3, (3, 5, 2)), (3, (3, 3, 4)), (4, (3, 3, 3)), (4, (2, 2, 3))])
+def test_laplacian_block_remainders(gpu, porder, size):
+    m = host.periodic_cube(porder, *size, jitter=0.05, seed=4, elem_shuffle=True, ordering=1)
+    ctx = gpu.Context(m, gpu.default_phys())
+    w = m.lpoin_w - 1
+    p = np.zeros(m.npoin)
+    p[w] = np.random.default_rng(1).normal(size=w.size)
+    ref = O.laplacian(O.OracleMesh(m, np.float64), p)
+    # the oracle forms its FP64 geometry from the FP32 coordinates: 1e-6
+    out64 = torch.zeros(m.npoin, dtype=torch.float64, device="cuda")
+    ctx.call("sod_gpu_eval_laplacian_mult64", gpu.dptr(dv(p)), gpu.dptr(out64))
+    assert rel_l2(out64.cpu().numpy()[w], ref[w]) < 1e-6
+    out = torch.zeros(m.npoin, device="cuda")
+    p32 = p.astype(np.float32)
+    ref32 = O.laplacian(O.OracleMesh(m), p32)
+    ctx.call("sod_gpu_eval_laplacian_mult", gpu.dptr(dv(p32)), gpu.dptr(out))
+    # sums of 4 to 5 FP32 products in two passes and up to 8 contributions: a few ulp
+    assert rel_l2(out.cpu().numpy()[w], ref32[w]) < 2e-6
+    ctx.close()
+
+
+# batches of 20 iterations: one, a whole batch, one more, and convergence inside a batch
+@pytest.mark.parametrize("porder,maxit,tol", [(3, 1, 1e-6), (3, 20, 1e-6), (3, 21, 1e-6), (4, 45, 1e-7), (4, 200, 1e-3)])
+def test_fp32_pressure_cg_batches(gpu, porder, maxit, tol):
+    m = host.periodic_cube(porder, 3, 4, 5, jitter=0.05, seed=8, ordering=1, elem_shuffle=True)
+    om = O.OracleMesh(m)
+    ctx = gpu.Context(m, gpu.default_phys())
+    w = m.lpoin_w - 1
+    rng = np.random.default_rng(2)
+    p, x0 = np.zeros(m.npoin, np.float32), np.zeros(m.npoin, np.float32)
+    p[w] = rng.normal(size=w.size)
+    x0[w] = 0.1 * rng.normal(size=w.size)
+    b = O.laplacian(om, p)
+    ref_x, ref_it, ref_res = O.cg_pressure(om, O.laplacian_diag(om), x0, b, maxIter=maxit, tol=tol)
+    dR, it, res = dv(b.copy()), C.c_int(), C.c_double()
+    ctx.call("sod_gpu_conjgrad_pressure", gpu.dptr(dv(x0)), gpu.dptr(dR), maxit, tol, C.byref(it), C.byref(res))
+    assert abs(it.value - ref_it) <= (0 if maxit <= 21 else 1)
+    assert abs(res.value - ref_res) <= 0.05 * ref_res + 1e-7
+    # the error at the stop differs by what FP32 rounding has done to the
+    # directions: of the order of the residual there
+    assert rel_l2(dR.cpu().numpy()[w], ref_x[w]) < 1e-4
+    ctx.close()
+
+
+def test_fp32_pressure_cg_zero_rhs_is_refused(gpu):
+    """A zero residual gives 0/0 in the reference's alpha: reported as before."""
+    m = host.periodic_cube(3, 2)
+    ctx = gpu.Context(m, gpu.default_phys())
+    z, R = torch.zeros(m.npoin, device="cuda"), torch.zeros(m.npoin, device="cuda")
+    rc = gpu.lib().sod_gpu_conjgrad_pressure(ctx.h, gpu.dptr(z), gpu.dptr(R), 20, 1e-2, None, None)
+    assert rc == -4
+    ctx.close()
+
+
+# the IMEX solve reads its scalars every second iteration
+@pytest.mark.parametrize("porder,maxit", [(3, 1), (3, 3), (4, 4)])
+def test_imex_iteration_batches(gpu, porder, maxit):
+    m = host.periodic_cube(porder, 3, 4, 5)
+    ic = host.tgv_comp_init(m, Ma=1.25)
+    prm = O.comp_params(ic, cfl_conv=0.95, cfl_diff=1000.5, stages=4, imex=True, first_mue=True, imex_maxiter=maxit,
+                        imex_tol=1e-12)
+    ref_hist, ref_fin = O.tgv_comp_run(O.OracleMesh(m), ic, prm, 3)
+    s = gpu.CompSolver(m, ic, stages=4, fp64_state=False, cfl_conv=0.95, cfl_diff=1000.5, imex=True,
+                       imex_maxiter=maxit, imex_tol=1e-12)
+    s.run(3)
+    fin = s.state()
+    its = C.c_int()
+    s.ctx.call("sod_gpu_comp_imex_stats", C.byref(its), None)
+    s.close()
+    assert its.value == 3 * maxit
+    w = m.lpoin_w - 1
+    for k in ("rho", "E"):
+        assert rel_l2(fin[k][w], ref_fin[k][w]) < 1e-5, k
+
+
+@pytest.mark.parametrize("stages,fp64", [(3, True), (3, False), (4, True), (5, False)])
+def test_rk_levels_match_oracle(gpu, stages, fp64):
+    """Schemes whose stages read the first level at different places."""
+    m = host.periodic_cube(3, 3, 4, 5)
+    ic = host.tgv_comp_init(m, Ma=1.25)
+    _, ref_fin = O.tgv_comp_run(O.OracleMesh(m), ic, O.comp_params(ic, stages=stages, first_mue=True), 4)
+    s = gpu.CompSolver(m, ic, stages=stages, fp64_state=fp64)
+    s.run(4)
+    fin = s.state()
+    s.close()
+    w = m.lpoin_w - 1
+    for k in ("rho", "E"):
+        assert rel_l2(fin[k][w], ref_fin[k][w]) < 1e-5, k
+
+
+@pytest.mark.parametrize("porder,n", [(3, 4), (4, 3)])
+def test_rhs_under_capture(gpu, porder, n):
+    """sod_gpu_updateF in asynchronous mode recorded into a graph on a stream
+    of its own gives the eager call's values, for new inputs too."""
+    m = host.periodic_cube(porder, n, jitter=0.05, seed=3)
+    ic = host.tgv_comp_init(m, Ma=0.1)
+    ctx = gpu.Context(m, gpu.phys_from_ic(ic))
+    N = m.npoin
+    f = [dv(a) for a in host.random_comp_state(m, seed=5)]
+    mu_e, tau = torch.rand(m.nelem * m.nnode, device="cuda") * 1e-3, torch.rand(m.nelem, device="cuda")
+    out = [torch.zeros(k * N, device="cuda") for k in (1, 3, 1)]
+
+    def call():
+        ctx.call("sod_gpu_updateF", *(gpu.dptr(t) for t in f), gpu.dptr(mu_e), float(ic.mu_factor), gpu.dptr(tau),
+                 *(gpu.dptr(t) for t in out), None, None, None, None)
+
+    call()
+    eager = [t.clone() for t in out]
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    ctx.call("sod_gpu_set_stream", C.c_void_p(st.cuda_stream))
+    ctx.call("sod_gpu_set_async", 1)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        call()
+    for t in out:
+        t.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(out, eager))
+    for a, b in zip(f, host.random_comp_state(m, seed=6)):
+        a.copy_(dv(b))
+    g.replay()
+    torch.cuda.synchronize()
+    replayed = [t.clone() for t in out]
+    ctx.call("sod_gpu_set_async", 0)
+    ctx.call("sod_gpu_set_stream", None)
+    call()
+    assert all(torch.equal(a, b) for a, b in zip(out, replayed))
+    ctx.close()
