@@ -480,9 +480,9 @@ int imex_stage_dev(sod_gpu_ctx *c, int is, const ImexCoef &K, float dt, int maxI
   const unsigned nb = nblk(N, IMEX_THREADS);
   const float gm1 = c->phys.gamma_gas - 1.0f, Rgas = c->phys.Rgas, fact = K.ai[is][is];
   const cudaStream_t st = c->stream;
-  k_imex_start<<<nb, IMEX_THREADS, 0, st>>>(N, c->is_work, is, K, dt, fact, gm1, Rgas, tol, c->Ml, X.R, X.D, X.stab,
-                                            X.lvl1, X.Dx0, S.rho32, S.E32, S.q32, X.x, X.r, X.p, X.au, X.aT, G.S,
-                                            G.gpart, G.ticket);
+  (is == 2 ? k_imex_start<2> : is == 3 ? k_imex_start<3> : k_imex_start<4>)<<<nb, IMEX_THREADS, 0, st>>>(
+      N, c->is_work, K, dt, fact, gm1, Rgas, tol, c->Ml, X.R, X.D, X.stab, X.lvl1, X.Dx0, S.rho32, S.E32, S.q32, X.x,
+      X.r, X.p, X.au, X.aT, G.S, G.gpart, G.ticket);
   RhsArgs A{};
   A.rho = X.p; A.rho_n = X.x; A.u = X.au; A.Tem = X.aT; A.mu_fluid = S.mu_fluid; A.mue_t = c->mue_t;
   A.fact_d = 1.0f;

@@ -135,9 +135,12 @@ constexpr int IMEX_THREADS = 256;
 
 // Stage right-hand side (k_imex_comb), x = x0 = level 1, r = b - (x0 Ml +
 // fact dt D(x0)), p = r / M with its velocity and temperature; ||r||^2 and
-// r.z start the scalars.
-static __global__ void __launch_bounds__(IMEX_THREADS)
-k_imex_start(long long npoin, const int *__restrict__ work, int is, ImexCoef k, float dt, float fact, float gm1,
+// r.z start the scalars.  One instantiation per stage: with the stage loop
+// unrolled all its loads are in flight together (a runtime loop walked them
+// two at a time: 104 us at 32^3, stage mean).
+template <int is>
+__global__ void __launch_bounds__(IMEX_THREADS)
+k_imex_start(long long npoin, const int *__restrict__ work, ImexCoef k, float dt, float fact, float gm1,
              float Rgas, double tol, const float *__restrict__ Ml, const float *__restrict__ R,
              const float *__restrict__ D, const float *__restrict__ stab, const float *__restrict__ lvl1,
              const float *__restrict__ Dx0, float *__restrict__ rho2, float *__restrict__ E2, float *__restrict__ q2,
@@ -150,22 +153,30 @@ k_imex_start(long long npoin, const int *__restrict__ work, int is, ImexCoef k, 
     const float ml = Ml[n], M = __fdiv_rn(ml, dt);
     const bool w = work[n] != 0;
     float *out[5] = {rho2, E2, q2, q2 + npoin, q2 + 2 * npoin};
-    float pv[5], x0 = 0.f;
+    float pv[5], x0 = 0.f, st[5], lv[5], dx[5], Rv[is - 1][5], Dv[is - 1][5];
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
       const long long o = n + npoin * f;
-      float a = __fmul_rn(-dt, stab[o]);
+      st[f] = stab[o]; lv[f] = lvl1[o]; dx[f] = Dx0[o];
+#pragma unroll
+      for (int js = 0; js < is - 1; ++js) { Rv[js][f] = R[js * B + o]; Dv[js][f] = D[js * B + o]; }
+    }
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
+      const long long o = n + npoin * f;
+      float a = __fmul_rn(-dt, st[f]);
+#pragma unroll
       for (int js = 1; js < is; ++js) {
-        a = __fsub_rn(a, __fmul_rn(__fmul_rn(dt, k.ae[is][js]), R[(js - 1) * B + o]));
-        a = __fsub_rn(a, __fmul_rn(__fmul_rn(dt, k.ai[is][js]), D[(js - 1) * B + o]));
+        a = __fsub_rn(a, __fmul_rn(__fmul_rn(dt, k.ae[is][js]), Rv[js - 1][f]));
+        a = __fsub_rn(a, __fmul_rn(__fmul_rn(dt, k.ai[is][js]), Dv[js - 1][f]));
       }
-      const float l1 = lvl1[o], xm = __fmul_rn(l1, ml), bb = __fadd_rn(a, xm);
+      const float l1 = lv[f], xm = __fmul_rn(l1, ml), bb = __fadd_rn(a, xm);
       if (!w) {
         out[f][n] = bb;
         continue;
       }
       if (f == 0) x0 = l1;
-      const float rr = __fsub_rn(bb, __fadd_rn(xm, __fmul_rn(__fmul_rn(Dx0[o], fact), dt)));
+      const float rr = __fsub_rn(bb, __fadd_rn(xm, __fmul_rn(__fmul_rn(dx[f], fact), dt)));
       pv[f] = __fdiv_rn(rr, M);
       x[o] = l1;
       r[o] = rr;
