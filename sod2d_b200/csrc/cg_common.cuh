@@ -72,11 +72,11 @@ template <class V>
 inline void lap(sod_gpu_ctx *c, const V *p, V *out) {
   dispatch(c, [&](auto L) {
     constexpr int P = decltype(L)::P_;
-    k_lap_elem<P, V><<<nblk(c->nelem, LapCfg<P>::EPB), 32 * LAP_WARPS, 0, c->stream>>>(c->md(), dmat<P, V>(c), p,
-                                                                                      (V *)c->slotsB);
+    launch_pdl(k_lap_elem<P, V>, nblk(c->nelem, LapCfg<P>::EPB), 32 * LAP_WARPS, 0, c->stream, c->md(), dmat<P, V>(c), p,
+               (V *)c->slotsB, nullptr, nullptr, nullptr);
     return 0;
   });
-  k_gather1<V><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), (const V *)c->slotsB, out, 0);
+  launch_pdl(k_gather_sorted1<V>, nblk(c->npoin, 256), 256, 0, c->stream, c->md(), (const V *)c->slotsB, out, 0);
 }
 
 // Dot products over the working nodes, or over the owned ones on a
@@ -101,7 +101,7 @@ inline int ensure_diag(sod_gpu_ctx *c) {
     k_lap_diag_elem<LL::P_><<<nblk(EN, 256), 256, 0, c->stream>>>(c->md(), c->slotsB);
     return 0;
   });
-  k_gather1<float><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, G.diag, 0);
+  k_gather_sorted1<float><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, G.diag, 0);
   if ((rc = halo_sum(c, halo_soa_view(c, G.diag, 1)))) return rc;  // mod_operators.f90:677
   G.have_diag = true;
   return 0;

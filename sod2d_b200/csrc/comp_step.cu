@@ -134,7 +134,7 @@ int sod_gpu_generic_scalar_convec_ijk(sod_gpu_ctx *c, const float *q, const floa
                                                                                         nullptr, c->slotsB, fact);
     return 0;
   });
-  k_gather_sorted1<<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, R, initialze ? 0 : 1);
+  k_gather_sorted1<float><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, R, initialze ? 0 : 1);
   return c->finish();
 }
 

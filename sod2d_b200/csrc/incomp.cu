@@ -8,7 +8,6 @@ extern "C" {
 
 int sod_gpu_eval_laplacian_mult(sod_gpu_ctx *c, const float *p, float *ResP) {
   if (!c || !p || !ResP) return fail(SOD_GPU_EINVAL, "bad argument");
-  CUDA_TRY(cudaMemsetAsync(ResP, 0, (size_t)c->npoin * 4, c->stream));
   lap<float>(c, p, ResP);
   int rc = halo_sum(c, halo_soa_view(c, ResP, 1));  // mod_operators.f90:102
   return rc ? rc : c->finish();
@@ -16,7 +15,6 @@ int sod_gpu_eval_laplacian_mult(sod_gpu_ctx *c, const float *p, float *ResP) {
 
 int sod_gpu_eval_laplacian_mult64(sod_gpu_ctx *c, const double *p, double *ResP) {
   if (!c || !p || !ResP) return fail(SOD_GPU_EINVAL, "bad argument");
-  CUDA_TRY(cudaMemsetAsync(ResP, 0, (size_t)c->npoin * 8, c->stream));
   lap<double>(c, p, ResP);
   HaloViewT<double> hv{};
   hv.width = 1;
@@ -38,13 +36,10 @@ int sod_gpu_eval_gradient(sod_gpu_ctx *c, const float *x, float *gradX) {
   if (!c || !x || !gradX) return fail(SOD_GPU_EINVAL, "bad argument");
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_vec_elem<LL::P_, LL::EPB, 0><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), x, nullptr, nullptr, c->slotsB);
+    launch_pdl(k_vec_elem<LL::P_, LL::EPB, 0>, LL::grid(c->nelem), LL::TPB, 0, c->stream, c->md(), x, nullptr, nullptr, c->slotsB);
     return 0;
   });
-  OutPtrs o{};
-  const long long N = c->npoin;
-  o.p[0] = gradX; o.p[1] = gradX + N; o.p[2] = gradX + 2 * N;
-  k_gather<4, 3, false><<<nblk(N, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, nullptr, o, 0, 1);
+  launch_pdl(k_gather_sorted3, nblk(c->npoin, 256), 256, 0, c->stream, c->md(), c->slotsB, gradX, 1);
   int rc = halo_sum(c, halo_soa_view(c, gradX, 3));  // mod_operators.f90:274
   return rc ? rc : c->finish();
 }
@@ -53,12 +48,10 @@ int sod_gpu_eval_divergence(sod_gpu_ctx *c, const float *u, float *divU) {
   if (!c || !u || !divU) return fail(SOD_GPU_EINVAL, "bad argument");
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_vec_elem<LL::P_, LL::EPB, 1><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), nullptr, u, nullptr, c->slotsB);
+    launch_pdl(k_vec_elem<LL::P_, LL::EPB, 1>, LL::grid(c->nelem), LL::TPB, 0, c->stream, c->md(), nullptr, u, nullptr, c->slotsB);
     return 0;
   });
-  OutPtrs o{};
-  o.p[0] = divU;
-  k_gather<4, 1, false><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, nullptr, o, 0, 0);
+  launch_pdl(k_gather_sorted1<float>, nblk(c->npoin, 256), 256, 0, c->stream, c->md(), c->slotsB, divU, 0);
   int rc = halo_sum(c, halo_soa_view(c, divU, 1));  // mod_operators.f90:566
   return rc ? rc : c->finish();
 }
@@ -67,13 +60,10 @@ int sod_gpu_full_convec_ijk_incomp(sod_gpu_ctx *c, const float *u, const float *
   if (!c || !u || !q || !Rmom) return fail(SOD_GPU_EINVAL, "bad argument");
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_vec_elem<LL::P_, LL::EPB, 2><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), nullptr, u, q, c->slotsB);
+    launch_pdl(k_vec_elem<LL::P_, LL::EPB, 2>, LL::grid(c->nelem), LL::TPB, 0, c->stream, c->md(), nullptr, u, q, c->slotsB);
     return 0;
   });
-  OutPtrs o{};
-  const long long N = c->npoin;
-  o.p[0] = Rmom; o.p[1] = Rmom + N; o.p[2] = Rmom + 2 * N;
-  k_gather<4, 3, false><<<nblk(N, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, nullptr, o, 0, 0);
+  launch_pdl(k_gather_sorted3, nblk(c->npoin, 256), 256, 0, c->stream, c->md(), c->slotsB, Rmom, 0);
   return c->finish();
 }
 
@@ -672,13 +662,13 @@ int ensure_velo(sod_gpu_ctx *c) {
 }
 
 // LPS projection of v into V.tauP (node-major, mass-divided)
-int velo_tau(sod_gpu_ctx *c, const float *v) {
+int velo_tau(sod_gpu_ctx *c, const float *v, const int *stop = nullptr) {
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_tauv_elem<LL::P_, LL::EPB><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), v, c->slotsB);
+    launch_pdl(k_tauv_elem<LL::P_, LL::EPB>, LL::grid(c->nelem), LL::TPB, 0, c->stream, c->md(), v, c->slotsB, stop);
     return 0;
   });
-  k_gather_tauv<<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, c->Ml, c->velo.tauP);
+  launch_pdl(k_gather_tauv, nblk(c->npoin, 256), 256, 0, c->stream, c->md(), c->slotsB, c->Ml, c->velo.tauP, stop);
   // halo sum of the six projected components (mod_operators.f90:467-469)
   HaloView hv{};
   hv.width = 6;
@@ -687,19 +677,22 @@ int velo_tau(sod_gpu_ctx *c, const float *v) {
   return halo_sum(c, hv);
 }
 
-// out (npoin,3) = full_diff_stab_incomp(v) with the projection in V.tauP
-void velo_diff(sod_gpu_ctx *c, const float *v, const float *mu_fluid, const float *musgs_t, const float *tau_e,
-               float *out) {
+// full_diff_stab_incomp(v) with the projection in V.tauP, into slotsB
+void velo_diff_elem(sod_gpu_ctx *c, const float *v, const float *mu_fluid, const float *musgs_t, const float *tau_e,
+                    const int *stop = nullptr) {
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_diffv_elem<LL::P_, LL::EPB><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), v, mu_fluid, musgs_t,
-                                                                                c->velo.tauP, tau_e, c->slotsB);
+    launch_pdl(k_diffv_elem<LL::P_, LL::EPB>, LL::grid(c->nelem), LL::TPB, 0, c->stream, c->md(), v, mu_fluid, musgs_t,
+               c->velo.tauP, tau_e, c->slotsB, stop);
     return 0;
   });
-  OutPtrs o{};
-  const long long N = c->npoin;
-  o.p[0] = out; o.p[1] = out + N; o.p[2] = out + 2 * N;
-  k_gather<4, 3, false><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, nullptr, o, 0, 0);
+}
+
+// the same, assembled into out (npoin,3)
+void velo_diff(sod_gpu_ctx *c, const float *v, const float *mu_fluid, const float *musgs_t, const float *tau_e,
+               float *out) {
+  velo_diff_elem(c, v, mu_fluid, musgs_t, tau_e);
+  launch_pdl(k_gather_sorted3, nblk(c->npoin, 256), 256, 0, c->stream, c->md(), c->slotsB, out, 0);
 }
 
 // FP64 sums of the products of two (npoin,3) vectors (two pairs at once)
@@ -719,6 +712,49 @@ int velo_dots(sod_gpu_ctx *c, const float *a0, const float *b0, const float *c0,
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   h[0] = (t[0] + t[1]) + t[2];
   h[1] = (t[3] + t[4]) + t[5];
+  return 0;
+}
+
+// conjGrad_veloc_incomp with its scalars on the device (single rank): seven
+// launches per iteration without a host read, where eleven and three reads
+// took twice as long; the scalars are read after four iterations (a step
+// takes three to five).
+int conjgrad_veloc_dev(sod_gpu_ctx *c, float fact, float dt, const float *mu_fluid, const float *musgs, int maxIter,
+                       double tol, int *iters, double *res_rel) {
+  int rc;
+  if ((rc = ensure_cg_loop(c))) return rc;
+  auto &V = c->velo;
+  auto &G = c->cg;
+  const long long N = c->npoin;
+  const unsigned nb = nblk(N, VELO_THREADS);
+  const cudaStream_t st = c->stream;
+  auto apply = [&](const float *v, const int *stop) {
+    velo_tau(c, v, stop);
+    velo_diff_elem(c, v, mu_fluid, musgs, V.tau_e, stop);
+  };
+  apply(V.x, nullptr);
+  launch_pdl(k_veloc_gather_op<true>, nb, VELO_THREADS, 0, st, c->md(), c->is_work, c->slotsB, c->Ml, fact, dt, tol,
+             V.x, V.b, V.q, V.r, V.p, G.S, G.gpart, G.ticket);
+  int it = 0;
+  while (it < maxIter) {
+    const int it0 = it, nbat = std::min(4, maxIter - it);
+    for (int k = 0; k < nbat; ++k) {
+      apply(V.p, &G.S->status);
+      launch_pdl(k_veloc_gather_op<false>, nb, VELO_THREADS, 0, st, c->md(), c->is_work, c->slotsB, c->Ml, fact, dt,
+                 tol, V.p, V.b, V.q, V.r, V.p, G.S, G.gpart, G.ticket);
+      launch_pdl(k_veloc_update, nb, VELO_THREADS, 0, st, N, c->is_work, c->Ml, dt, V.p, V.q, V.x, V.r, G.S, G.gpart,
+                 G.ticket);
+      launch_pdl(k_veloc_dir, nb, VELO_THREADS, 0, st, N, c->is_work, c->Ml, dt, V.r, V.p, G.S);
+    }
+    CUDA_TRY(cudaMemcpyAsync(G.S_h, G.S, sizeof(CgScal), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    it = G.S_h->iter;
+    if (G.S_h->status == 3) return fail(SOD_GPU_ENONFINITE, "non-finite residual in velocity CG");
+    if (G.S_h->status == 1) break;
+    if (it == it0) return fail(SOD_GPU_ECUDA, "velocity CG did not advance");
+  }
+  if (iters) *iters = it;
+  if (res_rel) *res_rel = G.S_h->bnorm > 0 ? std::sqrt(G.S_h->rr) / G.S_h->bnorm : 0.0;
   return 0;
 }
 
@@ -782,6 +818,13 @@ int sod_gpu_conjgrad_veloc(sod_gpu_ctx *c, float fact, float dt, const float *mu
   CUDA_TRY(cudaMemcpyAsync(V.b, R, 3 * N * 4, cudaMemcpyDeviceToDevice, c->stream));
   k_species_tau<<<nblk(c->nelem, 8), 256, 0, c->stream>>>(c->nelem, c->N, c->conn, c->helem, V.x, N,
                                                           c->phys.c_species_stab / (float)c->P, V.tau_e);
+  if (!c->halo.on) {
+    rc = conjgrad_veloc_dev(c, fact, dt, mu_fluid, musgs, maxIter, tol, iters, res_rel);
+    c->async = was_async;
+    if (rc) return rc;
+    CUDA_TRY(cudaMemcpyAsync(R, V.x, 3 * N * 4, cudaMemcpyDeviceToDevice, c->stream));
+    return c->finish();
+  }
   auto apply = [&](const float *v) {  // q = v Ml + fact dt D(v)
     int arc = velo_tau(c, v);
     if (arc) return arc;

@@ -30,11 +30,10 @@ struct DMat {
 
 // ---- Laplacian: ResP = sum_e int grad N . grad p  (mod_operators.f90:16-112)
 // V = float (reference arithmetic) or double.  Writes one V per element node
-// into slots (width 1), element-ordered.
+// into node-sorted slots (slot_pos), which the assembly sums contiguously.
 // DIR (the CG iteration): the operand is the new search direction
 // z + beta p, formed on the fly from z, the previous p and *beta (the
-// update p = z + beta p itself is stored by k_cg_q), and the slots are
-// written node-sorted (slot_pos) for k_cg_q's contiguous sums.
+// update p = z + beta p itself is stored by k_cg_q).
 //
 // A thread owns the line of P + 1 points along zeta over its (i, j); 16
 // lanes (P = 3) or 25 of 32 (P = 4) take an element, so nothing but warp
@@ -74,7 +73,7 @@ k_lap_elem(MeshDev m, DMat<P, V> D, const V *__restrict__ p, V *__restrict__ slo
 #pragma unroll
     for (int k = 0; k < N1; ++k) {
       n[k] = m.conn[b + N2 * k];
-      if (DIR) pos[k] = m.slot_pos[b + N2 * k];
+      pos[k] = m.slot_pos[b + N2 * k];
     }
     const float *g = m.geo + e * 10 * N + c;
 #pragma unroll
@@ -144,25 +143,57 @@ k_lap_elem(MeshDev m, DMat<P, V> D, const V *__restrict__ p, V *__restrict__ slo
       const int mm = ref_order<P>(q);
       acc += D.d[mm][k] * C2[mm];
     }
-    slots[DIR ? (long long)pos[k] : e * N + c + N2 * k] = acc;
+    slots[pos[k]] = acc;
   }
 }
 
-// Scalar-slot assembly out(p) = scale * sum(slots of p); float sums are
-// Kahan-compensated.  Only nodes with slots are written (masters).
+// Scalar node-sorted slots: out(p) = their Kahan sum in element order, onto
+// out(p) when accumulate is set.
 template <class V>
-__global__ void k_gather1(MeshDev m, const V *__restrict__ slots, V *__restrict__ out, int use_invMl) {
+__global__ void k_gather_sorted1(MeshDev m, const V *__restrict__ slots, V *__restrict__ out, int accumulate) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= m.npoin) return;
   const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
-  V sum = 0, cmp = 0;
+  pdl_wait();
+  pdl_trigger();
+  V sum = accumulate ? out[p] : (V)0, cmp = 0;
   for (int s = b; s < en; ++s) {
-    const V y = slots[m.slot_idx[s]] - cmp;
+    const V y = slots[s] - cmp;
     const V tt = sum + y;
     cmp = (tt - sum) - y;
     sum = tt;
   }
-  out[p] = use_invMl ? sum * (V)m.invMl[p] : sum;
+  out[p] = sum;
+}
+
+// Three values of a node from 4-wide node-sorted slots, the same sums.
+__device__ __forceinline__ void node_sum3(const float4 *__restrict__ s4, int b, int en, float (&sum)[3]) {
+  float cmp[3] = {0.f, 0.f, 0.f};
+  sum[0] = sum[1] = sum[2] = 0.f;
+  for (int s = b; s < en; ++s) {
+    const float4 v = s4[s];
+    const float x[3] = {v.x, v.y, v.z};
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const float y = x[f] - cmp[f];
+      const float tt = sum[f] + y;
+      cmp[f] = (tt - sum[f]) - y;
+      sum[f] = tt;
+    }
+  }
+}
+static __global__ void k_gather_sorted3(MeshDev m, const float *__restrict__ slots, float *__restrict__ out,
+                                        int use_invMl) {
+  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= m.npoin) return;
+  const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
+  const float sc = use_invMl ? m.invMl[p] : 1.f;
+  pdl_wait();
+  pdl_trigger();
+  float sum[3];
+  node_sum3(reinterpret_cast<const float4 *>(slots), b, en, sum);
+#pragma unroll
+  for (int f = 0; f < 3; ++f) out[p + m.npoin * f] = sum[f] * sc;
 }
 
 // ---- eval_laplacian_diag, mod_operators.f90:638-682 --------------------
@@ -179,28 +210,39 @@ __global__ void k_lap_diag_elem(MeshDev m, float *__restrict__ slots) {
   const int ia = a % N1, ja = (a / N1) % N1, ka = a / (N1 * N1);
   const float *g = m.geo + e * 10 * N;
   float d = 0.f;
-  for (int gp = 0; gp < N; ++gp) {
-    const int i = gp % N1, j = (gp / N1) % N1, k = gp / (N1 * N1);
+  auto add = [&](int i, int j, int k) {
+    const int gp = i + N1 * (j + N1 * k);
     // iso-derivatives of N_a at gp: D[i][ia] d_{j,ja} d_{k,ka}, ...
-    float d0 = (j == ja && k == ka) ? m.Dnat[i * N1 + ia] : 0.f;
-    float d1 = (i == ia && k == ka) ? m.Dnat[j * N1 + ja] : 0.f;
-    float d2 = (i == ia && j == ja) ? m.Dnat[k * N1 + ka] : 0.f;
-    if (d0 == 0.f && d1 == 0.f && d2 == 0.f) continue;
+    const float d0 = (j == ja && k == ka) ? m.Dnat[i * N1 + ia] : 0.f;
+    const float d1 = (i == ia && k == ka) ? m.Dnat[j * N1 + ja] : 0.f;
+    const float d2 = (i == ia && j == ja) ? m.Dnat[k * N1 + ka] : 0.f;
+    if (d0 == 0.f && d1 == 0.f && d2 == 0.f) return;
     const float gv = g[9 * N + gp];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const float gc = g[c * N + gp] * d0 + g[(c + 3) * N + gp] * d1 + g[(c + 6) * N + gp] * d2;
       d += gv * gc * gc;
     }
+  };
+  // the points of the three lines in ascending order; testing all N of an
+  // element for each of its nodes took 390 us at 8,000 order-4 elements
+  for (int k = 0; k < N1; ++k) {
+    if (k != ka) { add(ia, ja, k); continue; }
+    for (int j = 0; j < N1; ++j) {
+      if (j != ja) { add(ia, j, k); continue; }
+      for (int i = 0; i < N1; ++i) add(i, j, k);
+    }
   }
-  slots[idx] = d;
+  slots[m.slot_pos[idx]] = d;
 }
 
 // ---- gradient / divergence / incompressible convection ----------------
+// Node-sorted slots.
 // MODE 0: gradient of a scalar x: slots (width 4) = gpvol*grad x (3)
-// MODE 1: divergence of u: slot[0] = gpvol * div u
+// MODE 1: divergence of u: slots (width 1) = gpvol * div u
 // MODE 2: full_convec_ijk_incomp (elem_convec_incomp.f90:19-125): slots
 //         (width 4) = gpvol * 0.5*(div(q u) + u div q + (u.grad) q)
+// The mesh loads come before the programmatic wait and the staging barrier.
 template <int P, int EPB, int MODE>
 __global__ void __launch_bounds__(EPB *Cfg<P>::NT)
 k_vec_elem(MeshDev m, const float *__restrict__ x, const float *__restrict__ u, const float *__restrict__ q,
@@ -213,8 +255,19 @@ k_vec_elem(MeshDev m, const float *__restrict__ x, const float *__restrict__ u, 
   const bool active = (e < m.nelem) && (t < N);
   const long long NP = m.npoin;
   float ul[3] = {0.f, 0.f, 0.f}, ql[3] = {0.f, 0.f, 0.f};
+  int node = 0, pos = 0;
+  float He[9], gv = 0.f;
   if (active) {
-    const int node = m.conn[e * N + t];
+    node = m.conn[e * N + t];
+    pos = m.slot_pos[e * N + t];
+    const float *g = m.geo + e * 10 * N + t;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) He[c] = g[c * N];
+    gv = g[9 * N];
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (active) {
     if (MODE == 0) sm[el][0][t] = x[node];
     if (MODE >= 1)
       for (int d = 0; d < 3; ++d) { ul[d] = u[node + NP * d]; sm[el][d][t] = (MODE == 1) ? ul[d] : 0.f; }
@@ -230,11 +283,6 @@ k_vec_elem(MeshDev m, const float *__restrict__ x, const float *__restrict__ u, 
   float Di[N1], Dj[N1], Dk[N1];
 #pragma unroll
   for (int s = 0; s < N1; ++s) { Di[s] = m.Dnat[i * N1 + s]; Dj[s] = m.Dnat[j * N1 + s]; Dk[s] = m.Dnat[k * N1 + s]; }
-  const float *g = m.geo + e * 10 * N + t;
-  float He[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) He[c] = g[c * N];
-  const float gv = g[9 * N];
   float out[3] = {0.f, 0.f, 0.f};
   float a0, a1, a2;
   if (MODE == 0) {
@@ -273,7 +321,10 @@ k_vec_elem(MeshDev m, const float *__restrict__ x, const float *__restrict__ u, 
       out[a] = gv * r;
     }
   }
-  reinterpret_cast<float4 *>(slots + (e * N + t) * 4)[0] = make_float4(out[0], out[1], out[2], 0.f);
+  if (MODE == 1)
+    slots[pos] = out[0];
+  else
+    reinterpret_cast<float4 *>(slots)[pos] = make_float4(out[0], out[1], out[2], 0.f);
 }
 
 // ---- CG vector kernels (FP64 reductions, deterministic) ---------------

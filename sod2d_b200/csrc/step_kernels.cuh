@@ -243,22 +243,6 @@ __global__ void k_gather_entropy(MeshDev m, const float *__restrict__ slots, lon
   }
 }
 
-// Node sums of scalar node-sorted slots into (or onto) out, Kahan, element order.
-static __global__ void k_gather_sorted1(MeshDev m, const float *__restrict__ slots, float *__restrict__ out,
-                                        int accumulate) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= m.npoin) return;
-  const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
-  float sum = accumulate ? out[p] : 0.f, cmp = 0.f;
-  for (int s = b; s < en; ++s) {
-    const float y = slots[s] - cmp;
-    const float tt = sum + y;
-    cmp = (tt - sum) - y;
-    sum = tt;
-  }
-  out[p] = sum;
-}
-
 // auxReta = (1.5 R2 - 0.5 R1) + (eta2 - eta1)/dt; R1 <- R2 (time_integ_ls.f90:437-443)
 static __global__ void k_aux_reta(int npoin_w, const int *__restrict__ lpoin_w, float dt, float *__restrict__ Reta1,
                            const float *__restrict__ Reta2, const float *__restrict__ eta1,

@@ -6,7 +6,7 @@
 // (full_diff_stab_incomp).  Same element layout and deterministic
 // slot assembly as the other element kernels.
 #pragma once
-#include "rhs_kernels.cuh"
+#include "incomp_kernels.cuh"
 
 namespace sod {
 
@@ -29,25 +29,32 @@ static __global__ void k_species_tau(long long nelem, int N, const int *__restri
 }
 
 // Stage the 3 velocity components of an element and return grad u at the
-// thread's Gauss point (gradU[a][b] = d u_a / d x_b).
+// thread's Gauss point (gradU[a][b] = d u_a / d x_b).  The mesh loads come
+// before the programmatic wait; false: *stop is set, leave at once.
 template <int P, int EPB>
-__device__ __forceinline__ void stage_grad_u(const MeshDev &m, const float *__restrict__ u, float (*sm)[Cfg<P>::N],
+__device__ __forceinline__ bool stage_grad_u(const MeshDev &m, const float *__restrict__ u, float (*sm)[Cfg<P>::N],
                                              long long e, int t, bool active, float (&gradU)[3][3], float &gv,
-                                             float (&He)[9], int &node) {
+                                             float (&He)[9], int &node, int &pos, const int *__restrict__ stop) {
   constexpr int N1 = Cfg<P>::N1, N = Cfg<P>::N;
   const long long NP = m.npoin;
   if (active) {
     node = m.conn[e * N + t];
+    pos = m.slot_pos[e * N + t];
     const float *g = m.geo + e * 10 * N + t;
 #pragma unroll
     for (int c = 0; c < 9; ++c) He[c] = g[c * N];
     gv = g[9 * N];
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (stop && *stop) return false;
+  if (active) {
     sm[0][t] = u[node];
     sm[1][t] = u[node + NP];
     sm[2][t] = u[node + 2 * NP];
   }
   __syncthreads();
-  if (!active) return;
+  if (!active) return true;
   const int i = t % N1, j = (t / N1) % N1, k = t / (N1 * N1);
   float Di[N1], Dj[N1], Dk[N1];
 #pragma unroll
@@ -59,24 +66,24 @@ __device__ __forceinline__ void stage_grad_u(const MeshDev &m, const float *__re
   for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int b = 0; b < 3; ++b) gradU[a][b] = He[b] * gU[a][0] + He[b + 3] * gU[a][1] + He[b + 6] * gU[a][2];
+  return true;
 }
 
 // eval_tau_veloc, src/lib_sod2d_incomp/sources/mod_operators.f90:373-483,
 // element part: gpvol * (grad u + grad u^T), whose 6 distinct entries
-// (00 01 02 11 12 22) go to 8-wide slots.
+// (00 01 02 11 12 22) go to 8-wide node-sorted slots.
 template <int P, int EPB>
 __global__ void __launch_bounds__(EPB *Cfg<P>::NT)
-k_tauv_elem(MeshDev m, const float *__restrict__ u, float *__restrict__ slots) {
+k_tauv_elem(MeshDev m, const float *__restrict__ u, float *__restrict__ slots, const int *__restrict__ stop) {
   constexpr int N = Cfg<P>::N, NT = Cfg<P>::NT;
   __shared__ __align__(16) float sm[EPB][3][N];
   const int el = threadIdx.x / NT, t = threadIdx.x % NT;
   const long long e = (long long)blockIdx.x * EPB + el;
   const bool active = (e < m.nelem) && (t < N);
   float gradU[3][3], gv = 0.f, He[9];
-  int node = 0;
-  stage_grad_u<P, EPB>(m, u, sm[el], e, t, active, gradU, gv, He, node);
-  if (!active) return;
-  float4 *o = reinterpret_cast<float4 *>(slots + (e * N + t) * 8);
+  int node = 0, pos = 0;
+  if (!stage_grad_u<P, EPB>(m, u, sm[el], e, t, active, gradU, gv, He, node, pos, stop) || !active) return;
+  float4 *o = reinterpret_cast<float4 *>(slots + (long long)pos * 8);
   o[0] = make_float4(gv * (gradU[0][0] + gradU[0][0]), gv * (gradU[0][1] + gradU[1][0]),
                      gv * (gradU[0][2] + gradU[2][0]), gv * (gradU[1][1] + gradU[1][1]));
   o[1] = make_float4(gv * (gradU[1][2] + gradU[2][1]), gv * (gradU[2][2] + gradU[2][2]), 0.f, 0.f);
@@ -86,13 +93,17 @@ k_tauv_elem(MeshDev m, const float *__restrict__ u, float *__restrict__ slots) {
 // lumped mass (lumped_solver_vect, mod_solver.f90:61-79), node-major
 // [npoin][8] (6 used); nodes without slots get 0.
 static __global__ void k_gather_tauv(MeshDev m, const float *__restrict__ slots, const float *__restrict__ Ml,
-                              float *__restrict__ tauP) {
+                              float *__restrict__ tauP, const int *__restrict__ stop) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= m.npoin) return;
   const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
+  const float ml = Ml[p];
+  pdl_wait();
+  pdl_trigger();
+  if (stop && *stop) return;
   float sum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, cmp[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int s = b; s < en; ++s) {
-    const float4 *v = reinterpret_cast<const float4 *>(slots + (long long)m.slot_idx[s] * 8);
+    const float4 *v = reinterpret_cast<const float4 *>(slots + (long long)s * 8);
     const float4 v0 = v[0], v1 = v[1];
     const float x[6] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y};
 #pragma unroll
@@ -104,7 +115,6 @@ static __global__ void k_gather_tauv(MeshDev m, const float *__restrict__ slots,
     }
   }
   if (b != en) {
-    const float ml = Ml[p];
 #pragma unroll
     for (int f = 0; f < 6; ++f) sum[f] = sum[f] / ml;
   }
@@ -136,20 +146,21 @@ static __global__ void k_pack_tauv(long long npoin, const float *__restrict__ GX
 // 12-153: fluxes F_r = (mu_fluid + mu_sgs + tau_e)(grad u + grad u^T)(r,:)
 // - tau_e TauP(r,:) at each Gauss point, their contravariant components
 // staged, then the weak divergence; 3 residuals per element node into
-// 4-wide slots.
+// 4-wide node-sorted slots.
 template <int P, int EPB>
 __global__ void __launch_bounds__(EPB *Cfg<P>::NT)
 k_diffv_elem(MeshDev m, const float *__restrict__ u, const float *__restrict__ mu_fluid,
              const float *__restrict__ musgs_t, const float *__restrict__ tauP, const float *__restrict__ tau_e,
-             float *__restrict__ slots) {
+             float *__restrict__ slots, const int *__restrict__ stop) {
   constexpr int N1 = Cfg<P>::N1, N = Cfg<P>::N, NT = Cfg<P>::NT;
   __shared__ __align__(16) float sm[EPB][9][N];
   const int el = threadIdx.x / NT, t = threadIdx.x % NT;
   const long long e = (long long)blockIdx.x * EPB + el;
   const bool active = (e < m.nelem) && (t < N);
   float gradU[3][3], gv = 0.f, He[9];
-  int node = 0;
-  stage_grad_u<P, EPB>(m, u, reinterpret_cast<float(*)[N]>(sm[el]), e, t, active, gradU, gv, He, node);
+  int node = 0, pos = 0;
+  if (!stage_grad_u<P, EPB>(m, u, reinterpret_cast<float(*)[N]>(sm[el]), e, t, active, gradU, gv, He, node, pos, stop))
+    return;
   float C[3][3];
   if (active) {
     const float ts = tau_e[e];
@@ -196,7 +207,121 @@ k_diffv_elem(MeshDev m, const float *__restrict__ u, const float *__restrict__ m
     }
     wd[r] = acc;
   }
-  reinterpret_cast<float4 *>(slots)[e * N + t] = make_float4(wd[0], wd[1], wd[2], 0.f);
+  reinterpret_cast<float4 *>(slots)[pos] = make_float4(wd[0], wd[1], wd[2], 0.f);
+}
+
+// ---- the solve on the device (single rank) ---------------------------------
+// The vector passes of conjGrad_veloc_incomp with their sums, as those of the
+// IMEX solve: the assembly forms qn = v Ml + fact dt D(v) and either the
+// start (r = b - qn, p = z = r / M, M = Ml / dt) or p.qn and alpha.
+constexpr int VELO_THREADS = 256;
+template <bool START>
+__global__ void __launch_bounds__(VELO_THREADS)
+k_veloc_gather_op(MeshDev m, const int *__restrict__ work, const float *__restrict__ slots,
+                  const float *__restrict__ Ml, float fact, float dt, double tol, const float *__restrict__ v,
+                  const float *__restrict__ b0, float *__restrict__ qn, float *__restrict__ r, float *__restrict__ p,
+                  CgScal *S, double *__restrict__ part, unsigned *ticket) {
+  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x, N = m.npoin;
+  int b = 0, en = 0;
+  float ml = 0.f;
+  const bool w = n < N && work[n] != 0;
+  if (w) { b = m.slot_ptr[n]; en = m.slot_ptr[n + 1]; ml = Ml[n]; }
+  pdl_wait();
+  pdl_trigger();
+  if (!START && S->status) return;
+  double a[2] = {0.0, 0.0};
+  if (w) {
+    float sum[3];
+    node_sum3(reinterpret_cast<const float4 *>(slots), b, en, sum);
+    const float M = ml / dt;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const long long k = n + N * d;
+      const float vk = v[k], qk = vk * ml + sum[d] * fact * dt;
+      if (START) {
+        const float rk = b0[k] - qk, zk = rk / M;
+        r[k] = rk;
+        p[k] = zk;
+        a[0] += (double)(rk * rk);
+        a[1] += (double)(rk * zk);
+      } else {
+        qn[k] = qk;
+        a[0] += (double)(vk * qk);
+      }
+    }
+  }
+  double tot[2];
+  if (grid_sum<2>(a, part, ticket, tot) && threadIdx.x == 0) {
+    if (START) {
+      S->rz = tot[1];
+      S->rr = tot[0];
+      S->bnorm = sqrt(tot[0]);
+      S->thr2 = tol * S->bnorm;
+      S->iter = S->status = 0;
+    } else {
+      S->alpha = (double)(float)(S->rz / tot[0]);
+    }
+  }
+}
+
+// x += alpha p ; r -= alpha q ; ||r||^2, r.z and r.(z - z_old): beta and status
+static __global__ void __launch_bounds__(VELO_THREADS)
+k_veloc_update(long long N, const int *__restrict__ work, const float *__restrict__ Ml, float dt,
+               const float *__restrict__ p, const float *__restrict__ q, float *__restrict__ x, float *__restrict__ r,
+               CgScal *S, double *__restrict__ part, unsigned *ticket) {
+  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool w = n < N && work[n] != 0;
+  const float M = w ? Ml[n] / dt : 1.f;
+  pdl_wait();
+  pdl_trigger();
+  if (S->status) return;
+  const float al = (float)S->alpha;
+  double a[3] = {0.0, 0.0, 0.0};
+  if (w) {
+    float pv[3], qv[3], xv[3], rv[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const long long k = n + N * d;
+      pv[d] = p[k]; qv[d] = q[k]; xv[d] = x[k]; rv[d] = r[k];
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const long long k = n + N * d;
+      x[k] = xv[d] + al * pv[d];
+      const float rn = rv[d] - al * qv[d], zn = rn / M, zo = rv[d] / M;
+      r[k] = rn;
+      a[0] += (double)(rn * rn);
+      a[1] += (double)(rn * zn);
+      a[2] += (double)(rn * (zn - zo));
+    }
+  }
+  double tot[3];
+  if (grid_sum<3>(a, part, ticket, tot) && threadIdx.x == 0) {
+    S->iter += 1;
+    S->rr = tot[0];
+    const double nrm = sqrt(tot[0]);
+    S->status = !isfinite(nrm) ? 3 : (nrm < S->thr2 ? 1 : 0);
+    S->beta = (double)(float)(tot[2] / S->rz);
+    S->rz = tot[1];
+  }
+}
+
+// p = z + beta p
+static __global__ void __launch_bounds__(VELO_THREADS)
+k_veloc_dir(long long N, const int *__restrict__ work, const float *__restrict__ Ml, float dt,
+            const float *__restrict__ r, float *__restrict__ p, const CgScal *S) {
+  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool w = n < N && work[n] != 0;
+  const float M = w ? Ml[n] / dt : 1.f;
+  pdl_wait();
+  pdl_trigger();
+  if (!w || S->status) return;
+  const float be = (float)S->beta;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const long long k = n + N * d;
+    p[k] = r[k] / M + be * p[k];
+  }
 }
 
 // qn = v Ml + qn fact dt over working nodes, 3 components (npoin,3)

@@ -162,3 +162,26 @@ def test_rhs_under_capture(gpu, porder, n):
     call()
     assert all(torch.equal(a, b) for a, b in zip(out, replayed))
     ctx.close()
+
+
+# the velocity solve reads its scalars every fourth iteration
+@pytest.mark.parametrize("porder,maxit", [(3, 1), (3, 4), (4, 5)])
+def test_velocity_cg_batches(gpu, porder, maxit):
+    m = host.periodic_cube(porder, 3, 4, 5, jitter=0.05, seed=8, ordering=1, elem_shuffle=True)
+    N, w = m.npoin, m.lpoin_w - 1
+    rng = np.random.default_rng(9)
+    u = rng.normal(size=3 * N).astype(np.float32)
+    mu = np.full(N, 1e-2, np.float32)
+    sgs = rng.uniform(0.0, 1e-2, m.nelem * m.nnode).astype(np.float32)
+    b = (u.reshape(3, N) * m.Ml + 0.1 * rng.normal(size=(3, N)) * m.Ml).reshape(-1).astype(np.float32)
+    dt = 0.05
+    xr, itr, rr = O.cg_veloc(O.OracleMesh(m), 1.0, dt, mu, sgs, u, b, maxIter=maxit, tol=1e-12)
+    ctx = gpu.Context(m, gpu.default_phys())
+    R, its, res = dv(b.copy()), C.c_int(), C.c_double()
+    dmu, dsgs, du = dv(mu), dv(sgs), dv(u)
+    ctx.call("sod_gpu_conjgrad_veloc", 1.0, dt, gpu.dptr(dmu), gpu.dptr(dsgs), gpu.dptr(du), gpu.dptr(R), maxit, 1e-12,
+             C.byref(its), C.byref(res))
+    assert its.value == itr == maxit
+    assert abs(res.value - rr) <= 0.05 * rr
+    assert rel_l2(R.cpu().numpy().reshape(3, N)[:, w], xr.reshape(3, N)[:, w]) < 1e-5
+    ctx.close()
