@@ -60,14 +60,6 @@ __global__ void k_add_all(long long n, const V *__restrict__ a, const V *__restr
   if (i < n) out[i] = a[i] + b[i];
 }
 
-template <int P, class V>
-inline DMat<P, V> dmat(const sod_gpu_ctx *c) {
-  DMat<P, V> D;
-  for (int a = 0; a <= P; ++a)
-    for (int b = 0; b <= P; ++b) D.d[a][b] = (V)c->D_h[a * (P + 1) + b];
-  return D;
-}
-
 template <class V>
 inline void lap(sod_gpu_ctx *c, const V *p, V *out) {
   dispatch(c, [&](auto L) {

@@ -367,24 +367,30 @@ inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 // ended).  Pass B never does (64^3: 1515 / 1484), the residual gather always.
 inline bool pdl_chain(const sod_gpu_ctx *c) { return (long long)c->nelem * c->N <= 5000000; }
 
+// The derivative matrix by value, in V.
+template <int P, class V>
+inline DMat<P, V> dmat(const sod_gpu_ctx *c) {
+  DMat<P, V> D;
+  for (int a = 0; a <= P; ++a)
+    for (int b = 0; b <= P; ++b) D.d[a][b] = (V)c->D_h[a * (P + 1) + b];
+  return D;
+}
+
 // ---- launch helpers templated on the element order --------------------
 
 template <int P>
 struct Launch {
   static constexpr int P_ = P;
-  // One element per block (64 threads for P=3, 128 for P=4) for every
-  // element kernel but pass A, whose latency-bound gathers do better with
-  // two elements per block for P=3 (0.405 against 0.447 ms at 64^3), while
-  // pass B and the Laplacian do better with one (0.94 against 1.05 ms).
+  // One element per block (64 threads for P=3, 128 for P=4) for the element
+  // kernels with a point per thread (0.94 against 1.05 ms with two for pass B
+  // at 64^3).
   static constexpr int EPB = 1;
   static constexpr int TPB = EPB * Cfg<P>::NT;
-  static constexpr int EPB_A = (Cfg<P>::NT <= 64) ? 2 : 1;
-  static constexpr int TPB_A = EPB_A * Cfg<P>::NT;
   static unsigned grid(int nelem) { return nblk(nelem, EPB); }
 
   static void proj(sod_gpu_ctx *c, bool prim, const float *a0, const float *a1, const float *a2) {
-    launch_pdl_if(pdl_chain(c), prim ? k_proj<P, EPB_A, true> : k_proj<P, EPB_A, false>, nblk(c->nelem, EPB_A), TPB_A, 0, c->stream,
-               c->md(), c->ph, c->phys.Rgas, a0, a1, a2, c->slotsA);
+    launch_pdl_if(pdl_chain(c), prim ? k_proj<P, true> : k_proj<P, false>, nblk(c->nelem, ColCfg<P>::EPB),
+                  32 * COL_WARPS, 0, c->stream, c->md(), dmat<P, float>(c), c->ph, c->phys.Rgas, a0, a1, a2, c->slotsA);
   }
   // Persistent pass B: as many blocks as fit on the GPU at once (at most
   // one per element group), each walking the groups with a stride.

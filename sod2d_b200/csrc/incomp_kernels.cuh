@@ -21,13 +21,6 @@ __device__ __forceinline__ void load_rot(const MeshDev &m, int c, bool col, floa
   load_drot<P>(m.Drot + (col ? 8 * (P + 1) : 0), c, D);
 }
 
-// The derivative matrix as a kernel argument: entries at fixed indices are
-// operands from the constant bank.
-template <int P, class V>
-struct DMat {
-  V d[P + 1][P + 1];
-};
-
 // ---- Laplacian: ResP = sum_e int grad N . grad p  (mod_operators.f90:16-112)
 // V = float (reference arithmetic) or double.  Writes one V per element node
 // into node-sorted slots (slot_pos), which the assembly sums contiguously.
@@ -45,11 +38,10 @@ struct DMat {
 // loads per point -- and bound the kernel; this form has 12 and 4.  All of a
 // thread's mesh loads (J^-1, weights, nodes, slot positions: 48 at P = 3)
 // are in flight before the programmatic wait.
-constexpr int LAP_WARPS = 2;
+constexpr int LAP_WARPS = COL_WARPS;
 template <int P>
-struct LapCfg {
-  static constexpr int LPE = P == 3 ? 16 : 32, EPW = 32 / LPE, EPB = LAP_WARPS * EPW;  // lanes and elements
-  static constexpr int MINB = P == 3 ? 8 : 6;                                          // blocks per SM
+struct LapCfg : ColCfg<P> {
+  static constexpr int MINB = P == 3 ? 8 : 6;  // blocks per SM
 };
 template <int P, class V, bool DIR = false>
 __global__ void __launch_bounds__(32 * LAP_WARPS, LapCfg<P>::MINB)

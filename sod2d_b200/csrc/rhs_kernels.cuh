@@ -212,6 +212,61 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
   return false;
 }
 
+// The derivative matrix as a kernel argument: entries at fixed indices are
+// operands from the constant bank.
+template <int P, class V>
+struct DMat {
+  V d[P + 1][P + 1];
+};
+
+// Line-per-thread kernels: a thread owns the P + 1 points along zeta over its
+// (i, j); 16 lanes (P = 3) or 25 of 32 (P = 4) take an element.
+constexpr int COL_WARPS = 2;
+template <int P>
+struct ColCfg {
+  static constexpr int LPE = P == 3 ? 16 : 32, EPW = 32 / LPE, EPB = COL_WARPS * EPW;  // lanes and elements
+};
+// The q-th node of a line is this many cyclic steps from the own node, own last.
+template <int P>
+__device__ __forceinline__ int col_step(int q) {
+  return q == P ? 0 : (q == P - 1 ? 1 : q + 2);
+}
+// Matrix rows i and j for col_grad2: rotated at P = 3, natural at P = 4.
+template <int P>
+__device__ __forceinline__ void col_rows(const MeshDev &m, int i, int j, float (&Di)[P + 1], float (&Dj)[P + 1]) {
+  if (P == 3) {
+    load_drot<P>(m.Drot, i, Di);
+    load_drot<P>(m.Drot, j, Dj);
+  } else {
+#pragma unroll
+    for (int q = 0; q <= P; ++q) { Di[q] = m.Dnat[i * (P + 1) + q]; Dj[q] = m.Dnat[j * (P + 1) + q]; }
+  }
+}
+// xi and eta derivatives at point (i, j, k) of a field staged in tensor
+// order, its own value given; summed in the order in which pass B sums the
+// gradients that the projections are compared with (their roundings cancel:
+// rotated at P = 4, the mass residual's error grew by 5 %).
+template <int P>
+__device__ __forceinline__ void col_grad2(const float *__restrict__ f, int i, int j, int k, float own,
+                                          const float (&Di)[P + 1], const float (&Dj)[P + 1], float &g0, float &g1) {
+  constexpr int N1 = P + 1;
+  const int r = N1 * N1 * k, c = i + N1 * j + r;
+  g0 = g1 = 0.f;
+#pragma unroll
+  for (int q = 0; q < N1; ++q) {
+    if (P == 3) {
+      const int s = col_step<P>(q);
+      const int ci = c + (i + s < N1 ? s : s - N1), cj = c + (j + s < N1 ? s : s - N1) * N1;
+      g0 = fmaf(Di[s], q == P ? own : f[ci], g0);
+      g1 = fmaf(Dj[s], q == P ? own : f[cj], g1);
+    } else {
+      const int mm = ref_order<P>(q);
+      g0 = fmaf(Di[mm], f[mm + N1 * j + r], g0);
+      g1 = fmaf(Dj[mm], f[i + N1 * mm + r], g1);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------
 // Pass A: LPS projections (full_proj_ijk, elem_stab.f90:474-562).  Writes
 // gpvol * {tau00, tau01, tau02, tau11, tau12, tau22, grad rho (3), grad T
@@ -222,87 +277,105 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
 // Input: conserved state (SoA, reference layout) -> EOS in registers, or
 // primitive rho/u/T (prim = true).
 // ---------------------------------------------------------------------
-// P = 3: 16 blocks per SM (32 registers, full occupancy) hide more of the
-// latency of the state gather: 1.636 against 1.643 ms per RHS at 64^3 with
-// 44 registers (11 blocks); 40 registers (12 blocks) gave 1.643.
-template <int P, int EPB, bool PRIM>
-__global__ void __launch_bounds__(EPB *Cfg<P>::NT, P == 3 ? 16 : 1)
-k_proj(MeshDev m, Phys ph, float Rgas, const float *__restrict__ a0, const float *__restrict__ a1,
+// A thread owns a line along zeta (ColCfg): the shared and L1 pipe, not HBM,
+// bound the one-point-per-thread form (75 % busy at 32^3: 60 staged words and
+// 12 matrix words read per point; here 30 and 2).  RHS at 64^3 1.47 -> 1.43 ms.
+// 8 to 10 blocks per SM are alike at order 3, 12 spill (1.53 ms).
+template <int P, bool PRIM>
+__global__ void __launch_bounds__(32 * COL_WARPS, P == 3 ? 10 : 8)
+k_proj(MeshDev m, DMat<P, float> D, Phys ph, float Rgas, const float *__restrict__ a0, const float *__restrict__ a1,
        const float *__restrict__ a2, float *__restrict__ slots) {
-  constexpr int N1 = Cfg<P>::N1, N = Cfg<P>::N, NT = Cfg<P>::NT, NF = 5;
-  __shared__ __align__(16) float sm[EPB][NF][N];
-  const int el = threadIdx.x / NT, t = threadIdx.x % NT;
-  const long long e = (long long)blockIdx.x * EPB + el;
-  const bool active = (e < m.nelem) && (t < N);
+  using L = ColCfg<P>;
+  constexpr int N1 = P + 1, N2 = N1 * N1, N = N1 * N2, NF = 5;
+  __shared__ __align__(16) float sm[L::EPB][NF][N];
+  __shared__ __align__(16) float ost[L::EPB * N * 12];
+  const int el = threadIdx.x / L::LPE, c = threadIdx.x % L::LPE;
+  const long long e = (long long)blockIdx.x * L::EPB + el;
+  const bool active = e < m.nelem && c < N2;
+  const int i = c % N1, j = c / N1;
   const long long NP = m.npoin;
-  float He[9], gv = 0.f;
-  int node = 0;
+  int n[N1];
+  float G[N1][10], Di[N1], Dj[N1];
   if (active) {  // mesh loads first: they depend on no earlier kernel
-    node = m.conn[e * N + t];
-    const float *g = m.geo + e * 10 * N + t;
+    const long long b = e * N + c;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) He[c] = g[c * N];
-    gv = g[9 * N];
+    for (int k = 0; k < N1; ++k) n[k] = m.conn[b + N2 * k];
+    const float *g = m.geo + e * 10 * N + c;
+#pragma unroll
+    for (int k = 0; k < N1; ++k)
+#pragma unroll
+      for (int q = 0; q < 10; ++q) G[k][q] = g[q * N + N2 * k];
+    col_rows<P>(m, i, j, Di, Dj);
   }
   pdl_wait();
   pdl_trigger();
+  float f[NF][N1];  // rho, T, u
   if (active) {
-    float rho, u0, u1, u2, T;
-    if (PRIM) {  // a0 = rho, a1 = u(N,3), a2 = Tem
-      rho = a0[node]; u0 = a1[node]; u1 = a1[node + NP]; u2 = a1[node + 2 * NP]; T = a2[node];
-    } else {     // a0 = rho, a1 = q(N,3), a2 = E
-      NodeQ s;
-      eos_fast(ph, __frcp_rn(Rgas), 1.f, a0[node], a1[node], a1[node + NP], a1[node + 2 * NP], a2[node], s);
-      rho = s.rho; u0 = s.u0; u1 = s.u1; u2 = s.u2; T = s.T;
+    float in[5][N1];
+#pragma unroll
+    for (int k = 0; k < N1; ++k) {  // PRIM: a0 = rho, a1 = u(N,3), a2 = Tem; else rho, q(N,3), E
+      in[0][k] = a0[n[k]];
+      in[1][k] = a1[n[k]];
+      in[2][k] = a1[n[k] + NP];
+      in[3][k] = a1[n[k] + 2 * NP];
+      in[4][k] = a2[n[k]];
     }
-    sm[el][0][t] = rho; sm[el][1][t] = T;
-    sm[el][2][t] = u0; sm[el][3][t] = u1; sm[el][4][t] = u2;
+    const float invR = __frcp_rn(Rgas);
+#pragma unroll
+    for (int k = 0; k < N1; ++k) {
+      if (PRIM) {
+        f[0][k] = in[0][k]; f[1][k] = in[4][k]; f[2][k] = in[1][k]; f[3][k] = in[2][k]; f[4][k] = in[3][k];
+      } else {
+        NodeQ s;
+        eos_fast(ph, invR, 1.f, in[0][k], in[1][k], in[2][k], in[3][k], in[4][k], s);
+        f[0][k] = s.rho; f[1][k] = s.T; f[2][k] = s.u0; f[3][k] = s.u1; f[4][k] = s.u2;
+      }
+#pragma unroll
+      for (int q = 0; q < NF; ++q) sm[el][q][c + N2 * k] = f[q][k];
+    }
   }
-  __syncthreads();
-  // the element's 12-wide slots are staged in shared memory and written
-  // out with coalesced 16-byte stores
-  __shared__ __align__(16) float ost[EPB * N * 12];
+  __syncwarp();
   if (active) {
-  const int i = t % N1, j = (t / N1) % N1, k = t / (N1 * N1);
-  float Di[N1], Dj[N1], Dk[N1];
 #pragma unroll
-  for (int s = 0; s < N1; ++s) { Di[s] = m.Dnat[i * N1 + s]; Dj[s] = m.Dnat[j * N1 + s]; Dk[s] = m.Dnat[k * N1 + s]; }
-  float gR[3], gT[3], gU[3][3];
-  iso_grad<P>(sm[el][0], i, j, k, Di, Dj, Dk, gR[0], gR[1], gR[2]);
-  iso_grad<P>(sm[el][1], i, j, k, Di, Dj, Dk, gT[0], gT[1], gT[2]);
+    for (int k = 0; k < N1; ++k) {
+      const float *He = G[k];
+      const float gv = G[k][9];
+      float gr[NF][3];  // physical gradients
 #pragma unroll
-  for (int c = 0; c < 3; ++c) iso_grad<P>(sm[el][2 + c], i, j, k, Di, Dj, Dk, gU[c][0], gU[c][1], gU[c][2]);
-  float gradRho[3], gradT[3], gradU[3][3];
+      for (int q = 0; q < NF; ++q) {
+        float g0, g1, g2 = 0.f;
+        col_grad2<P>(sm[el][q], i, j, k, f[q][k], Di, Dj, g0, g1);
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    gradRho[a] = He[a] * gR[0] + He[a + 3] * gR[1] + He[a + 6] * gR[2];
-    gradT[a] = He[a] * gT[0] + He[a + 3] * gT[1] + He[a + 6] * gT[2];
-  }
+        for (int s = 0; s < N1; ++s) {
+          const int mm = ref_order<P>(s);
+          g2 = fmaf(D.d[k][mm], f[q][mm], g2);
+        }
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+        for (int a = 0; a < 3; ++a) gr[q][a] = He[a] * g0 + He[a + 3] * g1 + He[a + 6] * g2;
+      }
+      const float divU = gr[2][0] + gr[3][1] + gr[4][2];
+      float tau[3][3];
 #pragma unroll
-    for (int b = 0; b < 3; ++b) gradU[a][b] = He[b] * gU[a][0] + He[b + 3] * gU[a][1] + He[b + 6] * gU[a][2];
-  const float divU = gradU[0][0] + gradU[1][1] + gradU[2][2];
-  float4 *o = reinterpret_cast<float4 *>(ost + (el * N + t) * 12);
-  float tau[3][3];
+      for (int a = 0; a < 3; ++a) {
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-#pragma unroll
-    for (int b = 0; b < 3; ++b) tau[a][b] = gradU[a][b] + gradU[b][a];
-    tau[a][a] = tau[a][a] - ph.twoThirds * divU;
-  }
-  o[0] = make_float4(gv * tau[0][0], gv * tau[0][1], gv * tau[0][2], gv * tau[1][1]);
-  o[1] = make_float4(gv * tau[1][2], gv * tau[2][2], gv * gradRho[0], gv * gradRho[1]);
-  o[2] = make_float4(gv * gradRho[2], gv * gradT[0], gv * gradT[1], gv * gradT[2]);
+        for (int b = 0; b < 3; ++b) tau[a][b] = gr[2 + a][b] + gr[2 + b][a];
+        tau[a][a] = tau[a][a] - ph.twoThirds * divU;
+      }
+      float4 *o = reinterpret_cast<float4 *>(ost + (el * N + c + N2 * k) * 12);
+      o[0] = make_float4(gv * tau[0][0], gv * tau[0][1], gv * tau[0][2], gv * tau[1][1]);
+      o[1] = make_float4(gv * tau[1][2], gv * tau[2][2], gv * gr[0][0], gv * gr[0][1]);
+      o[2] = make_float4(gv * gr[0][2], gv * gr[1][0], gv * gr[1][1], gv * gr[1][2]);
+    }
   }
   bulk_s2g_fence();
-  __syncthreads();
-  // one bulk copy (48 N bytes per element, a multiple of 16) by one thread
-  const long long e0 = (long long)blockIdx.x * EPB;
-  const long long ne = (m.nelem - e0) < EPB ? (m.nelem - e0) : EPB;
-  if (threadIdx.x == 0) {
-    bulk_s2g(slots + e0 * N * 12, ost, (unsigned)(ne * N * 48));
-    bulk_s2g_wait_read();
+  __syncwarp();
+  // the warp's elements leave by one bulk copy (48 N bytes each, a multiple of 16)
+  if (threadIdx.x % 32 == 0) {
+    const long long left = m.nelem - e;
+    if (left > 0) {
+      bulk_s2g(slots + e * N * 12, ost + el * N * 12, (unsigned)((left < L::EPW ? left : L::EPW) * N * 48));
+      bulk_s2g_wait_read();
+    }
   }
 }
 
