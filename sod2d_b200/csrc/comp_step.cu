@@ -78,14 +78,14 @@ int comp_updateF(sod_gpu_ctx *c) {
   return halo_sum(c, halo_res_view(c, S.Rmass, S.Rmom, S.Rener));
 }
 
-// Entropy residual (+ divergence and vorticity when dc) of (feta, eta1, u1[, u2]).
+// Entropy residual (+ divergence and vorticity when dc) of (u1 eta1, eta1, u1[, u2]).
 int comp_entropy_pass(sod_gpu_ctx *c, float *Reta_out, bool dc) {
   auto &S = c->comp;
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
     constexpr int P = LL::P_;
-    launch_pdl(dc ? k_entropy_elem<P, LL::EPB, true> : k_entropy_elem<P, LL::EPB, false>, LL::grid(c->nelem), LL::TPB, 0,
-               c->stream, c->md(), S.feta, S.eta1, S.u1, S.u2, c->slotsB, 1.0f);
+    launch_pdl(dc ? k_entropy_elem<P, true> : k_entropy_elem<P, false>, nblk(c->nelem, ColCfg<P>::EPB),
+               32 * COL_WARPS, 0, c->stream, c->md(), dmat<P, float>(c), nullptr, S.eta1, S.u1, S.u2, c->slotsB, 1.0f);
     return 0;
   });
   launch_pdl(dc ? k_gather_entropy<true> : k_gather_entropy<false>, nblk(c->npoin, 256), 256, 0, c->stream, c->md(),
@@ -130,8 +130,9 @@ int sod_gpu_generic_scalar_convec_ijk(sod_gpu_ctx *c, const float *q, const floa
   if (!c || !q || !eta || !u || !R) return fail(SOD_GPU_EINVAL, "bad argument");
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_entropy_elem<LL::P_, LL::EPB, false><<<LL::grid(c->nelem), LL::TPB, 0, c->stream>>>(c->md(), q, eta, u,
-                                                                                        nullptr, c->slotsB, fact);
+    constexpr int P = LL::P_;
+    k_entropy_elem<P, false><<<nblk(c->nelem, ColCfg<P>::EPB), 32 * COL_WARPS, 0, c->stream>>>(
+        c->md(), dmat<P, float>(c), q, eta, u, nullptr, c->slotsB, fact);
     return 0;
   });
   k_gather_sorted1<float><<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->md(), c->slotsB, R, initialze ? 0 : 1);
@@ -206,7 +207,7 @@ int sod_gpu_comp_init_state(sod_gpu_ctx *c, const sod_rk_cfg_t *cfg, const float
                     &S.Reta1, &S.Reta2, &S.aux, &S.divU, &S.mu_fluid, &S.Rmass, &S.Rener};
     for (auto pp : f1)
       if ((rc = c->alloc(pp, N))) return rc;
-    float **f3[] = {&S.q32, &S.u1, &S.u2, &S.feta, &S.vort, &S.Rmom};
+    float **f3[] = {&S.q32, &S.u1, &S.u2, &S.vort, &S.Rmom};
     for (auto pp : f3)
       if ((rc = c->alloc(pp, 3 * N))) return rc;
     if ((rc = c->alloc(&S.tau, NE)) || (rc = c->alloc(&S.part, 3 * NE)) || (rc = c->alloc(&S.bits, 4)) ||
@@ -271,7 +272,6 @@ int sod_gpu_comp_rk_ls_step(sod_gpu_ctx *c, float dt) {
   if (S.first) CUDA_TRY(cudaMemcpyAsync(S.eta1, S.eta2, N * 4, cudaMemcpyDeviceToDevice, st));
   if (S.first) {
     S.first = false;
-    k_feta<<<nblk(c->npoin_w, 256), 256, 0, st>>>(c->npoin_w, c->npoin, c->lpoin_w, S.u1, S.eta1, S.feta);
     int rc;
     if ((rc = comp_entropy_pass(c, S.Reta1, false)) || (rc = comp_visc(c, S.Reta1, S.rho32, S.u1, false)) ||
         (rc = comp_updateF(c)))
@@ -295,8 +295,8 @@ int sod_gpu_comp_rk_ls_step(sod_gpu_ctx *c, float dt) {
   launch_pdl(k_eos_end, nblk(c->npoin_w, 256), 256, 0, st, c->npoin_w, c->npoin, c->lpoin_w, gm - 1.0f, gm,
              c->phys.Rgas, S.rho32, S.q32, S.E32, S.u2, S.eint, S.pr, S.csound, S.machno, S.Tem, S.mu_factor,
              S.mu_fluid);
-  launch_pdl(k_thermo_entropy, nblk(c->npoin_w, 256), 256, 0, st, c->npoin_w, c->npoin, c->lpoin_w, gm, c->phys.p_inf,
-             c->phys.rho_inf, S.rho32, S.pr, S.u1, S.eta1, S.eta2, S.feta);
+  launch_pdl(k_thermo_entropy, nblk(c->npoin_w, 256), 256, 0, st, c->npoin_w, c->lpoin_w, gm, c->phys.p_inf, c->phys.rho_inf,
+             S.rho32, S.pr, S.eta1, S.eta2);
   int rc = comp_entropy_pass(c, S.Reta2, true);
   if (rc) return rc;
   k_aux_reta<<<nblk(c->npoin_w, 256), 256, 0, st>>>(c->npoin_w, c->lpoin_w, dt, S.Reta1, S.Reta2, S.eta1, S.eta2,
@@ -545,7 +545,6 @@ int sod_gpu_comp_imex_step(sod_gpu_ctx *c, float dt, int maxIter, double tol) {
   const long long B = 5 * N;
   if (S.first) {  // time_integ_imex.f90:240-273
     S.first = false;
-    k_feta<<<nb, 256, 0, st>>>(nw, N, c->lpoin_w, S.u1, S.eta1, S.feta);
     k_aux_h<<<nb, 256, 0, st>>>(nw, c->lpoin_w, gm / (gm - 1.0f), S.rho32, S.pr, X.aux_h);
     if ((rc = comp_entropy_pass(c, S.Reta1, false)) || (rc = comp_visc(c, S.Reta1, S.rho32, S.u1, false)) ||
         (rc = imex_convec(c, S.rho32, S.u2, S.q32, S.pr, X.aux_h, X.R)) ||
@@ -610,8 +609,8 @@ int sod_gpu_comp_imex_step(sod_gpu_ctx *c, float dt, int maxIter, double tol) {
   }
   X.cg_iters = iters;
   // entropy viscosity of the new state (time_integ_imex.f90:454-505)
-  k_thermo_entropy<<<nb, 256, 0, st>>>(nw, N, c->lpoin_w, gm, c->phys.p_inf, c->phys.rho_inf, S.rho32, S.pr, S.u1,
-                                       S.eta1, S.eta2, S.feta);
+  k_thermo_entropy<<<nb, 256, 0, st>>>(nw, c->lpoin_w, gm, c->phys.p_inf, c->phys.rho_inf, S.rho32, S.pr, S.eta1,
+                                       S.eta2);
   if ((rc = comp_entropy_pass(c, S.Reta2, true))) {
     c->async = was_async;
     return rc;
@@ -639,7 +638,7 @@ int sod_gpu_comp_adapt_dt(sod_gpu_ctx *c, float cfl_conv, float cfl_diff, float 
   CUDA_TRY(cudaMemsetAsync(S.bits + 1, 0x7f, 4, c->stream));
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
-    k_dt<LL::P_><<<dt_grid(c->nelem), 256, 0, c->stream>>>(c->md(), c->helem, S.u2, S.csound, S.mu_fluid,
+    k_dt<LL::P_><<<nblk(c->nelem, DtCfg<LL::P_>::EPB), 256, 0, c->stream>>>(c->md(), c->helem, S.u2, S.csound, S.mu_fluid,
                                                             c->mue_t, S.rho32, cfl_conv, cfl_diff, S.bits + 1);
     return 0;
   });

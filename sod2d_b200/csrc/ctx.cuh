@@ -129,7 +129,7 @@ struct sod_gpu_ctx {
     double lam[7][7], gam[7][7];
     float mu_factor = 1.f;
     void *U1[5], *U2[5];  // double or float
-    float *rho32, *q32, *E32, *u1, *u2, *eint, *pr, *csound, *machno, *Tem, *eta1, *eta2, *feta, *Reta1, *Reta2,
+    float *rho32, *q32, *E32, *u1, *u2, *eint, *pr, *csound, *machno, *Tem, *eta1, *eta2, *Reta1, *Reta2,
         *aux, *divU, *vort, *mu_fluid, *tau, *Rmass, *Rmom, *Rener, *part;
     unsigned int *bits;  // [0] min rho, [1] dt, [2] max Mach
     double *sums;        // [3]
@@ -418,9 +418,6 @@ inline int dispatch(sod_gpu_ctx *c, F &&f) {
   if (c->P == 4) return f(Launch<4>());
   return fail(SOD_GPU_EINVAL, "unsupported element order");
 }
-
-// grid of k_dt: eight elements per block and trip, at most 8 blocks per SM
-inline unsigned dt_grid(int nelem) { return std::min(nblk(nelem, 8), 8u * (unsigned)num_sms()); }
 
 inline void comp_tau(sod_gpu_ctx *c, const float *csound, const float *u, float *tau) {
   dispatch(c, [&](auto L) {

@@ -1026,7 +1026,7 @@ int sod_gpu_incomp_adapt_dt(sod_gpu_ctx *c, float cfl_conv, float *dt) {
   dispatch(c, [&](auto L) {
     using LL = decltype(L);
     // zero sound speed and viscosities: only the convective limit acts
-    k_dt<LL::P_><<<dt_grid(c->nelem), 256, 0, c->stream>>>(c->md(), c->helem, I.u[0], I.zero, I.zero, I.zeroE,
+    k_dt<LL::P_><<<nblk(c->nelem, DtCfg<LL::P_>::EPB), 256, 0, c->stream>>>(c->md(), c->helem, I.u[0], I.zero, I.zero, I.zeroE,
                                                             I.one, cfl_conv, 1.0f, I.bits);
     return 0;
   });

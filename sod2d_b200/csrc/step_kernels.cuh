@@ -84,12 +84,11 @@ static __global__ void k_eos_end(int npoin_w, long long npoin, const int *__rest
 }
 
 // ---- thermo_entropy, mod_entropy_viscosity.f90:411-433 ----------------
-// eta1 <- eta2; eta2 <- rho/(g-1) log(max(p/p_inf, eps)/(rho/rho_inf)^g);
-// feta = u1 * eta1.
-static __global__ void k_thermo_entropy(int npoin_w, long long npoin, const int *__restrict__ lpoin_w, float gamma,
+// eta1 <- eta2; eta2 <- rho/(g-1) log(max(p/p_inf, eps)/(rho/rho_inf)^g)
+// (the flux u1 eta1 is formed by k_entropy_elem).
+static __global__ void k_thermo_entropy(int npoin_w, const int *__restrict__ lpoin_w, float gamma,
                                  float p_inf, float rho_inf, const float *__restrict__ rho,
-                                 const float *__restrict__ pr, const float *__restrict__ u1,
-                                 float *__restrict__ eta1, float *__restrict__ eta2, float *__restrict__ feta) {
+                                 const float *__restrict__ pr, float *__restrict__ eta1, float *__restrict__ eta2) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npoin_w) return;
   const long long p = lpoin_w[t];
@@ -99,18 +98,6 @@ static __global__ void k_thermo_entropy(int npoin_w, long long npoin, const int 
   eta1[p] = e1;
   const float r = rho[p];
   eta2[p] = (r / (gamma - 1.0f)) * logf(fmaxf(pr[p] / p_inf, 1.1920929e-07f) / powf(r / rho_inf, gamma));
-#pragma unroll
-  for (int d = 0; d < 3; ++d) feta[p + npoin * d] = u1[p + npoin * d] * e1;
-}
-
-// feta = u1 * eta1 at working nodes (first step, time_integ_ls.f90:274-281).
-static __global__ void k_feta(int npoin_w, long long npoin, const int *__restrict__ lpoin_w, const float *__restrict__ u1,
-                       const float *__restrict__ eta1, float *__restrict__ feta) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= npoin_w) return;
-  const long long p = lpoin_w[t];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) feta[p + npoin * d] = u1[p + npoin * d] * eta1[p];
 }
 
 // ---- entropy flux residual + divergence + vorticity, one element pass --
@@ -119,85 +106,126 @@ static __global__ void k_feta(int npoin_w, long long npoin, const int *__restric
 // (elem_convec.f90:472-594), 1 = eval_divergence of u2
 // (mod_operators.f90:485-570), 2..4 = compute_vorticity of u2 before the
 // per-node averaging (mod_operators.f90:684-775).  WANT_DC = 0 skips 1..4.
-template <int P, int EPB, bool WANT_DC>
-__global__ void __launch_bounds__(EPB *Cfg<P>::NT)
-k_entropy_elem(MeshDev m, const float *__restrict__ feta, const float *__restrict__ eta1,
+// A thread owns a line along zeta (ColCfg), the fields taken one after the
+// other: with a point per thread the shared and L1 pipe was 84 % busy with
+// 120 staged words and 12 matrix words per point (here 70 and 2).
+// The gathers of node values are the rest of its load: feta = u1 eta1, which
+// thermo_entropy forms, is that product again here (feta null), not three
+// more gathers.
+template <int P, bool WANT_DC>
+__global__ void __launch_bounds__(32 * COL_WARPS, P == 3 ? 6 : 4)
+k_entropy_elem(MeshDev m, DMat<P, float> D, const float *__restrict__ feta, const float *__restrict__ eta1,
                const float *__restrict__ u1, const float *__restrict__ u2, float *__restrict__ slots,
-               float fact = 1.0f) {
-  constexpr int N1 = Cfg<P>::N1, N = Cfg<P>::N, NT = Cfg<P>::NT, NF = 10;
-  __shared__ __align__(16) float sm[EPB][NF][N];
-  const int el = threadIdx.x / NT, t = threadIdx.x % NT;
-  const long long e = (long long)blockIdx.x * EPB + el;
-  const bool active = (e < m.nelem) && (t < N);
+               float fact) {
+  using L = ColCfg<P>;
+  constexpr int N1 = P + 1, N2 = N1 * N1, N = N1 * N2, NF = WANT_DC ? 10 : 7;  // eta, u1, feta, u2
+  __shared__ float sm[L::EPB][NF][N];
+  const int el = threadIdx.x / L::LPE, c = threadIdx.x % L::LPE;
+  const long long e = (long long)blockIdx.x * L::EPB + el;
+  const bool active = e < m.nelem && c < N2;
+  const int i = c % N1, j = c / N1;
   const long long NP = m.npoin;
-  // mesh loads first (no other kernel writes them): J^-1 after the staging
-  // barrier doubled the latency chain
-  int node = 0, pos = 0;
-  float He[9], gv = 0.f;
-  if (active) {
-    node = m.conn[e * N + t];
-    pos = m.slot_pos[e * N + t];
-    const float *g = m.geo + e * 10 * N + t;
+  int n[N1], pos[N1];
+  float G[N1][10], Di[N1], Dj[N1];
+  if (active) {  // mesh loads first (no other kernel writes them)
+    const long long b = e * N + c;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) He[c] = g[c * N];
-    gv = g[9 * N];
+    for (int k = 0; k < N1; ++k) { n[k] = m.conn[b + N2 * k]; pos[k] = m.slot_pos[b + N2 * k]; }
+    const float *g = m.geo + e * 10 * N + c;
+#pragma unroll
+    for (int k = 0; k < N1; ++k)
+#pragma unroll
+      for (int q = 0; q < 10; ++q) G[k][q] = g[q * N + N2 * k];
+    col_rows<P>(m, i, j, Di, Dj);
   }
   pdl_wait();
   pdl_trigger();
   if (active) {
-    sm[el][0][t] = eta1[node];
+    float in[NF][N1];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      sm[el][1 + d][t] = u1[node + NP * d];
-      sm[el][4 + d][t] = feta[node + NP * d];
-      if (WANT_DC) sm[el][7 + d][t] = u2[node + NP * d];
+    for (int k = 0; k < N1; ++k) {
+      in[0][k] = eta1[n[k]];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        in[1 + d][k] = u1[n[k] + NP * d];
+        if (feta) in[4 + d][k] = feta[n[k] + NP * d];
+        if (WANT_DC) in[(WANT_DC ? 7 : 0) + d][k] = u2[n[k] + NP * d];
+      }
     }
+#pragma unroll
+    for (int k = 0; k < N1; ++k)
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (!feta) in[4 + d][k] = in[1 + d][k] * in[0][k];
+#pragma unroll
+    for (int q = 0; q < NF; ++q)
+#pragma unroll
+      for (int k = 0; k < N1; ++k) sm[el][q][c + N2 * k] = in[q][k];
   }
-  __syncthreads();
+  __syncwarp();
   if (!active) return;
-  const int i = t % N1, j = (t / N1) % N1, k = t / (N1 * N1);
-  float Di[N1], Dj[N1], Dk[N1];
+  // physical gradient of field q at this thread's points
+  auto grad = [&](int q, float (&g)[N1][3]) {
+    float col[N1];
 #pragma unroll
-  for (int s = 0; s < N1; ++s) { Di[s] = m.Dnat[i * N1 + s]; Dj[s] = m.Dnat[j * N1 + s]; Dk[s] = m.Dnat[k * N1 + s]; }
-  float a0, a1, a2;
-  iso_grad<P>(sm[el][0], i, j, k, Di, Dj, Dk, a0, a1, a2);
-  float gradE[3];
+    for (int k = 0; k < N1; ++k) col[k] = sm[el][q][c + N2 * k];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) gradE[a] = He[a] * a0 + He[a + 3] * a1 + He[a + 6] * a2;
-  float divU = 0.f, divFe = 0.f;
+    for (int k = 0; k < N1; ++k) {
+      float g0, g1, g2 = 0.f;
+      col_grad2<P>(sm[el][q], i, j, k, col[k], Di, Dj, g0, g1);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    iso_grad<P>(sm[el][1 + c], i, j, k, Di, Dj, Dk, a0, a1, a2);
-    divU += He[c] * a0 + He[c + 3] * a1 + He[c + 6] * a2;
-    iso_grad<P>(sm[el][4 + c], i, j, k, Di, Dj, Dk, a0, a1, a2);
-    divFe += He[c] * a0 + He[c + 3] * a1 + He[c + 6] * a2;
-  }
-  const float etal = sm[el][0][t];
-  float Re = 0.5f * (divFe + etal * divU);
+      for (int s = 0; s < N1; ++s) {
+        const int mm = ref_order<P>(s);
+        g2 = fmaf(D.d[k][mm], col[mm], g2);
+      }
+      const float *He = G[k];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) Re = Re + 0.5f * (sm[el][1 + a][t] * gradE[a]);
-  float out[5] = {fact * (gv * Re), 0.f, 0.f, 0.f, 0.f};
-  if (WANT_DC) {
-    float gu[3][3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      iso_grad<P>(sm[el][7 + c], i, j, k, Di, Dj, Dk, a0, a1, a2);
-#pragma unroll
-      for (int b = 0; b < 3; ++b) gu[c][b] = He[b] * a0 + He[b + 3] * a1 + He[b + 6] * a2;  // d u_c / d x_b
+      for (int a = 0; a < 3; ++a) g[k][a] = He[a] * g0 + He[a + 3] * g1 + He[a + 6] * g2;
     }
-    out[1] = gv * (gu[0][0] + gu[1][1] + gu[2][2]);
-    // curl with the reference's Levi-Civita table (CFDSolverBase.f90:1600-1606):
-    // curl_0 = g(1,2) - g(2,1), curl_1 = g(2,0) - g(0,2), curl_2 = g(0,1) - g(1,0)
-    // where g(j,k) = d u_j / d x_k.
-    out[2] = gu[1][2] - gu[2][1];
-    out[3] = -gu[0][2] + gu[2][0];
-    out[4] = gu[0][1] - gu[1][0];
+  };
+  float g[N1][3], Re[N1], divU[N1], divFe[N1];
+#pragma unroll
+  for (int k = 0; k < N1; ++k) divU[k] = divFe[k] = 0.f;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    grad(1 + d, g);
+#pragma unroll
+    for (int k = 0; k < N1; ++k) divU[k] += g[k][d];
+    grad(4 + d, g);
+#pragma unroll
+    for (int k = 0; k < N1; ++k) divFe[k] += g[k][d];
   }
-  if (WANT_DC) {
-    reinterpret_cast<float4 *>(slots)[pos] = make_float4(out[0], out[1], out[2], out[3]);
-    slots[(long long)m.nelem * N * 4 + pos] = out[4];
-  } else {
-    slots[pos] = out[0];
+  grad(0, g);
+#pragma unroll
+  for (int k = 0; k < N1; ++k) {
+    const int t = c + N2 * k;
+    Re[k] = 0.5f * (divFe[k] + sm[el][0][t] * divU[k]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) Re[k] = Re[k] + 0.5f * (sm[el][1 + a][t] * g[k][a]);
+    Re[k] = fact * (G[k][9] * Re[k]);
+  }
+  if (!WANT_DC) {
+#pragma unroll
+    for (int k = 0; k < N1; ++k) slots[pos[k]] = Re[k];
+    return;
+  }
+  // divergence and the curl with the reference's Levi-Civita table
+  // (CFDSolverBase.f90:1600-1606): curl_0 = g(1,2) - g(2,1), curl_1 =
+  // g(2,0) - g(0,2), curl_2 = g(0,1) - g(1,0), g(j,k) = d u_j / d x_k
+  float dv[N1], cu[N1][3];
+  grad(NF - 3, g);
+#pragma unroll
+  for (int k = 0; k < N1; ++k) { dv[k] = g[k][0]; cu[k][1] = -g[k][2]; cu[k][2] = g[k][1]; }
+  grad(NF - 2, g);
+#pragma unroll
+  for (int k = 0; k < N1; ++k) { dv[k] += g[k][1]; cu[k][0] = g[k][2]; cu[k][2] -= g[k][0]; }
+  grad(NF - 1, g);
+#pragma unroll
+  for (int k = 0; k < N1; ++k) { dv[k] += g[k][2]; cu[k][0] -= g[k][1]; cu[k][1] += g[k][0]; }
+#pragma unroll
+  for (int k = 0; k < N1; ++k) {
+    reinterpret_cast<float4 *>(slots)[pos[k]] = make_float4(Re[k], G[k][9] * dv[k], cu[k][0], cu[k][1]);
+    slots[(long long)m.nelem * N * 4 + pos[k]] = cu[k][2];
   }
 }
 
@@ -426,48 +454,65 @@ static __global__ void k_sutherland(int npoin_w, const int *__restrict__ lpoin_w
 }
 
 // ---- adapt_dt_cfl, mod_time_ops.f90:11-62: per element, then min -------
-// Warps stride over the elements and a block issues one atomic: one atomic
-// per element to the same word was half of this kernel's time (110,592
-// elements: 120 us).  out_bits starts as 0x7f7f7f7f; the caller applies the
-// reference's initial 1e14.
+// A warp takes two elements at P = 3 (one at P = 4), all loads of a lane's
+// four nodes in flight, and a block issues one atomic: one atomic per element
+// to the same word was half of this kernel's time (110,592 elements: 120 us).
+// out_bits starts as 0x7f7f7f7f; the caller applies the reference's initial 1e14.
+template <int P>
+struct DtCfg {
+  static constexpr int EPW = P == 3 ? 2 : 1, EPB = 8 * EPW;  // elements per warp, per block
+};
 template <int P>
 __global__ void __launch_bounds__(256)
 k_dt(MeshDev m, const float *__restrict__ helem, const float *__restrict__ u, const float *__restrict__ csound,
      const float *__restrict__ mu_fluid, const float *__restrict__ mue_t, const float *__restrict__ rho, float cfl_conv,
      float cfl_diff, unsigned int *__restrict__ out_bits) {
-  constexpr int N = Cfg<P>::N, IT = (N + 31) / 32;
+  constexpr int N = Cfg<P>::N, IT = (N + 31) / 32, EPW = DtCfg<P>::EPW;
   __shared__ unsigned sh[8];
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const long long NP = m.npoin;
-  unsigned best = 0x7f7f7f7fu;
-  for (long long e = (long long)blockIdx.x * 8 + warp; e < m.nelem; e += (long long)gridDim.x * 8) {
-    int p[IT];
-    float me[IT];
+  const long long NP = m.npoin, e0 = (long long)blockIdx.x * DtCfg<P>::EPB + warp * EPW;
+  int p[EPW][IT];
+  float me[EPW][IT], um[EPW][IT], cs[EPW][IT], mu[EPW][IT], rh[EPW][IT];
+#pragma unroll
+  for (int w = 0; w < EPW; ++w)
 #pragma unroll
     for (int q = 0; q < IT; ++q) {
       const int t = lane + 32 * q;
-      p[q] = t < N ? m.conn[e * N + t] : -1;
-      me[q] = t < N ? mue_t[e * N + t] : 0.f;
+      const bool in = e0 + w < m.nelem && t < N;
+      p[w][q] = in ? m.conn[(e0 + w) * N + t] : -1;
+      me[w][q] = in ? mue_t[(e0 + w) * N + t] : 0.f;
     }
+#pragma unroll
+  for (int w = 0; w < EPW; ++w)
+#pragma unroll
+    for (int q = 0; q < IT; ++q) {
+      if (p[w][q] < 0) continue;
+      const long long n = p[w][q];
+      um[w][q] = fmaxf(fmaxf(fabsf(u[n]), fabsf(u[n + NP])), fabsf(u[n + 2 * NP]));
+      cs[w][q] = csound[n];
+      mu[w][q] = mu_fluid[n];
+      rh[w][q] = rho[n];
+    }
+  unsigned best = 0x7f7f7f7fu;
+#pragma unroll
+  for (int w = 0; w < EPW; ++w) {
     float L3 = 0.f, maxMU = 0.f;
 #pragma unroll
     for (int q = 0; q < IT; ++q) {
-      if (p[q] < 0) continue;
-      const long long n = p[q];
-      float um = fabsf(u[n]);
-      um = fmaxf(um, fabsf(u[n + NP]));
-      um = fmaxf(um, fabsf(u[n + 2 * NP]));
-      L3 = fmaxf(L3, um + csound[n]);
-      maxMU = fmaxf(maxMU, (0.0f + mu_fluid[n] + me[q]) / rho[n]);
+      if (p[w][q] < 0) continue;
+      L3 = fmaxf(L3, um[w][q] + cs[w][q]);
+      maxMU = fmaxf(maxMU, (0.0f + mu[w][q] + me[w][q]) / rh[w][q]);
     }
     for (int o = 16; o > 0; o >>= 1) {
       L3 = fmaxf(L3, __shfl_xor_sync(0xffffffffu, L3, o));
       maxMU = fmaxf(maxMU, __shfl_xor_sync(0xffffffffu, maxMU, o));
     }
-    const float hp = helem[e] / (float)(2 * P + 1);
-    const float dconv = cfl_conv * hp / L3;
-    const float ddiff = cfl_diff * (hp * hp) / maxMU;
-    best = min(best, __float_as_uint(fminf(dconv, ddiff)));  // dt > 0: bit order = value order
+    if (e0 + w < m.nelem) {
+      const float hp = helem[e0 + w] / (float)(2 * P + 1);
+      const float dconv = cfl_conv * hp / L3;
+      const float ddiff = cfl_diff * (hp * hp) / maxMU;
+      best = min(best, __float_as_uint(fminf(dconv, ddiff)));  // dt > 0: bit order = value order
+    }
   }
   if (lane == 0) sh[warp] = best;
   __syncthreads();
