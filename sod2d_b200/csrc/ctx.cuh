@@ -428,9 +428,9 @@ inline void comp_tau(sod_gpu_ctx *c, const float *csound, const float *u, float 
 }
 
 inline void gather_proj_aos(sod_gpu_ctx *c) {
-  OutPtrs none{};
   // 128-thread blocks: 1.642-1.650 ms per RHS against 1.660 with 256 (64^3 bench)
-  launch_pdl_if(pdl_chain(c), k_gather<12, 12, true>, nblk(c->npoin, 128), 128, 0, c->stream, c->md(), c->slotsA, c->proj12, none, 0, 1);
+  launch_pdl_if(pdl_chain(c), k_gather_proj<false>, nblk(c->npoin, 128), 128, 0, c->stream, c->md(), c->slotsA, c->proj12,
+                OutPtrs{});
 }
 
 // Sum the view's components over the ranks that share each node (no-op

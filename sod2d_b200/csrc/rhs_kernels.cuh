@@ -960,78 +960,56 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
 }
 
 // ---------------------------------------------------------------------
-// Node-centric assembly: out_f(p) = scale(p) * (base_f(p) + sum of the
-// node's slot contributions), Kahan-compensated, slots visited in element
-// order (deterministic).  W = slot width, NFO = fields summed.
-// Output layout: SoA (reference, out[f][p] = out + f*npoin) when AOS is
-// false; node-major [p][W] when true.
+// Node-centric assembly of pass A: the 12 projections of a node are invMl
+// times the Kahan-compensated sum of its slots in element order
+// (deterministic).  Node-major [p][12] for pass B, or (REF) the reference's
+// five (npoin,3) arrays, whose symmetric stress rows share entries.
 // ---------------------------------------------------------------------
 struct OutPtrs {
-  float *p[16];
+  float *p[5];
 };
-
-template <int W, int NFO, bool AOS>
-__global__ void k_gather(MeshDev m, const float *__restrict__ slots, float *__restrict__ out,
-                         OutPtrs out_soa, int accumulate, int use_invMl) {
+template <bool REF>
+__global__ void k_gather_proj(MeshDev m, const float *__restrict__ slots, float *__restrict__ out, OutPtrs ref) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= m.npoin) return;
-  constexpr int MS = W >= 12 ? 1 : 4;  // slots whose loads are issued together (registers permitting)
   const int b = m.slot_ptr[p], en = m.slot_ptr[p + 1];
-  const float sc = use_invMl ? m.invMl[p] : 1.f;
+  const float sc = m.invMl[p];
   pdl_wait();
   pdl_trigger();
-  float sum[NFO], cmp[NFO];
+  float sum[12], cmp[12];
 #pragma unroll
-  for (int f = 0; f < NFO; ++f) {
-    sum[f] = (accumulate && !AOS) ? out_soa.p[f][p] : 0.f;
-    cmp[f] = 0.f;
-  }
-  for (int s0 = b; s0 < en; s0 += MS) {
-    int id[MS];
+  for (int f = 0; f < 12; ++f) sum[f] = cmp[f] = 0.f;
+  for (int s = b; s < en; ++s) {
+    const float4 *v = reinterpret_cast<const float4 *>(slots + (long long)m.slot_idx[s] * 12);
+    const float4 v0 = v[0], v1 = v[1], v2 = v[2];
+    const float x[12] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w};
 #pragma unroll
-    for (int k = 0; k < MS; ++k) id[k] = s0 + k < en ? m.slot_idx[s0 + k] : -1;
-    float4 v[MS][W / 4];
-#pragma unroll
-    for (int k = 0; k < MS; ++k)
-#pragma unroll
-      for (int c = 0; c < W / 4; ++c)
-        v[k][c] = id[k] >= 0 ? reinterpret_cast<const float4 *>(slots + (long long)id[k] * W)[c]
-                             : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < MS; ++k) {
-      if (id[k] < 0) break;
-      float x[W];
-#pragma unroll
-      for (int c = 0; c < W / 4; ++c) {
-        x[4 * c] = v[k][c].x; x[4 * c + 1] = v[k][c].y; x[4 * c + 2] = v[k][c].z; x[4 * c + 3] = v[k][c].w;
-      }
-#pragma unroll
-      for (int f = 0; f < NFO; ++f) {  // Kahan summation
-        const float y = x[f] - cmp[f];
-        const float tt = sum[f] + y;
-        cmp[f] = (tt - sum[f]) - y;
-        sum[f] = tt;
-      }
+    for (int f = 0; f < 12; ++f) {  // Kahan summation
+      const float y = x[f] - cmp[f];
+      const float tt = sum[f] + y;
+      cmp[f] = (tt - sum[f]) - y;
+      sum[f] = tt;
     }
   }
-  if (AOS) {
-    float4 *o = reinterpret_cast<float4 *>(out + p * W);
-    float r[W];
 #pragma unroll
-    for (int f = 0; f < W; ++f) r[f] = f < NFO ? sum[f] * sc : 0.f;
+  for (int f = 0; f < 12; ++f) sum[f] = sum[f] * sc;
+  if (REF) {  // ref: ProjMX, ProjMY, ProjMZ, ProjMass, ProjEner
+    constexpr int row[5][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}, {6, 7, 8}, {9, 10, 11}};
 #pragma unroll
-    for (int c = 0; c < W / 4; ++c) o[c] = make_float4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+    for (int a = 0; a < 5; ++a)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) ref.p[a][p + m.npoin * d] = sum[row[a][d]];
   } else {
+    float4 *o = reinterpret_cast<float4 *>(out + p * 12);
 #pragma unroll
-    for (int f = 0; f < NFO; ++f) out_soa.p[f][p] = sum[f] * sc;
+    for (int q = 0; q < 3; ++q) o[q] = make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]);
   }
 }
 
 // ---------------------------------------------------------------------
 // Assembly from node-sorted slots (written at slot_pos by k_rhs): node p's
 // contributions are slots slot_ptr[p] .. slot_ptr[p+1]-1, in element
-// order, so a warp streams one contiguous range with no index loads.  Same
-// Kahan-compensated order as k_gather (bit-identical sums).
+// order, so a warp streams one contiguous range with no index loads.
 // ---------------------------------------------------------------------
 // The 5 residuals from node-sorted pass-B slots into the reference's SoA
 // outputs (optionally accumulated onto them), x invMl.

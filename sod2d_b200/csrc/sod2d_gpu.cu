@@ -351,8 +351,14 @@ int sod_gpu_full_proj_ijk(sod_gpu_ctx *c, const float *rho, const float *u, cons
     return 0;
   });
   if (rc) return rc;
-  // assemble into the node-major 12-wide buffer, then expand to the
-  // reference's five (npoin,3) arrays
+  if (!c->halo.on) {
+    const OutPtrs ref{{ProjMX, ProjMY, ProjMZ, ProjMass, ProjEner}};
+    launch_pdl_if(pdl_chain(c), k_gather_proj<true>, nblk(c->npoin, 128), 128, 0, c->stream, c->md(), c->slotsA, nullptr,
+                  ref);
+    return c->finish();
+  }
+  // a partitioned mesh sums the node-major 12-wide buffer over the ranks,
+  // then expands it to the reference's five (npoin,3) arrays
   gather_proj_aos(c);
   if ((rc = halo_sum(c, halo_proj_view(c)))) return rc;
   k_unpack_proj<<<nblk(c->npoin, 256), 256, 0, c->stream>>>(c->npoin, c->proj12, ProjMX, ProjMY, ProjMZ, ProjMass,
