@@ -380,6 +380,22 @@ int imex_convec(sod_gpu_ctx *c, const float *rho, const float *u, const float *q
   return halo_block5(c, out);
 }
 
+// The same from the conserved state alone, whose velocity, pressure and
+// enthalpy k_eos_end and k_aux_h would form: the split form with one product
+// per line node (see RhsPlan::FLUX2) on 5 gathered arrays instead of 9.
+int imex_convec_state(sod_gpu_ctx *c, float *out) {
+  auto &S = c->comp;
+  RhsArgs A{};
+  A.rho = S.rho32; A.q = S.q32; A.E = S.E32; A.mu_factor = S.mu_factor; A.fact_c = 1.0f;
+  dispatch(c, [&](auto L) {
+    L.template rhs<MODE_CONV, IN_CONS>(c, A);
+    return 0;
+  });
+  const long long N = c->npoin;
+  gather_res(c, out, out + 2 * N, out + N, 0, 0);
+  return halo_block5(c, out);
+}
+
 // diffusion without LPS (fact +1) into a five-variable block; rho_n null: rho
 int imex_diffusion(sod_gpu_ctx *c, const float *rho_n, const float *rho, const float *u, const float *Tem,
                     float *out) {
@@ -600,8 +616,7 @@ int sod_gpu_comp_imex_step(sod_gpu_ctx *c, float dt, int maxIter, double tol) {
     iters += X.cg_iters;
     k_eos_end<<<nb, 256, 0, st>>>(nw, N, c->lpoin_w, gm - 1.0f, gm, c->phys.Rgas, S.rho32, S.q32, S.E32, S.u2, S.eint,
                                   S.pr, S.csound, S.machno, S.Tem, 0.f, nullptr);
-    k_aux_h<<<nb, 256, 0, st>>>(nw, c->lpoin_w, gm / (gm - 1.0f), S.rho32, S.pr, X.aux_h);
-    if ((rc = imex_convec(c, S.rho32, S.u2, S.q32, S.pr, X.aux_h, X.R + (is - 1) * B)) ||
+    if ((rc = imex_convec_state(c, X.R + (is - 1) * B)) ||
         (rc = imex_diffusion(c, nullptr, S.rho32, S.u2, S.Tem, X.D + (is - 1) * B))) {
       c->async = was_async;
       return rc;

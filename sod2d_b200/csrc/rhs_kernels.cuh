@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(EPB *Cfg<P>::NT, SOD_RHS_THREADS_PER_SM / (EPB
 k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
   using L = RhsPlan<P, EPB, MODE, IN>;
   constexpr int N1 = L::N1, N = L::N, NT = L::NT, NTB = L::NTB, NC = L::NC, SMF = L::SMF, PB_T = L::PB_T;
-  constexpr bool CONV = L::CONV, DIFF = L::DIFF, LPS = L::LPS, FLUX2 = L::FLUX2, ROT = P == 3 && DIFF;
+  constexpr bool CONV = L::CONV, DIFF = L::DIFF, LPS = L::LPS, FLUX2 = L::FLUX2, ROT = P == 3 && (DIFF || FLUX2);
   static_assert(FLUX2 || !(CONV && DIFF), "convection with diffusion runs on the conserved state");
   extern __shared__ __align__(16) float dsm[];
   const int tid = threadIdx.x, el = tid / NT, t = tid % NT;
