@@ -208,7 +208,8 @@ k_imex_gather_op(MeshDev m, const int *__restrict__ work, const float *__restric
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x, N = m.npoin;
   int b = 0, en = 0;
   float ml = 0.f;
-  if (n < N && work[n]) { b = m.slot_ptr[n]; en = m.slot_ptr[n + 1]; ml = Ml[n]; }
+  const bool w = n < N && work[n] != 0;
+  if (w) { b = m.slot_ptr[n]; en = m.slot_ptr[n + 1]; ml = Ml[n]; }
   pdl_wait();
   pdl_trigger();
   if (S->status) return;
@@ -227,7 +228,7 @@ k_imex_gather_op(MeshDev m, const int *__restrict__ work, const float *__restric
     }
   }
   double v[1] = {0.0};
-  if (b != en) {
+  if (w) {
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
       const long long o = n + N * f;
