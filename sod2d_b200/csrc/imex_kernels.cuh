@@ -137,7 +137,7 @@ constexpr int IMEX_THREADS = 256;
 // fact dt D(x0)), p = r / M with its velocity and temperature; ||r||^2 and
 // r.z start the scalars.  One instantiation per stage: with the stage loop
 // unrolled all its loads are in flight together (a runtime loop walked them
-// two at a time: 104 us at 32^3, stage mean).
+// two at a time: IMEX step at 32^3 2.45 against 2.25 ms).
 template <int is>
 __global__ void __launch_bounds__(IMEX_THREADS)
 k_imex_start(long long npoin, const int *__restrict__ work, ImexCoef k, float dt, float fact, float gm1,

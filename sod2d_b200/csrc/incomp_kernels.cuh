@@ -522,7 +522,7 @@ __device__ bool grid_sum(double (&v)[ND], double *__restrict__ part, unsigned *t
   return true;
 }
 
-// q = assembled Laplacian slots (Kahan, as k_gather1; node-sorted by
+// q = assembled Laplacian slots (Kahan, as k_gather_sorted1; written by
 // k_lap_elem<DIR>) with the p.q partials; the last block sets alpha = rz / pq.
 // The new search direction p = z + beta p is formed and stored here for every
 // node with slots (the working nodes).  V = float: the reference's FP32

@@ -15,9 +15,9 @@ struct State5 {
 // ---- RK stage update (time_integ_ls.f90:323-332 and :350-359) ---------
 // first != 0: U2 += g*dt*R.  Otherwise U2 = l1*U1 + li*U2 + g*dt*R.
 // The FP32 shadow (reference layout: rho, q(N,3), E) receives the result.
-// The first stage also fills U1: U1 receives the level that U2 held, in place of a copy
-// before the step; U1 is read only where l1 is not zero.  Bound by HBM
-// (48^3, FP64: 192 B a node in 71-80 us, 6.0 TB/s).
+// The first stage also fills U1 with the level that U2 held, in place of a
+// copy before the step; U1 is read only where l1 is not zero.  Bound by HBM
+// (48^3, FP64, l1 = 0: 124 B a node in 62 us, 6.0 TB/s).
 template <class T>
 __global__ void k_stage(int npoin_w, long long npoin, const int *__restrict__ lpoin_w, State5<T> U1, State5<T> U2,
                         const float *__restrict__ Rmass, const float *__restrict__ Rmom,
