@@ -42,7 +42,7 @@ sys.path.insert(0, str(ROOT))
 B_PER_NODE_STAGE = 402.0
 # DRAM bytes (read + write) of one RHS evaluation per working node, from one
 # ncu capture of the four RHS kernels on the 64^3 workload itself
-# (5,535,995,392 B for 7,077,888 working nodes).
+# (5,519,768,960 B for 7,077,888 working nodes).
 DRAM_B_PER_NODE_STAGE = 5519768960 / 7077888
 NELEM_1D = 64
 PORDER = 3
