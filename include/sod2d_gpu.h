@@ -136,8 +136,11 @@ int sod_gpu_halo_update(sod_gpu_ctx *ctx, float *field, int ncomp);
  * SOD_REDUCE_MAX_F32 (float) or SOD_REDUCE_SUM_F64 (double); when it
  * returns the result is in `buf` or enqueued on `stream`.  Every rank of the
  * plan makes the same calls in the same order.  Setting it (a collective
- * call) also sums the mesh volume of the analysis over the ranks.  With a
- * halo plan, sod_gpu_comp_rk_ls_step, sod_gpu_comp_imex_step,
+ * call) also sums the mesh volume of the analysis over the ranks.  It is
+ * called with or without a halo plan: a part that shares no node has no
+ * plan and joins the same reductions (but for sod_gpu_pressure_solve, which
+ * without a plan solves this part's system alone).  With a halo plan,
+ * sod_gpu_comp_rk_ls_step, sod_gpu_comp_imex_step,
  * sod_gpu_comp_adapt_dt and sod_gpu_comp_analysis do the halo sums and
  * reductions of rk_4_ls_main and imex_main; the IMEX solve's dot products
  * run over the working nodes this rank owns (a shared node belongs to the

@@ -598,7 +598,7 @@ int sod_gpu_comp_imex_step(sod_gpu_ctx *c, float dt, int maxIter, double tol) {
     }
   }
   int iters = 0;
-  const bool dev = !c->halo.on;
+  const bool dev = solves_alone(c);
   if (dev) {  // D(x0) of the step's initial state, the first residual's operator in every stage
     k_imex_prim<<<nb, 256, 0, st>>>(nw, N, c->lpoin_w, gm - 1.0f, c->phys.Rgas, X.lvl1, X.lvl1, X.au, X.aT);
     if ((rc = ensure_cg_loop(c)) || (rc = imex_diffusion(c, X.lvl1, X.lvl1, X.au, X.aT, X.Dx0))) {

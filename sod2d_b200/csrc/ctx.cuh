@@ -507,6 +507,12 @@ inline int allreduce(sod_gpu_ctx *c, void *buf, int count, int kind) {
   return 0;
 }
 
+// Whether a solve's dot products are this rank's alone: its iteration may
+// then run on the device.  With a halo plan or an allreduce callback (a part
+// that shares no node has no plan, but the same reductions as the other
+// ranks) every sum passes through the callback.
+inline bool solves_alone(const sod_gpu_ctx *c) { return !c->halo.on && !c->halo.reduce; }
+
 // Entry points whose solves need global dot products refuse a partitioned mesh.
 inline int no_partition(sod_gpu_ctx *c, const char *what) {
   if (c && c->halo.on) return fail(SOD_GPU_EINVAL, std::string(what) + " is not available with a halo plan");

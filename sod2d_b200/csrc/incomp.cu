@@ -76,8 +76,8 @@ namespace {
 // alpha; update, norms and beta) and one host read per batch of iterations,
 // where six launches and a host read per iteration left the GPU idle a third
 // of the time.  The scalars are rounded as on the host: same iterates but
-// for the order of the FP64 sums.  (A partitioned mesh, whose dot products
-// pass through the caller's allreduce, keeps the host loop below.)
+// for the order of the FP64 sums.  (Where dot products pass through the
+// caller's allreduce, the host loop below runs: solves_alone.)
 int conjgrad_pressure_dev(sod_gpu_ctx *c, const float *Rp0, float *R, int maxIter, double tol, int *iters,
                           double *res_rel) {
   int rc;
@@ -124,7 +124,7 @@ extern "C" {
 int sod_gpu_conjgrad_pressure(sod_gpu_ctx *c, const float *Rp0, float *R, int maxIter, double tol, int *iters,
                               double *res_rel) {
   if (!c || !Rp0 || !R || maxIter < 1) return fail(SOD_GPU_EINVAL, "bad argument");
-  if (!c->halo.on) return conjgrad_pressure_dev(c, Rp0, R, maxIter, tol, iters, res_rel);
+  if (solves_alone(c)) return conjgrad_pressure_dev(c, Rp0, R, maxIter, tol, iters, res_rel);
   int rc;
   if ((rc = ensure_diag(c)) || (rc = ensure_cg32(c))) return rc;
   auto &G = c->cg;
@@ -818,7 +818,7 @@ int sod_gpu_conjgrad_veloc(sod_gpu_ctx *c, float fact, float dt, const float *mu
   CUDA_TRY(cudaMemcpyAsync(V.b, R, 3 * N * 4, cudaMemcpyDeviceToDevice, c->stream));
   k_species_tau<<<nblk(c->nelem, 8), 256, 0, c->stream>>>(c->nelem, c->N, c->conn, c->helem, V.x, N,
                                                           c->phys.c_species_stab / (float)c->P, V.tau_e);
-  if (!c->halo.on) {
+  if (solves_alone(c)) {
     rc = conjgrad_veloc_dev(c, fact, dt, mu_fluid, musgs, maxIter, tol, iters, res_rel);
     c->async = was_async;
     if (rc) return rc;

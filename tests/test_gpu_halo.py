@@ -389,3 +389,119 @@ def test_partition_refuses_global_solves(gpu):
     with pytest.raises(RuntimeError, match="halo plan"):
         ctx.call("sod_gpu_incomp_step", C.c_float(1e-3), C.byref(gpu.SolveOpts(10, 1e-8, 1, 50, 0)), C.byref(st))
     ctx.close()
+
+
+# ---- parts that share no node: global reductions without a halo plan --------
+
+
+class _Part:
+    def __init__(self, rank):
+        self.rank = rank
+
+
+def _lone_parts(gpu, porder):
+    """Two meshes without a common node: ranks of one job with no halo plan."""
+    meshes = [host.periodic_cube(porder, 3, 4, 5, jitter=0.05, seed=8, ordering=1, elem_shuffle=True),
+              host.periodic_cube(porder, 2, 3, 3, jitter=0.05, seed=9)]
+    return meshes, LocalHaloGroup([_Part(0), _Part(1)], timeout=120.0)
+
+
+def _block_pcg(oms, x0, b, maxit, tol):
+    """Jacobi-PCG in FP64 on the two decoupled Laplacians as one system."""
+    cat = np.concatenate
+    A = lambda v: cat([O.laplacian(om, p) for om, p in zip(oms, np.split(v, [oms[0].mesh.npoin]))])
+    d = cat([O.laplacian_diag(om) for om in oms])
+    inv = np.divide(1.0, d, out=np.zeros_like(d), where=d != 0)
+    x = np.zeros_like(b)
+    r = np.where(d != 0, b - A(x0), 0.0)
+    z = inv * r
+    p, r0, rz = z.copy(), np.linalg.norm(r), r @ z
+    for it in range(1, maxit + 1):
+        q = A(p)
+        a = rz / (p @ q)
+        x, r = x + a * p, r - a * q
+        if np.linalg.norm(r) < tol * r0:
+            break
+        z = inv * r
+        rz, old = r @ z, rz
+        p = z + rz / old * p
+    return x0 + x, it
+
+
+@pytest.mark.parametrize("porder", [3, 4])
+def test_pressure_cg_reduces_without_a_plan(gpu, porder):
+    meshes, group = _lone_parts(gpu, porder)
+    oms = [O.OracleMesh(m, np.float64) for m in meshes]
+    rng = np.random.default_rng(3)
+    p = [np.zeros(m.npoin) for m in meshes]
+    for k, m in enumerate(meshes):
+        w = m.lpoin_w - 1
+        p[k][w] = (1.0, 4.0)[k] * rng.normal(size=w.size)
+    b = [O.laplacian(om, q).astype(np.float32) for om, q in zip(oms, p)]
+    x0 = [np.zeros(m.npoin, np.float32) for m in meshes]
+    ref, ref_it = _block_pcg(oms, np.concatenate(x0).astype(np.float64), np.concatenate(b).astype(np.float64), 200, 1e-3)
+
+    def job(k):
+        ctx = gpu.Context(meshes[k], gpu.default_phys())
+        ctx.set_allreduce(group, k)
+        dx, dR = torch.from_numpy(x0[k]).cuda(), torch.from_numpy(b[k].copy()).cuda()
+        it, res = C.c_int(), C.c_double()
+        ctx.call("sod_gpu_conjgrad_pressure", gpu.dptr(dx), gpu.dptr(dR), 200, 1e-3, C.byref(it), C.byref(res))
+        out = dR.cpu().numpy()
+        ctx.close()
+        return it.value, res.value, out
+
+    r = group.run([lambda k=k: job(k) for k in (0, 1)])
+    assert r[0][:2] == r[1][:2]  # one solve, not two
+    assert abs(r[0][0] - ref_it) <= 1
+    for k, m in enumerate(meshes):
+        w = m.lpoin_w - 1
+        x = np.split(ref, [meshes[0].npoin])[k][w]
+        # one iteration more or less moves the iterate by the residual's order
+        assert np.linalg.norm(r[k][2][w] - x) <= 5e-3 * np.linalg.norm(x)
+
+
+@pytest.mark.parametrize("porder", [3, 4])
+def test_velocity_cg_reduces_without_a_plan(gpu, porder):
+    meshes, group = _lone_parts(gpu, porder)
+
+    def job(k):
+        m = meshes[k]
+        N = m.npoin
+        rng = np.random.default_rng(5 + k)
+        dv = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+        u = rng.normal(size=3 * N).astype(np.float32)
+        ctx = gpu.Context(m, gpu.default_phys())
+        ctx.set_allreduce(group, k)
+        du, dmu, R = dv(u), dv(np.full(N, (1e-2, 2e-1)[k], np.float32)), dv((u.reshape(3, N) * m.Ml).reshape(-1))
+        it, res = C.c_int(), C.c_double()
+        ctx.call("sod_gpu_conjgrad_veloc", 1.0, 0.05, gpu.dptr(dmu), None, gpu.dptr(du), gpu.dptr(R), 60, 1e-5,
+                 C.byref(it), C.byref(res))
+        ctx.close()
+        return it.value, res.value
+
+    r = group.run([lambda k=k: job(k) for k in (0, 1)])
+    assert r[0] == r[1] and r[0][1] < 1e-5
+
+
+def test_imex_step_reduces_without_a_plan(gpu):
+    meshes, group = _lone_parts(gpu, 3)
+    ics = [host.tgv_comp_init(m, Ma=1.25) for m in meshes]
+
+    def job(k):
+        s = gpu.CompSolver(meshes[k], ics[k], stages=4, fp64_state=False, cfl_conv=0.95, cfl_diff=1000.5, imex=True,
+                           imex_maxiter=50, imex_tol=1e-6)
+        s.ctx.set_allreduce(group, k)
+        s.dt = s.adapt_dt()
+        out = []
+        for _ in range(2):
+            s.step()
+            it, res = C.c_int(), C.c_double()
+            s.ctx.call("sod_gpu_comp_imex_stats", C.byref(it), C.byref(res))
+            s.dt = s.adapt_dt()
+            out.append((it.value, res.value, s.dt))
+        s.close()
+        return out
+
+    r = group.run([lambda k=k: job(k) for k in (0, 1)])
+    assert r[0] == r[1]
