@@ -266,9 +266,8 @@ int sod_gpu_comp_rk_ls_step(sod_gpu_ctx *c, float dt) {
   // tau from level 2 (comp_tau)
   comp_tau(c, S.csound, S.u2, S.tau);
   // level 1 <- level 2 (CFDSolverBase.f90:1951-1960): the first stage fills
-  // U1, thermo_entropy eta1; the velocity changes buffers (u2 is written at
-  // the end of the step, and read before that nowhere)
-  std::swap(S.u1, S.u2);
+  // U1, k_eos_end u1, thermo_entropy eta1 (on the first step u1 holds the
+  // initial velocity, as u2 does)
   if (S.first) CUDA_TRY(cudaMemcpyAsync(S.eta1, S.eta2, N * 4, cudaMemcpyDeviceToDevice, st));
   if (S.first) {
     S.first = false;
@@ -294,7 +293,7 @@ int sod_gpu_comp_rk_ls_step(sod_gpu_ctx *c, float dt) {
   const float gm = c->phys.gamma_gas;
   launch_pdl(k_eos_end, nblk(c->npoin_w, 256), 256, 0, st, c->npoin_w, c->npoin, c->lpoin_w, gm - 1.0f, gm,
              c->phys.Rgas, S.rho32, S.q32, S.E32, S.u2, S.eint, S.pr, S.csound, S.machno, S.Tem, S.mu_factor,
-             S.mu_fluid);
+             S.mu_fluid, S.u1);
   launch_pdl(k_thermo_entropy, nblk(c->npoin_w, 256), 256, 0, st, c->npoin_w, c->lpoin_w, gm, c->phys.p_inf, c->phys.rho_inf,
              S.rho32, S.pr, S.eta1, S.eta2);
   int rc = comp_entropy_pass(c, S.Reta2, true);
@@ -615,7 +614,7 @@ int sod_gpu_comp_imex_step(sod_gpu_ctx *c, float dt, int maxIter, double tol) {
     }
     iters += X.cg_iters;
     k_eos_end<<<nb, 256, 0, st>>>(nw, N, c->lpoin_w, gm - 1.0f, gm, c->phys.Rgas, S.rho32, S.q32, S.E32, S.u2, S.eint,
-                                  S.pr, S.csound, S.machno, S.Tem, 0.f, nullptr);
+                                  S.pr, S.csound, S.machno, S.Tem, 0.f, nullptr, nullptr);
     if ((rc = imex_convec_state(c, X.R + (is - 1) * B)) ||
         (rc = imex_diffusion(c, nullptr, S.rho32, S.u2, S.Tem, X.D + (is - 1) * B))) {
       c->async = was_async;

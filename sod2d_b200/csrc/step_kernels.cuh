@@ -51,12 +51,17 @@ __global__ void k_stage(int npoin_w, long long npoin, const int *__restrict__ lp
 }
 
 // ---- end-of-step EOS (time_integ_ls.f90:391-407), with the Sutherland
-// viscosity of the new temperature (as k_sutherland) when mu is given ------
+// viscosity of the new temperature (as k_sutherland) when mu is given; u1,
+// when given, receives the velocity that u held (level 1 <- level 2: here
+// and not before the step, so that a step that fails in a callback leaves
+// the velocity as it was, and by a store instead of an exchange of pointers,
+// so that a captured step can be replayed; 24 B a node) ------------------
 static __global__ void k_eos_end(int npoin_w, long long npoin, const int *__restrict__ lpoin_w, float gm1, float gamma,
                           float Rgas, const float *__restrict__ rho, const float *__restrict__ q,
                           const float *__restrict__ E, float *__restrict__ u, float *__restrict__ eint,
                           float *__restrict__ pr, float *__restrict__ csound, float *__restrict__ machno,
-                          float *__restrict__ Tem, float mu_factor, float *__restrict__ mu) {
+                          float *__restrict__ Tem, float mu_factor, float *__restrict__ mu,
+                          float *__restrict__ u1) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npoin_w) return;
   const long long p = lpoin_w[t];
@@ -68,6 +73,7 @@ static __global__ void k_eos_end(int npoin_w, long long npoin, const int *__rest
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     uu[d] = q[p + npoin * d] / r;
+    if (u1) u1[p + npoin * d] = u[p + npoin * d];
     u[p + npoin * d] = uu[d];
     umag = umag + uu[d] * uu[d];
   }

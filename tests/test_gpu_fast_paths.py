@@ -185,3 +185,67 @@ def test_velocity_cg_batches(gpu, porder, maxit):
     assert abs(res.value - rr) <= 0.05 * rr
     assert rel_l2(R.cpu().numpy().reshape(3, N)[:, w], xr.reshape(3, N)[:, w]) < 1e-5
     ctx.close()
+
+
+@pytest.mark.parametrize("porder,stages,fp64", [(3, 4, True), (4, 5, False)])
+def test_rk_step_under_capture(gpu, porder, stages, fp64):
+    """A recorded RK step, replayed, is the next step each time: no level of
+    the state changes its buffer on the host."""
+    m = host.periodic_cube(porder, 3, 4, 5)
+    ic = host.tgv_comp_init(m, Ma=1.25)
+    eager, rec = (gpu.CompSolver(m, ic, stages=stages, fp64_state=fp64) for _ in range(2))
+    for s in (eager, rec):
+        s.step()  # the first step has a start-up of its own
+        s.dt = 0.5 * s.dt
+    for _ in range(3):
+        eager.step()
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    rec.ctx.call("sod_gpu_set_stream", C.c_void_p(st.cuda_stream))
+    rec.ctx.call("sod_gpu_set_async", 1)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        rec.ctx.call("sod_gpu_comp_rk_ls_step", float(rec.dt))
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    rec.ctx.call("sod_gpu_set_async", 0)
+    rec.ctx.call("sod_gpu_set_stream", None)
+    a, b = eager.state(), rec.state()
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
+    assert eager.adapt_dt() == rec.adapt_dt()
+    eager.close()
+    rec.close()
+
+
+@pytest.mark.parametrize("fail_at", [1, 2, 5])
+def test_failed_rk_step_keeps_the_velocity(gpu, fail_at):
+    """A halo exchange that fails inside a step: the CFL time step afterwards
+    is still that of the state before it."""
+    m = host.periodic_cube(3, 3, 4, 5)
+    ic = host.tgv_comp_init(m, Ma=1.25)
+    s = gpu.CompSolver(m, ic, stages=4, fp64_state=True, cfl_diff=1e6)  # the convective limit alone
+
+    class Plan:  # a neighbour that shares no node: the callback is called, nothing moves
+        rank, numRanksWithComms, numNodesToComm = 0, 1, 0
+        ranksToComm, commsMemPosInLoc, commsMemSize, nodesToComm = [1], [1], [0], []
+
+    class Transport:
+        left = -1
+
+        def exchange(self, plan, send, recv, width):
+            self.left -= 1
+            if self.left == 0:
+                raise ConnectionError("lost rank")
+
+    t = Transport()
+    s.ctx.set_halo(Plan, t)
+    for _ in range(2):
+        s.step()
+    dt = s.adapt_dt()
+    t.left = fail_at
+    with pytest.raises(RuntimeError, match="halo exchange failed"):
+        s.step()
+    assert s.adapt_dt() == dt
+    s.close()
