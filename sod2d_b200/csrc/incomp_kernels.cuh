@@ -55,6 +55,7 @@ k_lap_elem(MeshDev m, DMat<P, V> D, const V *__restrict__ p, V *__restrict__ slo
   const long long e = (long long)blockIdx.x * L::EPB + el;
   const bool active = e < m.nelem && c < N2;
   const int i = c % N1, j = c / N1;
+  if (ended_late(stop, 148 * L::MINB)) return;
   int n[N1], pos[N1];
   float G[N1][10];
   V Di[N1], Dj[N1];
@@ -431,8 +432,8 @@ __global__ void __launch_bounds__(DOT_THREADS) k_dot(int npoin_w, const int *__r
 
 // ---- device-resident preconditioned CG -------------------------------------
 // Scalars of the iteration kept in device memory between launches, so that
-// the host only reads them once per batch of iterations.  Every iteration
-// kernel returns at once when status != 0.
+// the host only reads them once per batch of iterations.  The iteration
+// kernels write nothing when status != 0 (what they still load: ended_late).
 struct CgScal {
   double rz;     // r . z of the current residual
   double pq;     // p . A p
@@ -446,6 +447,7 @@ struct CgScal {
 
 // threads per block; nodes per thread of the update and assembly kernels
 constexpr int CG_THREADS = 256, CG_U = 4, CG_QU = 2;
+constexpr unsigned CG_WAVE = 148 * 4;  // see ended_late
 
 // Node loops of the CG kernels handle several nodes per thread and issue all
 // their loads before any store, so that each thread keeps several memory
@@ -531,6 +533,7 @@ template <class V>
 __global__ void __launch_bounds__(CG_THREADS)
 k_cg_q(MeshDev m, const V *__restrict__ slots, V *__restrict__ p, V *__restrict__ q, CgScal *S,
        double *__restrict__ part, unsigned *ticket, const V *__restrict__ z) {
+  if (ended_late(&S->status, CG_WAVE)) return;
   constexpr int U = CG_QU, MS = 8;  // nodes per thread, slots loaded ahead per node
   const long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
   int b[U], en[U];
@@ -608,6 +611,7 @@ k_cg_update(long long npoin, const double *__restrict__ p, const double *__restr
             const double *__restrict__ Minv, double *__restrict__ x, double *__restrict__ r, double *__restrict__ z,
             CgScal *S, double *__restrict__ hist, int hist_cap, double *__restrict__ part, unsigned *ticket,
             float *__restrict__ uf) {
+  if (ended_late(&S->status, CG_WAVE)) return;
   constexpr int U = CG_U;
   const long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
   double mv[U];
@@ -671,6 +675,7 @@ static __global__ void __launch_bounds__(CG_THREADS)
 k_cg_update32(long long npoin, const float *__restrict__ p, const float *__restrict__ q, const float *__restrict__ M,
               float *__restrict__ x, float *__restrict__ r, float *__restrict__ z, CgScal *S,
               double *__restrict__ part, unsigned *ticket) {
+  if (ended_late(&S->status, CG_WAVE)) return;
   constexpr int U = CG_U;
   const long long base = (long long)blockIdx.x * blockDim.x * U + threadIdx.x;
   float mv[U];

@@ -53,7 +53,7 @@ def test_laplacian_block_remainders(gpu, porder, size):
     ctx.close()
 
 
-# batches of 20 iterations: one, a whole batch, one more, and convergence inside a batch
+# one iteration, the usual maximum, one more, and convergence inside a batch of iterations
 @pytest.mark.parametrize("porder,maxit,tol", [(3, 1, 1e-6), (3, 20, 1e-6), (3, 21, 1e-6), (4, 45, 1e-7), (4, 200, 1e-3)])
 def test_fp32_pressure_cg_batches(gpu, porder, maxit, tol):
     m = host.periodic_cube(porder, 3, 4, 5, jitter=0.05, seed=8, ordering=1, elem_shuffle=True)
@@ -164,7 +164,7 @@ def test_rhs_under_capture(gpu, porder, n):
     ctx.close()
 
 
-# the velocity solve reads its scalars every fourth iteration
+# one iteration, and batches cut by the maximum
 @pytest.mark.parametrize("porder,maxit", [(3, 1), (3, 4), (4, 5)])
 def test_velocity_cg_batches(gpu, porder, maxit):
     m = host.periodic_cube(porder, 3, 4, 5, jitter=0.05, seed=8, ordering=1, elem_shuffle=True)
@@ -249,3 +249,45 @@ def test_failed_rk_step_keeps_the_velocity(gpu, fail_at):
         s.step()
     assert s.adapt_dt() == dt
     s.close()
+
+
+def _launches(fn, kernel):
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    return sum(e.count for e in prof.key_averages() if kernel in e.key)
+
+
+@pytest.mark.parametrize("porder", [3, 4])
+def test_solves_that_converge_at_once_queue_no_tail(gpu, porder):
+    """Iterations queued beyond convergence are launches and mesh reads for
+    nothing: none after one or two pressure iterations but the second, none
+    after one velocity iteration."""
+    m = host.periodic_cube(porder, 3, 4, 5, jitter=0.05, seed=8)
+    N, w = m.npoin, m.lpoin_w - 1
+    rng = np.random.default_rng(3)
+    p = np.zeros(N, np.float32)
+    p[w] = rng.normal(size=w.size)
+    b, x0, u = dv(O.laplacian(O.OracleMesh(m), p)), torch.zeros(N, device="cuda"), dv(rng.normal(size=3 * N).astype(np.float32))
+    mu = torch.full((N,), 1e-2, device="cuda")
+    bv = u * dv(m.Ml).repeat(3)
+    ctx = gpu.Context(m, gpu.default_phys())
+    it, res = C.c_int(), C.c_double()
+
+    def pressure(maxit, tol):
+        R = b.clone()
+        ctx.call("sod_gpu_conjgrad_pressure", gpu.dptr(x0), gpu.dptr(R), maxit, tol, C.byref(it), C.byref(res))
+
+    def velocity(maxit, tol):
+        R = bv.clone()
+        ctx.call("sod_gpu_conjgrad_veloc", 1.0, 0.05, gpu.dptr(mu), None, gpu.dptr(u), gpu.dptr(R), maxit, tol,
+                 C.byref(it), C.byref(res))
+
+    for solve, kernel, its, queued in ((pressure, "k_lap_elem", 1, 2), (pressure, "k_lap_elem", 2, 2),
+                                       (velocity, "k_tauv_elem", 1, 1)):
+        solve(its, 1e-30)  # the residual after `its` iterations is the next solve's tolerance
+        tol = 1.001 * res.value
+        assert _launches(lambda: solve(20, tol), kernel) == 1 + queued  # and the residual of the start
+        assert it.value <= its
+    ctx.close()
