@@ -615,15 +615,20 @@ k_rhs(MeshDev m, Phys ph, float Rgas, RhsArgs A, float *__restrict__ slots) {
     float mu = 0.f, rhon_in = 0.f, H = 0.f, rH = 0.f;
     if (active) {
       const float *in = cur + L::O_IN + tid;
-      if (IN == IN_CONS) {
+      if (IN == IN_CONS && DIFF) {
         eos_fast(ph, invR, A.mu_factor, in[0], in[NTB], in[2 * NTB], in[3 * NTB], in[4 * NTB], s);
         mu = s.mu;
         const float ri = __frcp_rn(s.rho);
-        if (FLUX2) {  // u = q / rho to half an ulp: rho u stands for q below
-          s.u0 = fmaf(fmaf(-s.rho, s.u0, s.q0), ri, s.u0);
-          s.u1 = fmaf(fmaf(-s.rho, s.u1, s.q1), ri, s.u1);
-          s.u2 = fmaf(fmaf(-s.rho, s.u2, s.q2), ri, s.u2);
-        }
+        // u = q / rho to half an ulp: rho u stands for q below
+        s.u0 = fmaf(fmaf(-s.rho, s.u0, s.q0), ri, s.u0);
+        s.u1 = fmaf(fmaf(-s.rho, s.u1, s.q1), ri, s.u1);
+        s.u2 = fmaf(fmaf(-s.rho, s.u2, s.q2), ri, s.u2);
+      } else if (IN == IN_CONS) {
+        // convection alone (the IMEX stages): u, p and h by the divisions of
+        // k_eos_end and k_aux_h.  eos_fast here raised the momentum's error
+        // at Ma = 0.1, order 4, by 2 %; the step takes as long (2.23 ms at 32^3).
+        eos(ph, Rgas, A.mu_factor, in[0], in[NTB], in[2 * NTB], in[3 * NTB], in[4 * NTB], s);
+        s.T = 0.f;
       } else if (IN == IN_PRIM) {
         s.rho = in[0];
         s.u0 = in[NTB]; s.u1 = in[2 * NTB]; s.u2 = in[3 * NTB];

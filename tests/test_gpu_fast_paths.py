@@ -291,3 +291,21 @@ def test_solves_that_converge_at_once_queue_no_tail(gpu, porder):
         assert _launches(lambda: solve(20, tol), kernel) == 1 + queued  # and the residual of the start
         assert it.value <= its
     ctx.close()
+
+
+@pytest.mark.parametrize("porder,size,stages", [(3, (6, 5, 7), 4), (4, (5, 4, 6), 3)])
+def test_imex_step_rounds_no_worse_than_fp32_reference(gpu, porder, size, stages):
+    """At Ma = 0.1 the pressure is 70 times rho u^2 and its rounding sets the
+    momentum's error: against FP64 it is no larger than that of the reference
+    arithmetic in FP32 (the oracle's)."""
+    m = host.periodic_cube(porder, *size)
+    ic = host.tgv_comp_init(m, Ma=0.1)
+    kw = dict(imex=True, cfl_conv=0.95, cfl_diff=1000.5)
+    prm = O.comp_params(ic, stages=stages, first_mue=True, **kw)
+    ref, f32 = (O.tgv_comp_run(O.OracleMesh(m, t), ic, prm, 1)[1] for t in (np.float64, np.float32))
+    s = gpu.CompSolver(m, ic, stages=stages, fp64_state=False, **kw)
+    s.step()
+    got = s.state()
+    s.close()
+    q = lambda f: np.asarray(f["q"], np.float64).reshape(3, -1)[:, m.lpoin_w - 1]
+    assert rel_l2(q(got), q(ref)) <= rel_l2(q(f32), q(ref))
