@@ -103,7 +103,7 @@ inline int ensure_cg32(sod_gpu_ctx *c) {
   auto &G = c->cg;
   if (G.ready32) return 0;
   int rc;
-  for (float **pp : {&G.x32, &G.r32, &G.p32, &G.q32, &G.z032, &G.z132, &G.b32})
+  for (float **pp : {&G.x32, &G.r32, &G.p32, &G.q32, &G.z032})
     if ((rc = c->alloc(pp, (size_t)c->npoin))) return rc;
   G.ready32 = true;
   return 0;

@@ -70,7 +70,8 @@ struct sod_gpu_ctx {
   struct Cg {
     bool ready32 = false, ready64 = false, have_diag = false;
     float *diag = nullptr;                                     // Jacobi diagonal (FP32)
-    float *x32, *r32, *p32, *q32, *z032, *z132, *b32;          // reference-arithmetic CG
+    float *x32, *r32, *p32, *q32, *z032;                       // reference-arithmetic CG
+    float *z132 = nullptr, *b32 = nullptr;                     //   its host-driven loop's
     double *x, *r, *p, *q, *z0, *z1, *b, *Minv;                // FP64 CG
     double *part, *dots;                                        // reductions
     CgScal *S = nullptr, *S_h = nullptr;                        // device-resident CG scalars (+ pinned host copy)
@@ -120,7 +121,8 @@ struct sod_gpu_ctx {
   // implicit velocity solve (conjGrad_veloc_incomp)
   struct Velo {
     float *tauP = nullptr, *tau_e = nullptr;                   // [npoin][8] projection, [E] tau
-    float *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *z1 = nullptr, *b = nullptr;  // (npoin,3)
+    float *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *b = nullptr;  // (npoin,3)
+    float *z = nullptr, *z1 = nullptr;                         // the host-driven loop's
   } velo;
   // compressible time-integration state
   struct Comp {
@@ -137,8 +139,10 @@ struct sod_gpu_ctx {
   // IMEX integrator scratch (five-variable blocks [mass][energy][momentum])
   struct Imex {
     float *R = nullptr, *D = nullptr;  // [4 stages][5N] explicit / implicit residuals
-    float *stab = nullptr, *lvl1 = nullptr, *aux_h = nullptr, *Dx0 = nullptr;
-    float *x = nullptr, *r = nullptr, *p = nullptr, *qn = nullptr, *b = nullptr, *z = nullptr, *z1 = nullptr;
+    float *stab = nullptr, *lvl1 = nullptr, *aux_h = nullptr;
+    float *x = nullptr, *r = nullptr, *p = nullptr, *qn = nullptr;
+    float *Dx0 = nullptr;                                    // the device loop's: D(x0) of the step
+    float *b = nullptr, *z = nullptr, *z1 = nullptr;         // the host-driven loop's
     float *au = nullptr, *aT = nullptr, *zmu = nullptr, *zmue = nullptr;  // CG primitives; zero viscosities
     int cg_iters = 0;
     double cg_res = 0.0;
@@ -175,6 +179,13 @@ struct sod_gpu_ctx {
     if (e != cudaSuccess) return fail(SOD_GPU_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     allocs.push_back(*p);
     bytes += b;
+    return 0;
+  }
+  // workspaces that one of a solve's two loops needs, at its first use
+  template <class... T>
+  int alloc_once(size_t count, T *...p) {
+    for (float **q : {p...})
+      if (int rc = *q ? 0 : alloc(q, count)) return rc;
     return 0;
   }
   template <class T>

@@ -309,3 +309,32 @@ def test_imex_step_rounds_no_worse_than_fp32_reference(gpu, porder, size, stages
     s.close()
     q = lambda f: np.asarray(f["q"], np.float64).reshape(3, -1)[:, m.lpoin_w - 1]
     assert rel_l2(q(got), q(ref)) <= rel_l2(q(f32), q(ref))
+
+
+def test_solves_allocate_their_own_loops_workspaces(gpu):
+    """Device memory that the solves add to a context without global
+    reductions, in arrays of npoin floats: those of the device loops only."""
+    m = host.periodic_cube(3, 6, 7, 8)
+    N, EN = m.npoin, m.nelem * m.nnode
+    small = 4 * (m.nelem + 6 * (N // 256 + 1)) + 64 * 1024  # per-element tau, partial sums, scalars
+    z = torch.zeros(3 * N, device="cuda")
+    one = torch.ones(3 * N, device="cuda")
+    mu = torch.full((N,), 1e-2, device="cuda")
+    ctx = gpu.Context(m, gpu.default_phys())
+    b0 = ctx.device_bytes
+    R = one.clone()
+    ctx.call("sod_gpu_conjgrad_veloc", 1.0, 0.05, gpu.dptr(mu), None, gpu.dptr(z), gpu.dptr(R), 5, 1e-2, None, None)
+    b1 = ctx.device_bytes
+    assert b1 - b0 <= 23 * 4 * N + small  # projection 8, x r p q b 15
+    R = one[:N].clone()
+    R[0] = 2.0
+    ctx.call("sod_gpu_conjgrad_pressure", gpu.dptr(z), gpu.dptr(R), 5, 1e-2, None, None)
+    assert ctx.device_bytes - b1 <= 6 * 4 * N + small  # diagonal, x r p q z
+    ctx.close()
+    s = gpu.CompSolver(m, host.tgv_comp_init(m, Ma=1.25), stages=4, fp64_state=False, cfl_conv=0.95, cfl_diff=1000.5,
+                       imex=True)
+    b0 = s.ctx.device_bytes
+    s.step()
+    # stages 40, stabilisation, level 1, D(x0), x r p qn 35, enthalpy, velocity, temperature, viscosity 6
+    assert s.ctx.device_bytes - b0 <= 4 * (81 * N + EN) + small
+    s.close()
