@@ -604,7 +604,8 @@ k_cg_q(MeshDev m, const V *__restrict__ slots, V *__restrict__ p, V *__restrict_
 // the last block records ||r||^2, detects convergence and, with JAC, sets
 // the Polak-Ribiere beta = r.(z - z_old) / rz_old.  Runs over all nodes in
 // order, with no index loads: Minv is 0 off the working nodes, which are
-// left alone.
+// left alone.  Minv (or D^-1/2) is read before the wait: k_cg_q, which comes
+// before this kernel, does not write it.
 template <bool JAC>
 __global__ void __launch_bounds__(CG_THREADS)
 k_cg_update(long long npoin, const double *__restrict__ p, const double *__restrict__ q,
@@ -670,7 +671,8 @@ k_cg_update(long long npoin, const double *__restrict__ p, const double *__restr
 // The same update of the reference's FP32 solve (mod_solver_incomp.f90:
 // 395-440): z = r / M with M the Laplacian's diagonal (0 off the working
 // nodes), FP64 sums of FP32 products, beta rounded to FP32, converged when
-// ||r|| < thr2 (here tol ||b||).
+// ||r|| < thr2 (here tol ||b||).  M is read before the wait: k_cg_q does not
+// write it.
 static __global__ void __launch_bounds__(CG_THREADS)
 k_cg_update32(long long npoin, const float *__restrict__ p, const float *__restrict__ q, const float *__restrict__ M,
               float *__restrict__ x, float *__restrict__ r, float *__restrict__ z, CgScal *S,
@@ -758,7 +760,8 @@ k_cg_start32(long long npoin, const float *__restrict__ R, const float *__restri
 // Learned preconditioner: z(n) = D^-1/2(n) (exp(alpha) D^-1/2(n) r(n) + sum of
 // the node's contributions, stored contiguously from pptr[n]) (as
 // k_patch_gather_perm), with the partials r.z and r.z_old; the last block
-// sets beta and rz.
+// sets beta and rz.  D^-1/2 and the parameter are read before the wait:
+// k_patch_apply_tc, which comes before this kernel, does not write them.
 static __global__ void __launch_bounds__(CG_THREADS)
 k_cg_patch_z(long long npoin, const int *__restrict__ pptr, const float *__restrict__ ctr,
              const double *__restrict__ r, const double *__restrict__ Dh, const float *__restrict__ prm, int o_alpha,

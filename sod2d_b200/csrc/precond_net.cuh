@@ -285,7 +285,7 @@ k_patch_apply_tc(long long nelem, const int *__restrict__ pt, const int *__restr
     B2[j * T::S2 + kpair_pos(k)] = b;
   }
   __syncthreads();
-  pdl_wait();  // the parameters do not change during a solve: staged while the update kernel ends
+  pdl_wait();  // the parameters were staged while k_cg_update, which does not write them, ends
   pdl_trigger();
   if (stop && *stop) return;
   const int g = lane >> 2, t = lane & 3;

@@ -43,11 +43,14 @@ struct Phys {
 };
 
 // Programmatic dependent launch: a kernel started with launch_pdl (ctx.cuh)
-// may begin while the kernel before it in the stream still runs.  What it
-// reads or writes of earlier kernels' results comes after pdl_wait(), which
-// returns when they are complete and visible; before it, only arrays that no
-// kernel of the stream's current work writes (the mesh).  pdl_trigger() lets
-// the next such kernel begin.  Both do nothing in an ordinary launch.
+// may begin while the kernel before it in the stream still runs.
+// pdl_wait() returns when the kernels before are complete and visible (at
+// once in an ordinary launch); pdl_trigger() lets a next kernel that was
+// started so begin.  Every kernel waits before it triggers, so when one
+// begins, all but its immediate predecessor are complete.  Before its wait
+// it writes nothing and reads only what that predecessor does not write: the
+// mesh, and in the loops of the solves arrays and parameters written before
+// the loop (k_cg_update, k_cg_update32, k_cg_patch_z, k_patch_apply_tc).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
