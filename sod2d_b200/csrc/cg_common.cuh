@@ -143,6 +143,7 @@ inline int ensure_cg_loop(sod_gpu_ctx *c) {
   CUDA_TRY(cudaMemset(G.ticket, 0, sizeof(unsigned)));
   CUDA_TRY(cudaMemset(G.S, 0, sizeof(CgScal)));
   void *h1 = nullptr, *h2 = nullptr;
+  CUDA_TRY(cudaEventCreateWithFlags(&G.read, cudaEventDisableTiming));
   CUDA_TRY(cudaMallocHost(&h1, sizeof(CgScal)));
   CUDA_TRY(cudaMallocHost(&h2, sizeof(double) * CG_HIST));
   G.S_h = (CgScal *)h1;
@@ -150,22 +151,6 @@ inline int ensure_cg_loop(sod_gpu_ctx *c) {
   c->host_allocs.push_back(h1);
   c->host_allocs.push_back(h2);
   return 0;
-}
-
-// Iterations of an FP32 solve to queue before the host reads the scalars S
-// again, `it` done of maxIter: `first` at the start, then as many as are left
-// at the mean rate so far, within least * it and most * it.  An iteration
-// queued after convergence is not free: its kernels issue their mesh loads,
-// and some the node loads, before they know the status (callers' figures).
-inline int cg_batch(const CgScal &S, int it, int maxIter, int first, double least, double most) {
-  double n = first;
-  if (it > 0) {
-    const double nrm = std::sqrt(S.rr), fall = std::log(nrm / S.bnorm), todo = std::log(S.thr2 / nrm);
-    double left = std::ceil(it * todo / fall);
-    if (!(fall < 0.0 && left < most * it)) left = most * it;
-    n = std::max({n, std::floor(least * it), std::floor(left)});
-  }
-  return (int)std::min(n, (double)(maxIter - it));
 }
 
 // start (or restart) of the device-resident CG: d = [r.z, r.r]

@@ -75,6 +75,7 @@ struct sod_gpu_ctx {
     double *x, *r, *p, *q, *z0, *z1, *b, *Minv;                // FP64 CG
     double *part, *dots;                                        // reductions
     CgScal *S = nullptr, *S_h = nullptr;                        // device-resident CG scalars (+ pinned host copy)
+    cudaEvent_t read = nullptr;                                 // a copy of the scalars has arrived
     double *hist = nullptr, *hist_h = nullptr;                  // ||r||^2 per iteration (ring)
     unsigned *ticket = nullptr;                                 // grid-sum ticket
     unsigned *dticket = nullptr;                                // ticket of k_dot

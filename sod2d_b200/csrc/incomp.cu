@@ -75,14 +75,16 @@ namespace {
 // per iteration (search direction and element Laplacian; assembly, p.Ap and
 // alpha; update, norms and beta) and one host read per batch of iterations,
 // where six launches and a host read per iteration left the GPU idle a third
-// of the time.  Batches: two iterations, then those left at the mean rate so
-// far, between 3 and 9 times those done.  An iteration queued after
-// convergence costs 17 of 126 us at 48^3, 5 of 25 at 20^3 order 4, a read 15.
-// Solves that converge after 1, 4, 12 iterations: 319, 783, 1899 us at 48^3
-// (504, 1140, 2808 with the host loop; 1607, 1776, 2243 with all 20 queued at
-// once).  The scalars are rounded as on the host: same iterates but for the
-// order of the FP64 sums.  (Where dot products pass through the
-// caller's allreduce, the host loop below runs: solves_alone.)
+// of the time.  Five iterations are queued, then up to four times as many as
+// were done (20, the reference's maximum, after one read).  One after
+// convergence costs 17 of 126 us at 48^3, 5 of 15 at 12^3 (ended_late).  One
+// more is queued behind each read, so that the GPU works while the host looks
+// (a read without it: 14 us).  Solves that converge after 1, 4, 12, 20
+// iterations: 410, 717, 1876, 2697 us at 48^3 (503, 1138, 2844, 4537 with the
+// host loop; 1602, 1772, 2249, 2680 with all 20 queued at once).
+// The scalars are rounded as on the host: same iterates but for the order of
+// the FP64 sums.  (Where dot products pass through the caller's allreduce, the
+// host loop below runs: solves_alone.)
 int conjgrad_pressure_dev(sod_gpu_ctx *c, const float *Rp0, float *R, int maxIter, double tol, int *iters,
                           double *res_rel) {
   int rc;
@@ -93,10 +95,9 @@ int conjgrad_pressure_dev(sod_gpu_ctx *c, const float *Rp0, float *R, int maxIte
   lap<float>(c, Rp0, G.q32);
   k_cg_start32<<<cg_blocks(N, CG_U), CG_THREADS, 0, st>>>(N, R, G.q32, G.diag, tol, G.x32, G.r32, G.p32, G.z032, G.S,
                                                           G.gpart, G.ticket);
-  int it = 0;
-  while (it < maxIter) {
-    const int it0 = it, nbat = cg_batch(*G.S_h, it, maxIter, 2, 3.0, 9.0);
-    for (int k = 0; k < nbat; ++k)
+  int queued = 0, it = 0;
+  auto queue_to = [&](int n) {
+    for (n = std::min(n, maxIter); queued < n; ++queued)
       dispatch(c, [&](auto L) {
         constexpr int P = decltype(L)::P_;
         launch_pdl(k_lap_elem<P, float, true>, nblk(c->nelem, LapCfg<P>::EPB), 32 * LAP_WARPS, 0, st, c->md(),
@@ -107,8 +108,14 @@ int conjgrad_pressure_dev(sod_gpu_ctx *c, const float *Rp0, float *R, int maxIte
                    G.z032, G.S, G.gpart, G.ticket);
         return 0;
       });
+  };
+  while (it < maxIter) {
+    const int it0 = it;
+    queue_to(it == 0 ? 5 : (int)std::min(4LL * it, (long long)maxIter));
     CUDA_TRY(cudaMemcpyAsync(G.S_h, G.S, sizeof(CgScal), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    CUDA_TRY(cudaEventRecord(G.read, st));
+    queue_to(queued + 1);
+    CUDA_TRY(cudaEventSynchronize(G.read));
     it = G.S_h->iter;
     if (G.S_h->status == 3) return fail(SOD_GPU_ENONFINITE, "non-finite residual in pressure CG");
     if (G.S_h->status == 1) break;
@@ -720,12 +727,11 @@ int velo_dots(sod_gpu_ctx *c, const float *a0, const float *b0, const float *c0,
 
 // conjGrad_veloc_incomp with its scalars on the device (single rank): seven
 // launches per iteration without a host read, where eleven and three reads
-// took 1.3 times (48^3) to four times (12^3) as long.  A step takes one or
-// two iterations, and one queued after convergence costs 290 of 570 us at
-// 48^3: the first is read by itself, then as many are queued as are left at
-// the mean rate, between half and twice those done.  Solves of 1, 2, 5
-// iterations at 48^3: 1.13, 1.71, 3.72 ms (1.28, 2.03, 4.27 with the host
-// loop; 2.01, 2.27, 4.28 in batches of four).
+// took 1.3 times (48^3) to four times (12^3) as long.  A step takes one to
+// four iterations.  One queued after convergence costs 290 of 570 us at 48^3,
+// 30 of 98 at 20^3 order 4, 9 of 28 at 12^3, a read 14: up to 600,000 element
+// nodes the first four are queued together, above that one, then half as many
+// as were done.
 int conjgrad_veloc_dev(sod_gpu_ctx *c, float fact, float dt, const float *mu_fluid, const float *musgs, int maxIter,
                        double tol, int *iters, double *res_rel) {
   int rc;
@@ -734,6 +740,7 @@ int conjgrad_veloc_dev(sod_gpu_ctx *c, float fact, float dt, const float *mu_flu
   auto &G = c->cg;
   const long long N = c->npoin;
   const unsigned nb = nblk(N, VELO_THREADS);
+  const int first = (long long)c->nelem * c->N <= 600000 ? 4 : 1;
   const cudaStream_t st = c->stream;
   auto apply = [&](const float *v, const int *stop) {
     velo_tau(c, v, stop);
@@ -744,7 +751,7 @@ int conjgrad_veloc_dev(sod_gpu_ctx *c, float fact, float dt, const float *mu_flu
              V.x, V.b, V.q, V.r, V.p, G.S, G.gpart, G.ticket);
   int it = 0;
   while (it < maxIter) {
-    const int it0 = it, nbat = cg_batch(*G.S_h, it, maxIter, 1, 0.5, 2.0);
+    const int it0 = it, nbat = std::min(it == 0 ? first : std::max(1, it / 2), maxIter - it);
     for (int k = 0; k < nbat; ++k) {
       apply(V.p, &G.S->status);
       launch_pdl(k_veloc_gather_op<false>, nb, VELO_THREADS, 0, st, c->md(), c->is_work, c->slotsB, c->Ml, fact, dt,

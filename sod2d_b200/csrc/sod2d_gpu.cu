@@ -171,6 +171,7 @@ int sod_gpu_finalize(sod_gpu_ctx *ctx) {
   for (void *p : ctx->halo.own) cudaFree(p);
   for (void *p : ctx->allocs) cudaFree(p);
   for (void *p : ctx->host_allocs) cudaFreeHost(p);
+  if (ctx->cg.read) cudaEventDestroy(ctx->cg.read);
   delete ctx;
   return 0;
 }

@@ -259,20 +259,22 @@ def _launches(fn, kernel):
     return sum(e.count for e in prof.key_averages() if kernel in e.key)
 
 
-@pytest.mark.parametrize("porder", [3, 4])
-def test_solves_that_converge_at_once_queue_no_tail(gpu, porder):
+@pytest.mark.parametrize("porder,n,velocity_queue", [(3, 22, 1), (4, 4, 4)])
+def test_solves_that_converge_at_once_queue_no_tail(gpu, porder, n, velocity_queue):
     """Iterations queued beyond convergence are launches and mesh reads for
-    nothing: none after one or two pressure iterations but the second, none
-    after one velocity iteration."""
-    m = host.periodic_cube(porder, 3, 4, 5, jitter=0.05, seed=8)
-    N, w = m.npoin, m.lpoin_w - 1
+    nothing.  After one or two iterations of the pressure solve: the first
+    five and the one behind the read; after one of the velocity solve: none
+    above 600,000 element nodes, the first four below."""
+    m = host.periodic_cube(porder, n, jitter=0.05, seed=8)
+    N = m.npoin
     rng = np.random.default_rng(3)
-    p = np.zeros(N, np.float32)
-    p[w] = rng.normal(size=w.size)
-    b, x0, u = dv(O.laplacian(O.OracleMesh(m), p)), torch.zeros(N, device="cuda"), dv(rng.normal(size=3 * N).astype(np.float32))
+    p, b, x0 = (torch.zeros(N, device="cuda") for _ in range(3))
+    p[dv(m.lpoin_w.astype(np.int64) - 1)] = dv(rng.normal(size=m.lpoin_w.size).astype(np.float32))
+    u = dv(rng.normal(size=3 * N).astype(np.float32))
     mu = torch.full((N,), 1e-2, device="cuda")
     bv = u * dv(m.Ml).repeat(3)
     ctx = gpu.Context(m, gpu.default_phys())
+    ctx.call("sod_gpu_eval_laplacian_mult", gpu.dptr(p), gpu.dptr(b))
     it, res = C.c_int(), C.c_double()
 
     def pressure(maxit, tol):
@@ -284,8 +286,8 @@ def test_solves_that_converge_at_once_queue_no_tail(gpu, porder):
         ctx.call("sod_gpu_conjgrad_veloc", 1.0, 0.05, gpu.dptr(mu), None, gpu.dptr(u), gpu.dptr(R), maxit, tol,
                  C.byref(it), C.byref(res))
 
-    for solve, kernel, its, queued in ((pressure, "k_lap_elem", 1, 2), (pressure, "k_lap_elem", 2, 2),
-                                       (velocity, "k_tauv_elem", 1, 1)):
+    for solve, kernel, its, queued in ((pressure, "k_lap_elem", 1, 6), (pressure, "k_lap_elem", 2, 6),
+                                       (velocity, "k_tauv_elem", 1, velocity_queue)):
         solve(its, 1e-30)  # the residual after `its` iterations is the next solve's tolerance
         tol = 1.001 * res.value
         assert _launches(lambda: solve(20, tol), kernel) == 1 + queued  # and the residual of the start
