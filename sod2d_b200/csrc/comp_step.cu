@@ -353,7 +353,6 @@ ImexCoef imex_coef(int S) {
   return k;
 }
 
-// explicit convection (fact +1) of a stage state into a five-variable block
 // Halo sum of a five-variable block [mass][energy][mom x][mom y][mom z].
 int halo_block5(sod_gpu_ctx *c, float *out) {
   HaloView v{};
@@ -364,6 +363,7 @@ int halo_block5(sod_gpu_ctx *c, float *out) {
   return halo_sum(c, v);
 }
 
+// explicit convection (fact +1) of a stage state into a five-variable block
 int imex_convec(sod_gpu_ctx *c, const float *rho, const float *u, const float *q, const float *pr, const float *h,
                 float *out) {
   RhsArgs A{};
@@ -484,8 +484,9 @@ int imex_cg(sod_gpu_ctx *c, float fact, float dt, int maxIter, double tol) {
 // right-hand side: D(x0) of the step's initial state is formed once per step
 // (X.Dx0; every stage starts from x0), an iteration is the diffusion pass,
 // its assembly with p.qn, the update and the next direction, and the host
-// reads the scalars once per pair of iterations (a stage takes one or two)
-// instead of four times in each.  IMEX step at 32^3: 3.71 -> 2.59 ms.
+// reads the scalars once per pair of iterations (a stage takes one or two; a
+// stopped k_rhs takes 3 of 77 us) instead of four times in each.  IMEX step
+// at 32^3 against the host-driven loop: 2.73 -> 2.24 ms, steps in a queue.
 int imex_stage_dev(sod_gpu_ctx *c, int is, const ImexCoef &K, float dt, int maxIter, double tol) {
   auto &S = c->comp;
   auto &X = c->imex;

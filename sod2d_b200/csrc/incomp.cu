@@ -649,10 +649,6 @@ __global__ void k_fill(long long n, float v, float *__restrict__ a) {
 
 }  // namespace
 
-extern "C" {
-
-}  // extern "C"
-
 // ---- implicit velocity solve (conjGrad_veloc_incomp) ----------------------
 
 namespace {
@@ -725,7 +721,7 @@ int velo_dots(sod_gpu_ctx *c, const float *a0, const float *b0, const float *c0,
   return 0;
 }
 
-// conjGrad_veloc_incomp with its scalars on the device (single rank): seven
+// conjGrad_veloc_incomp with its scalars on the device (solves_alone): seven
 // launches per iteration without a host read, where eleven and three reads
 // took 1.3 times (48^3) to four times (12^3) as long.  A step takes one to
 // four iterations.  One queued after convergence costs 290 of 570 us at 48^3,

@@ -5,9 +5,11 @@
 //                     (natural 1-D GLL order, xi ascending)
 //   geo[e][c][t]      c = 0..8: He(i,j) at c = i + 3j (= d xi_j / d x_i);
 //                     c = 9: gpvol
-//   slots             per element-node contributions of the RHS passes, at
-//                     the node-sorted position slot_pos[e][t] (W floats)
-// One thread owns one Gauss point (= node) of one element; an element's
+//   slots             per element-node contributions: pass A's in element
+//                     order (12 floats), all others at the node-sorted
+//                     position slot_pos[e][t]
+// A thread owns one Gauss point (= node) of one element, or a line of them
+// along zeta (ColCfg: pass A, the Laplacian, the entropy pass); an element's
 // nodal fields are staged in shared memory and differentiated with the 1-D
 // GLL derivative matrix D[m][n] = l'_n(xi_m) (sum factorisation).  The
 // 4x4 / 5x5 contractions are too small for tensor cores; they run on the
@@ -286,8 +288,8 @@ __device__ __forceinline__ void col_grad2(const float *__restrict__ f, int i, in
 // ---------------------------------------------------------------------
 // Pass A: LPS projections (full_proj_ijk, elem_stab.f90:474-562).  Writes
 // gpvol * {tau00, tau01, tau02, tau11, tau12, tau22, grad rho (3), grad T
-// (3)} per element node into element-ordered slots of width 12 (coalesced
-// stores; k_gather reads them through the node->slot CSR).  tau = grad u + grad u^T
+// (3)} per element node into element-ordered slots of width 12 (bulk copies;
+// k_gather_proj reads them through the node->slot CSR).  tau = grad u + grad u^T
 // - 2/3 div u I is symmetric (tau_ab and tau_ba are the same FP32 sum), so
 // the reference's ProjMX/MY/MZ rows are read back from its 6 entries.
 // Input: conserved state (SoA, reference layout) -> EOS in registers, or
@@ -397,15 +399,16 @@ k_proj(MeshDev m, DMat<P, float> D, Phys ph, float Rgas, const float *__restrict
 
 // ---------------------------------------------------------------------
 // Pass B: convection (full_convec_ijk) and/or stabilised diffusion
-// (full_diff_stab_ijk) of one element, summed per element node into slots
-// of width 8: {mass, energy, mom x, mom y, mom z, 0, 0, 0}.
+// (full_diff_stab_ijk) of one element, summed per element node into
+// node-sorted slots: a float4 array {mass, energy, mom x, mom y}, then a
+// float array mom z.
 //
 // MODE_CONV: convective residual * fact_c.
 // MODE_DIFF: LPS-stabilised diffusion * fact_d (full_diff_stab_ijk);
 //   with MODE_NOLPS the plain diffusion of full_diffusion_ijk
 //   (elem_diffu.f90:12-223).
 // Input kinds:
-//   IN_CONS : a0 = rho, a1 = q(N,3), a2 = E (conserved; EOS fused, h = E:=aux_h)
+//   IN_CONS : rho, q(N,3), E (conserved; EOS fused, h = E:=aux_h)
 //   IN_PRIM : convection inputs u, q, rho, pr, E given directly
 //   IN_DIFF : diffusion inputs rho, u, Tem, mu_fluid given directly
 // ---------------------------------------------------------------------

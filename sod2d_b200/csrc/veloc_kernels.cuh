@@ -210,7 +210,7 @@ k_diffv_elem(MeshDev m, const float *__restrict__ u, const float *__restrict__ m
   reinterpret_cast<float4 *>(slots)[pos] = make_float4(wd[0], wd[1], wd[2], 0.f);
 }
 
-// ---- the solve on the device (single rank) ---------------------------------
+// ---- the solve on the device (no global reductions) ---------------------------------
 // The vector passes of conjGrad_veloc_incomp with their sums, as those of the
 // IMEX solve: the assembly forms qn = v Ml + fact dt D(v) and either the
 // start (r = b - qn, p = z = r / M, M = Ml / dt) or p.qn and alpha.
