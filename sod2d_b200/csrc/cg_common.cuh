@@ -104,7 +104,7 @@ inline int ensure_cg32(sod_gpu_ctx *c) {
   if (G.ready32) return 0;
   int rc;
   for (float **pp : {&G.x32, &G.r32, &G.p32, &G.q32, &G.z032})
-    if ((rc = c->alloc(pp, (size_t)c->npoin))) return rc;
+    if ((rc = c->need(pp, (size_t)c->npoin))) return rc;
   G.ready32 = true;
   return 0;
 }
@@ -114,7 +114,7 @@ inline int ensure_cg64(sod_gpu_ctx *c) {
   if (G.ready64) return 0;
   int rc;
   for (double **pp : {&G.x, &G.r, &G.p, &G.q, &G.z0, &G.z1, &G.b, &G.Minv})
-    if ((rc = c->alloc(pp, (size_t)c->npoin))) return rc;
+    if ((rc = c->need(pp, (size_t)c->npoin))) return rc;
   G.ready64 = true;
   return 0;
 }
@@ -135,21 +135,24 @@ static_assert(TcDims<3>::WARPS == TcDims<4>::WARPS, "one block size for both ord
 
 inline int ensure_cg_loop(sod_gpu_ctx *c) {
   auto &G = c->cg;
-  if (G.S) return 0;
+  if (G.ready_loop) return 0;
   int rc;
-  if ((rc = c->alloc(&G.S, 1)) || (rc = c->alloc(&G.hist, CG_HIST)) || (rc = c->alloc(&G.ticket, 1)) ||
-      (rc = c->alloc(&G.gpart, (size_t)3 * cg_blocks(c->npoin, 1))))
+  if ((rc = c->need(&G.S, 1)) || (rc = c->need(&G.hist, CG_HIST)) || (rc = c->need(&G.ticket, 1)) ||
+      (rc = c->need(&G.gpart, (size_t)3 * cg_blocks(c->npoin, 1))))
     return rc;
   CUDA_TRY(cudaMemset(G.ticket, 0, sizeof(unsigned)));
   CUDA_TRY(cudaMemset(G.S, 0, sizeof(CgScal)));
-  void *h1 = nullptr, *h2 = nullptr;
-  CUDA_TRY(cudaEventCreateWithFlags(&G.read, cudaEventDisableTiming));
-  CUDA_TRY(cudaMallocHost(&h1, sizeof(CgScal)));
-  CUDA_TRY(cudaMallocHost(&h2, sizeof(double) * CG_HIST));
-  G.S_h = (CgScal *)h1;
-  G.hist_h = (double *)h2;
-  c->host_allocs.push_back(h1);
-  c->host_allocs.push_back(h2);
+  if (!G.read) CUDA_TRY(cudaEventCreateWithFlags(&G.read, cudaEventDisableTiming));
+  auto pinned = [&](auto **p, size_t bytes) -> int {
+    void *h = nullptr;
+    if (*p) return 0;
+    CUDA_TRY(cudaMallocHost(&h, bytes));
+    c->host_allocs.push_back(h);
+    *p = static_cast<std::remove_reference_t<decltype(*p)>>(h);
+    return 0;
+  };
+  if ((rc = pinned(&G.S_h, sizeof(CgScal))) || (rc = pinned(&G.hist_h, sizeof(double) * CG_HIST))) return rc;
+  G.ready_loop = true;
   return 0;
 }
 

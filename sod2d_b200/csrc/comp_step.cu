@@ -312,14 +312,21 @@ namespace {
 
 int ensure_imex(sod_gpu_ctx *c) {
   auto &X = c->imex;
-  if (X.R) return 0;
   const size_t N = c->npoin, EN = (size_t)c->nelem * c->N;
   int rc;
-  if ((rc = c->alloc(&X.R, 4 * 5 * N)) || (rc = c->alloc(&X.D, 4 * 5 * N)) || (rc = c->alloc(&X.stab, 5 * N)) ||
-      (rc = c->alloc(&X.lvl1, 5 * N)) || (rc = c->alloc(&X.aux_h, N)) || (rc = c->alloc(&X.x, 5 * N)) ||
-      (rc = c->alloc(&X.r, 5 * N)) || (rc = c->alloc(&X.p, 5 * N)) || (rc = c->alloc(&X.qn, 5 * N)) ||
-      (rc = c->alloc(&X.au, 3 * N)) || (rc = c->alloc(&X.aT, N)) || (rc = c->alloc(&X.zmu, N)) ||
-      (rc = c->alloc(&X.zmue, EN)))
+  // the workspaces of the loop that this step takes
+  if (solves_alone(c)) {
+    if ((rc = ensure_cg_loop(c)) || (rc = c->need(&X.Dx0, 5 * N))) return rc;
+  } else {
+    for (float **v : {&X.b, &X.z, &X.z1})
+      if ((rc = c->need(v, 5 * N))) return rc;
+  }
+  if (X.ready) return 0;
+  if ((rc = c->need(&X.R, 4 * 5 * N)) || (rc = c->need(&X.D, 4 * 5 * N)) || (rc = c->need(&X.stab, 5 * N)) ||
+      (rc = c->need(&X.lvl1, 5 * N)) || (rc = c->need(&X.aux_h, N)) || (rc = c->need(&X.x, 5 * N)) ||
+      (rc = c->need(&X.r, 5 * N)) || (rc = c->need(&X.p, 5 * N)) || (rc = c->need(&X.qn, 5 * N)) ||
+      (rc = c->need(&X.au, 3 * N)) || (rc = c->need(&X.aT, N)) || (rc = c->need(&X.zmu, N)) ||
+      (rc = c->need(&X.zmue, EN)))
     return rc;
   if (!c->cg.part && ((rc = c->alloc(&c->cg.part, 8 * DOT_BLOCKS)) || (rc = c->alloc(&c->cg.dots, 16)))) return rc;
   for (float *v : {X.R, X.D}) CUDA_TRY(cudaMemsetAsync(v, 0, 4 * 5 * N * 4, c->stream));
@@ -327,6 +334,7 @@ int ensure_imex(sod_gpu_ctx *c) {
   CUDA_TRY(cudaMemsetAsync(X.au, 0, 3 * N * 4, c->stream));
   for (float *v : {X.aT, X.zmu, X.aux_h}) CUDA_TRY(cudaMemsetAsync(v, 0, N * 4, c->stream));
   CUDA_TRY(cudaMemsetAsync(X.zmue, 0, EN * 4, c->stream));
+  X.ready = true;
   return 0;
 }
 
@@ -437,8 +445,7 @@ int imex_cg(sod_gpu_ctx *c, float fact, float dt, int maxIter, double tol) {
   const int nw = c->npoin_w;
   const unsigned nb = nblk(nw, 256);
   const float gm1 = c->phys.gamma_gas - 1.0f;
-  int rc = c->alloc_once(5 * N, &X.b, &X.z, &X.z1);
-  if (rc) return rc;
+  int rc;
   CUDA_TRY(cudaMemcpyAsync(X.x, X.lvl1, 5 * N * 4, cudaMemcpyDeviceToDevice, c->stream));
   CUDA_TRY(cudaMemcpyAsync(X.b, S.rho32, N * 4, cudaMemcpyDeviceToDevice, c->stream));
   CUDA_TRY(cudaMemcpyAsync(X.b + N, S.E32, N * 4, cudaMemcpyDeviceToDevice, c->stream));
@@ -600,8 +607,7 @@ int sod_gpu_comp_imex_step(sod_gpu_ctx *c, float dt, int maxIter, double tol) {
   const bool dev = solves_alone(c);
   if (dev) {  // D(x0) of the step's initial state, the first residual's operator in every stage
     k_imex_prim<<<nb, 256, 0, st>>>(nw, N, c->lpoin_w, gm - 1.0f, c->phys.Rgas, X.lvl1, X.lvl1, X.au, X.aT);
-    if ((rc = ensure_cg_loop(c)) || (rc = c->alloc_once(5 * N, &X.Dx0)) ||
-        (rc = imex_diffusion(c, X.lvl1, X.lvl1, X.au, X.aT, X.Dx0))) {
+    if ((rc = imex_diffusion(c, X.lvl1, X.lvl1, X.au, X.aT, X.Dx0))) {
       c->async = was_async;
       return rc;
     }

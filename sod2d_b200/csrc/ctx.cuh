@@ -68,12 +68,13 @@ struct sod_gpu_ctx {
   float volT = 0.f;
   // pressure-solve workspace (lazily allocated)
   struct Cg {
-    bool ready32 = false, ready64 = false, have_diag = false;
+    bool ready32 = false, ready64 = false, ready_loop = false, have_diag = false;
     float *diag = nullptr;                                     // Jacobi diagonal (FP32)
-    float *x32, *r32, *p32, *q32, *z032;                       // reference-arithmetic CG
+    float *x32 = nullptr, *r32 = nullptr, *p32 = nullptr, *q32 = nullptr, *z032 = nullptr;  // reference-arithmetic CG
     float *z132 = nullptr, *b32 = nullptr;                     //   its host-driven loop's
-    double *x, *r, *p, *q, *z0, *z1, *b, *Minv;                // FP64 CG
-    double *part, *dots;                                        // reductions
+    double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *z0 = nullptr, *z1 = nullptr, *b = nullptr,
+           *Minv = nullptr;                                     // FP64 CG
+    double *part = nullptr, *dots = nullptr;                    // reductions
     CgScal *S = nullptr, *S_h = nullptr;                        // device-resident CG scalars (+ pinned host copy)
     cudaEvent_t read = nullptr;                                 // a copy of the scalars has arrived
     double *hist = nullptr, *hist_h = nullptr;                  // ||r||^2 per iteration (ring)
@@ -121,6 +122,7 @@ struct sod_gpu_ctx {
   } inc;
   // implicit velocity solve (conjGrad_veloc_incomp)
   struct Velo {
+    bool ready = false;
     float *tauP = nullptr, *tau_e = nullptr;                   // [npoin][8] projection, [E] tau
     float *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *b = nullptr;  // (npoin,3)
     float *z = nullptr, *z1 = nullptr;                         // the host-driven loop's
@@ -139,6 +141,7 @@ struct sod_gpu_ctx {
   } comp;
   // IMEX integrator scratch (five-variable blocks [mass][energy][momentum])
   struct Imex {
+    bool ready = false;
     float *R = nullptr, *D = nullptr;  // [4 stages][5N] explicit / implicit residuals
     float *stab = nullptr, *lvl1 = nullptr, *aux_h = nullptr;
     float *x = nullptr, *r = nullptr, *p = nullptr, *qn = nullptr;
@@ -177,17 +180,19 @@ struct sod_gpu_ctx {
     size_t b = count * sizeof(T);
     if (b == 0) b = 16;
     cudaError_t e = cudaMalloc((void **)p, b);
-    if (e != cudaSuccess) return fail(SOD_GPU_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // reported here, not by the next call that asks
+      return fail(SOD_GPU_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     allocs.push_back(*p);
     bytes += b;
     return 0;
   }
-  // workspaces that one of a solve's two loops needs, at its first use
-  template <class... T>
-  int alloc_once(size_t count, T *...p) {
-    for (float **q : {p...})
-      if (int rc = *q ? 0 : alloc(q, count)) return rc;
-    return 0;
+  // Workspaces at their first use.  An allocation that failed is tried again
+  // on the next call, which finds those before it in place.
+  template <class T>
+  int need(T **p, size_t count) {
+    return *p ? 0 : alloc(p, count);
   }
   template <class T>
   int upload(T **p, const T *host, size_t count) {

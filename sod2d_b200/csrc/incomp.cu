@@ -139,7 +139,8 @@ int sod_gpu_conjgrad_pressure(sod_gpu_ctx *c, const float *Rp0, float *R, int ma
   int rc;
   auto &G = c->cg;
   const size_t N = c->npoin;
-  if ((rc = ensure_diag(c)) || (rc = ensure_cg32(c)) || (rc = c->alloc_once(N, &G.z132, &G.b32))) return rc;
+  if ((rc = ensure_diag(c)) || (rc = ensure_cg32(c)) || (rc = c->need(&G.z132, N)) || (rc = c->need(&G.b32, N)))
+    return rc;
   const cudaStream_t st = c->stream;
   for (float *z : {G.x32, G.r32, G.p32, G.q32, G.z032, G.z132, G.b32}) CUDA_TRY(cudaMemsetAsync(z, 0, N * 4, st));
   // b = R - A x0 ; r0 = b ; z0 = r0 / M ; p0 = z0   (mod_solver_incomp.f90:310-350)
@@ -655,15 +656,16 @@ namespace {
 
 int ensure_velo(sod_gpu_ctx *c) {
   auto &V = c->velo;
-  if (V.tauP) return 0;
+  if (V.ready) return 0;
   const size_t N = c->npoin;
   int rc;
-  if ((rc = c->alloc(&V.tauP, N * 8)) || (rc = c->alloc(&V.tau_e, (size_t)c->nelem)) ||
-      (rc = c->alloc(&V.x, 3 * N)) || (rc = c->alloc(&V.r, 3 * N)) || (rc = c->alloc(&V.p, 3 * N)) ||
-      (rc = c->alloc(&V.q, 3 * N)) || (rc = c->alloc(&V.b, 3 * N)))
+  if ((rc = c->need(&V.tauP, N * 8)) || (rc = c->need(&V.tau_e, (size_t)c->nelem)) ||
+      (rc = c->need(&V.x, 3 * N)) || (rc = c->need(&V.r, 3 * N)) || (rc = c->need(&V.p, 3 * N)) ||
+      (rc = c->need(&V.q, 3 * N)) || (rc = c->need(&V.b, 3 * N)))
     return rc;
   if (!c->cg.part && ((rc = c->alloc(&c->cg.part, 8 * DOT_BLOCKS)) || (rc = c->alloc(&c->cg.dots, 16)))) return rc;
   for (float *v : {V.x, V.r, V.p, V.q, V.b}) CUDA_TRY(cudaMemsetAsync(v, 0, 3 * N * 4, c->stream));
+  V.ready = true;
   return 0;
 }
 
@@ -835,7 +837,7 @@ int sod_gpu_conjgrad_veloc(sod_gpu_ctx *c, float fact, float dt, const float *mu
     CUDA_TRY(cudaMemcpyAsync(R, V.x, 3 * N * 4, cudaMemcpyDeviceToDevice, c->stream));
     return c->finish();
   }
-  if ((rc = c->alloc_once(3 * N, &V.z, &V.z1))) { c->async = was_async; return rc; }
+  if ((rc = c->need(&V.z, 3 * N)) || (rc = c->need(&V.z1, 3 * N))) { c->async = was_async; return rc; }
   auto apply = [&](const float *v) {  // q = v Ml + fact dt D(v)
     int arc = velo_tau(c, v);
     if (arc) return arc;

@@ -340,3 +340,44 @@ def test_solves_allocate_their_own_loops_workspaces(gpu):
     # stages 40, stabilisation, level 1, D(x0), x r p qn 35, enthalpy, velocity, temperature, viscosity 6
     assert s.ctx.device_bytes - b0 <= 4 * (81 * N + EN) + small
     s.close()
+
+
+def test_solves_after_a_failed_allocation(gpu):
+    """A workspace that did not fit is reported, and the same call works once
+    there is room: nothing is taken for allocated that is not."""
+    m = host.periodic_cube(3, 24, 24, 12)
+    N = m.npoin
+    ic = host.tgv_comp_init(m, Ma=1.25)
+    kw = dict(stages=4, fp64_state=False, cfl_conv=0.95, cfl_diff=1000.5, imex=True)
+    mu = torch.full((N,), 1e-2, device="cuda")
+    u = dv(np.random.default_rng(1).normal(size=3 * N).astype(np.float32))
+    b = u * dv(m.Ml).repeat(3)
+
+    def velocity(ctx):
+        R = b.clone()
+        rc = gpu.lib().sod_gpu_conjgrad_veloc(ctx.h, 1.0, 0.05, gpu.dptr(mu), None, gpu.dptr(u), gpu.dptr(R), 5, 1e-2,
+                                              None, None)
+        return rc, R
+
+    ref, s = (gpu.CompSolver(m, ic, **kw) for _ in range(2))
+    ref.step()
+    want = velocity(ref.ctx)[1]
+    room = b.clone()  # for the calls' own tensors while memory is full
+    del room
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    # room for the first of the step's workspaces (5 and 20 N floats), not for the next
+    full = torch.empty(max(free - 4 * 30 * N, 0) // (1 << 21) * (1 << 21), dtype=torch.uint8, device="cuda")
+    rc = gpu.lib().sod_gpu_comp_imex_step(s.ctx.h, float(s.dt), 200, 1e-3)
+    rc_v = velocity(s.ctx)[0]
+    del full
+    torch.cuda.empty_cache()
+    assert rc == -3
+    assert rc_v in (0, -3)
+    s.step()
+    got = velocity(s.ctx)
+    assert got[0] == 0 and torch.equal(got[1], want)
+    a, r = s.state(), ref.state()
+    assert all(np.array_equal(a[k], r[k]) for k in a)
+    s.close()
+    ref.close()
