@@ -728,8 +728,10 @@ int velo_dots(sod_gpu_ctx *c, const float *a0, const float *b0, const float *c0,
 // took 1.3 times (48^3) to four times (12^3) as long.  A step takes one to
 // four iterations.  One queued after convergence costs 290 of 570 us at 48^3,
 // 30 of 98 at 20^3 order 4, 9 of 28 at 12^3, a read 14: up to 600,000 element
-// nodes the first four are queued together, above that one, then half as many
-// as were done.
+// nodes the first four are queued together, up to two million two, above that
+// one, then half as many as were done.  Steps at 20^3 order 4 whose solve
+// takes 1, 2, 3, 4 iterations: 1014, 1077, 1186, 1301
+// us; with four first 1050, 1111, 1178, 1256.
 int conjgrad_veloc_dev(sod_gpu_ctx *c, float fact, float dt, const float *mu_fluid, const float *musgs, int maxIter,
                        double tol, int *iters, double *res_rel) {
   int rc;
@@ -738,7 +740,8 @@ int conjgrad_veloc_dev(sod_gpu_ctx *c, float fact, float dt, const float *mu_flu
   auto &G = c->cg;
   const long long N = c->npoin;
   const unsigned nb = nblk(N, VELO_THREADS);
-  const int first = (long long)c->nelem * c->N <= 600000 ? 4 : 1;
+  const long long EN = (long long)c->nelem * c->N;
+  const int first = EN <= 600000 ? 4 : (EN <= 2000000 ? 2 : 1);
   const cudaStream_t st = c->stream;
   auto apply = [&](const float *v, const int *stop) {
     velo_tau(c, v, stop);

@@ -259,12 +259,12 @@ def _launches(fn, kernel):
     return sum(e.count for e in prof.key_averages() if kernel in e.key)
 
 
-@pytest.mark.parametrize("porder,n,velocity_queue", [(3, 22, 1), (4, 4, 4)])
+@pytest.mark.parametrize("porder,n,velocity_queue", [(3, 32, 1), (3, 22, 2), (4, 4, 4)])
 def test_solves_that_converge_at_once_queue_no_tail(gpu, porder, n, velocity_queue):
     """Iterations queued beyond convergence are launches and mesh reads for
     nothing.  After one or two iterations of the pressure solve: the first
     five and the one behind the read; after one of the velocity solve: none
-    above 600,000 element nodes, the first four below."""
+    above two million element nodes, the first two above 600,000, four below."""
     m = host.periodic_cube(porder, n, jitter=0.05, seed=8)
     N = m.npoin
     rng = np.random.default_rng(3)
